@@ -123,6 +123,7 @@ public:
         cudaDeviceProp prop;
         check(cudaGetDeviceProperties(&prop, (int)params_.device_id), "cudaGetDeviceProperties");
         sms_ = prop.multiProcessorCount;
+        set_runs();
         allocate();
         configure();
         initialise();
@@ -946,23 +947,30 @@ private:
                 tile_info_.push_back({b.cell_base + t * tc, std::min(tc, b.C - t * tc) | (tc << 16), (uint32_t)r, 0u});
         }
         tiles_ = tiles;
-        // runs of up to 32 cells of one box (srd_run_kernel): {first cell, cells | box << 6},
-        // listed by batch class (16, 8, then 4 cells per batch; one launch per class)
+        pbuf_ = pbuf;
+        fill_ = fill;
+        for (auto& g : graph_) g.reset();   // graphs bake the tiling into their launches
+    }
+
+    // Runs of srd_run_kernel: up to 32 cells of one box, {first cell, cells | box << 6},
+    // listed by batch class (16, 8, then 4 cells per batch; one launch per class).
+    void set_runs()
+    {
         run_info_.clear();
+        for (BoxDesc& b : boxes_) {
+            b.run_cells = 32;
+        }
         for (int cls = 0; cls < 3; ++cls) {
             run_class_[cls] = (uint32_t)run_info_.size();
             const uint32_t batch = 16u >> cls;
             for (size_t r = 0; r < boxes_.size(); ++r) {
                 const BoxDesc& b = boxes_[r];
                 if (b.run_batch != batch) continue;
-                for (uint32_t c = 0; c < b.C; c += 32)
-                    run_info_.push_back(make_uint2(b.cell_base + c, std::min(32u, b.C - c) | ((uint32_t)r << 6)));
+                for (uint32_t c = 0; c < b.C; c += b.run_cells)
+                    run_info_.push_back(make_uint2(b.cell_base + c, std::min(b.run_cells, b.C - c) | ((uint32_t)r << 6)));
             }
         }
         run_class_[3] = (uint32_t)run_info_.size();
-        pbuf_ = pbuf;
-        fill_ = fill;
-        for (auto& g : graph_) g.reset();   // graphs bake the tiling into their launches
     }
 
     void retile(double fill, uint32_t pbuf)
@@ -1002,7 +1010,7 @@ private:
             check(cudaMemset(count_[k].p, 0, count_[k].bytes), "clear counts");
         }
         if (walls_) check(ghosts_.alloc(sizeof(GhostSum) * walls_), "alloc wall ghosts");
-        if (boxes_.size() > 1) check(box_shifts_.alloc(sizeof(float4) * 2 * boxes_.size()), "alloc box shifts");
+        check(box_shifts_.alloc(sizeof(float4) * 2 * boxes_.size()), "alloc box shifts");
         check(state_.alloc(sizeof(DeviceState)), "alloc state");
         check(cudaMemset(state_.p, 0, sizeof(DeviceState)), "clear state");
         check(samp_.alloc(sizeof(float4) * cells_ * 2), "alloc sample");   // two parities
@@ -1074,7 +1082,7 @@ private:
         a.boxes_n_max = n_max_;
         a.total_walls = walls_;
         a.ghosts = ghosts_.as<GhostSum>();
-        a.box_shifts = boxes_.size() > 1 ? box_shifts_.as<float4>() : nullptr;
+        a.box_shifts = box_shifts_.as<float4>();
         a.total_slots = total_slots_;
         a.ext_cap = ext_cap_;
         a.step = k;
@@ -1180,6 +1188,16 @@ private:
         return done;
     }
 
+    // Blocks of the prologue: a thread per wall cell whose ghosts it draws, and a warp
+    // per 256 cells for the overflow list (a few entries a warp in a dilute box, where
+    // one cell in 50 overflows).
+    int select_blocks(const StepArgs& a) const
+    {
+        const uint64_t walls = a.run_kernel ? a.total_walls : 0;
+        const uint64_t blocks = std::max<uint64_t>((walls + kThreads - 1) / kThreads, (cells_ + 2047) / 2048);
+        return (int)std::min<uint64_t>(blocks, (uint64_t)sms_ * 8);
+    }
+
     // The reference's choice of the particles that collide in overflowing cells,
     // made on the inputs of step k before its kernel runs.
     cudaError_t select_overflow(const StepArgs& a, uint64_t k, cudaStream_t st)
@@ -1187,7 +1205,7 @@ private:
         const unsigned p = (unsigned)(k & 1);
         return launch_overflow_select(a, slots_[p].as<Slot>(), ov_pos_[p].as<float4>(), ov_vel_[p].as<float4>(),
                                       ov_head_[p].as<uint32_t>(),
-                                      a.run_kernel && (a.total_walls || a.box_shifts) ? sms_ * 8 : sms_, st);
+                                      select_blocks(a), st);
     }
 
     // The wall-ghost array of srd_run_kernel for a step that it runs (its prologue
@@ -1286,8 +1304,8 @@ private:
         const uint64_t k = step_;
         for (uint64_t j = k; j < k + 2; ++j) {
             check(cudaMemsetAsync(count_[j % 3].p, 0, count_[j % 3].bytes, stream_), "clear counts");
-            check(cudaMemsetAsync((char*)state_.p + offsetof(DeviceState, ov_count) + sizeof(unsigned int) * (j % 3),
-                                  0, sizeof(unsigned int), stream_),
+            check(cudaMemsetAsync((char*)state_.p + offsetof(DeviceState, ov) + sizeof(OverflowFill) * (j % 3), 0,
+                                  sizeof(OverflowFill), stream_),
                   "clear overflow list");
         }
         check(cudaMemsetAsync((char*)state_.p + offsetof(DeviceState, ext_count) + sizeof(unsigned int) * (k & 1), 0,

@@ -203,7 +203,7 @@ __device__ __forceinline__ void sample_add(float4* samp, uint32_t lab, float3 v,
 __device__ __forceinline__ void push_overflow(const StepArgs& a, uint32_t key, float4 xp, float4 vp)
 {
     atomicAdd(&a.state->overflow_total, 1ull);
-    const unsigned q = atomicAdd(&a.state->ov_count[a.ov_out_slot], 1u);
+    const unsigned q = atomicAdd(&a.state->ov[a.ov_out_slot].count, 1u);
     if (q < a.ov_cap) {
         a.ov_out_pos[q] = xp;
         a.ov_out_vel[q] = vp;
@@ -535,10 +535,13 @@ __device__ __forceinline__ uint32_t fetch_count(const StepArgs& a, uint32_t firs
 // ids of a cell collide; the selection marked the entries it moved to the cell's
 // extension kTakenId): as in the reference, they skip the collision and keep the
 // unshifted position pbc(pbc(x + s) - s) (simulation_functions.cpp:90-93).
+// Called by every block of a launch, each taking its share of the list, and only
+// when the selection left such particles (OverflowFill::left): a list of 44,000 entries, all
+// of them taken, cost one block 300 us.
 __device__ void overflow_pass(const StepArgs& a, uint64_t step)
 {
-    const uint32_t n = min(a.state->ov_count[a.ov_in_slot], a.ov_cap);
-    for (uint32_t base = 0; base < n; base += kThreads) {
+    const uint32_t n = min(a.state->ov[a.ov_in_slot].count, a.ov_cap);
+    for (uint32_t base = blockIdx.x * kThreads; base < n; base += gridDim.x * kThreads) {
         const uint32_t q = base + threadIdx.x;
         const float4 w = q < n ? a.ov_in_vel[q] : make_float4(0, 0, 0, 0);
         const bool active = q < n && __float_as_uint(w.w) != kTakenId;
@@ -621,10 +624,10 @@ __global__ void __launch_bounds__(kThreads, 4) step_kernel(const StepArgs a, uin
     const uint64_t step = a.step_base ? *a.step_base + a.step : a.step;   // graph replays read the base
     float imp[2] = {0.0f, 0.0f};   // pressure estimator: this thread's outward wall impulses
 
-    if (blockIdx.x == 0) {
-        if (tid == 0 && !a.replay) a.state->ov_count[a.ov_zero_slot] = 0;   // list of step k-1, refilled by step k+1
-        overflow_pass(a, step);
+    if (blockIdx.x == 0 && tid == 0 && !a.replay) {   // list of step k-1, refilled by step k+1
+        a.state->ov[a.ov_zero_slot] = OverflowFill{0u, 0u};
     }
+    if (a.state->ov[a.ov_in_slot].left) overflow_pass(a, step);
 
     // the tile after the current one (tile_entry): its entry is read by one
     // thread (kLocator) while the current tile's ghosts are counted, its counts by
@@ -1228,8 +1231,8 @@ __device__ __forceinline__ uint2 run_entry(const StepArgs& a, uint32_t run)
 {
     if (run >= a.num_runs) return make_uint2(0u, 0u);
     if (!SINGLE) return __ldg(a.run_info + run);
-    const uint32_t c0 = run * kRunCells;
-    return make_uint2(a.box0.cell_base + c0, min(kRunCells, a.box0.C - c0));
+    const uint32_t c0 = run * a.box0.run_cells;
+    return make_uint2(a.box0.cell_base + c0, min(a.box0.run_cells, a.box0.C - c0));
 }
 
 template <bool SAMPLE, bool SINGLE, uint32_t BATCH, bool TAPE = false>
@@ -1243,10 +1246,7 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
     BoxDesc& sbox = shared_box[SINGLE ? 0 : threadIdx.x >> 5];
     const uint64_t step = a.step_base ? *a.step_base + a.step : a.step;   // graph replays read the base
 
-    if (blockIdx.x == 0 && first_launch) {   // once per step (ensembles launch once per batch size)
-        if (threadIdx.x == 0) a.state->ov_count[a.ov_zero_slot] = 0;   // list of step k-1, refilled by step k+1
-        overflow_pass(a, step);
-    }
+    const uint32_t left = a.state->ov[a.ov_in_slot].left;
     constexpr uint32_t kBatchCells = BATCH;
     constexpr uint32_t kBatchLanes = 32 / BATCH;   // lanes per cell in the sums
     static_assert(BATCH == 4 || BATCH == 8 || BATCH == 16, "batches of 4, 8 or 16 cells");
@@ -1254,8 +1254,15 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
     const BoxDesc& b = SINGLE ? a.box0 : sbox;
     float3 s = make_float3(0, 0, 0), sn = s;
     if (SINGLE) {
-        s = grid_shift(b, 0, step, a.state);
-        sn = grid_shift(b, 0, step + 1, a.state);
+        const float4 s0 = __ldg(a.box_shifts), s1 = __ldg(a.box_shifts + 1);   // drawn by the prologue
+        s = make_float3(s0.x, s0.y, s0.z);
+        sn = make_float3(s1.x, s1.y, s1.z);
+    }
+    if (first_launch) {   // once per step (ensembles launch once per batch size)
+        if (blockIdx.x == 0 && threadIdx.x == 0) {   // list of step k-1, refilled by step k+1
+            a.state->ov[a.ov_zero_slot] = OverflowFill{0u, 0u};
+        }
+        if (left) overflow_pass(a, step);
     }
     int cur_box = -1;
     const uint32_t warps = gridDim.x * (uint32_t)kRunWarps;
@@ -1353,7 +1360,7 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
             while (summed <= hi) {
                 const uint32_t c8 = summed;
                 summed += kBatchCells;
-                if (c8 + kBatchCells < kRunCells) {
+                if (c8 + kBatchCells < (cur.y & 63u)) {
                     if (lane >= c8 + kBatchCells && lane < c8 + 2 * kBatchCells && cnt)
                         prefetch_l2(a.in_slots + src_slot, cnt * (uint32_t)sizeof(Slot));
                 } else {
@@ -1468,13 +1475,19 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
 // in: the reference fills each cell's table in particle-index order, and the
 // particles past its depth skip the collision (simulation_functions.cpp:87-93) --
 // as min(raw, cap) contiguous slots of the extension area of step k's bucket set.
-// The thread of a cell's last overflow entry (the head of the cell's chain)
-// copies the bucket there, then walks the raw - depth entries of the chain: each
-// fills the next free slot (its list entry is marked taken), or, once cap slots
-// are filled, swaps with the set's largest id if its own id is smaller.  It then
-// records the extension offset in pos.w of the cell's first bucket slot and marks
-// the chain handled, so that a second selection of the same step changes
-// nothing.  Overflow is rare: without any, every thread returns after one load.
+// The warp that meets a cell's last overflow entry (the head of the cell's chain)
+// copies the bucket there, one lane per slot, then walks the raw - depth entries
+// of the chain: each fills the next free slot (its list entry is marked taken),
+// or, once cap slots are filled, swaps with the set's largest id if its own id is
+// smaller.  It then records the extension offset in pos.w of the cell's first
+// bucket slot and marks the chain handled, so that a second selection of the same
+// step changes nothing.  Overflow is rare: without any, every warp returns after
+// one load.  What bounds it is the chain of dependent loads of one cell, so the
+// entries are spread over all warps (one each while there are fewer entries than
+// warps) and the last blocks take the first of them: the wall ghosts keep the
+// first blocks busy.  One thread per cell copied the bucket slot by slot, a
+// memory round trip each (12.9 us a step at 61 x 61 x 85, n = 7; a
+// warp 6.3 us).
 // Run on the inputs of step k, so a replay of step k finds them in place.
 // Block 0 also empties the extension of the other parity (step k+1's: step k-1,
 // its last reader, is past replaying).
@@ -1487,7 +1500,7 @@ __global__ void __launch_bounds__(kThreads) overflow_select_kernel(const StepArg
     // velocity sums.  Drawn here, every thread busy, instead of by a few lanes
     // of each run.
     const uint64_t step = a.step_base ? *a.step_base + a.step : a.step;
-    if (a.run_kernel && a.box_shifts) {   // ensembles: every box's grid shifts of steps k and k+1
+    if (a.run_kernel) {   // every box's grid shifts of steps k and k+1
         for (uint32_t bi = blockIdx.x * blockDim.x + threadIdx.x; bi < (uint32_t)a.nboxes; bi += gridDim.x * blockDim.x) {
             const float3 s0 = grid_shift(a.boxes[bi], (int)bi, step, a.state);
             const float3 s1 = grid_shift(a.boxes[bi], (int)bi, step + 1, a.state);
@@ -1537,56 +1550,92 @@ __global__ void __launch_bounds__(kThreads) overflow_select_kernel(const StepArg
     }
     const uint32_t par = (uint32_t)(a.step & 1u);
     if (blockIdx.x == 0 && threadIdx.x == 0) a.state->ext_count[par ^ 1u] = 0;
-    const uint32_t n = min(a.state->ov_count[a.ov_in_slot], a.ov_cap);
-    for (uint32_t e0 = blockIdx.x * blockDim.x + threadIdx.x; e0 < n; e0 += gridDim.x * blockDim.x) {
-        const uint32_t id0 = __float_as_uint(ov_vel[e0].w);
-        if (id0 == kTakenId) continue;
-        const float4 p0 = ov_pos[e0];
-        const int bi = box_of_particle(a.boxes, a.nboxes, id0);
-        const BoxDesc& b = a.boxes[bi];
-        const uint32_t key = b.cell_base + storage_index(b, cell_of_wrapped(b, make_float3(p0.x, p0.y, p0.z)));
-        if (ov_head[key] != e0) continue;   // not the head of its cell's chain (or handled)
-        ov_head[key] = kChainDone;
-        const uint32_t raw = a.in_count[key];
-        const uint32_t m = min(raw, b.cap);
-        if (raw <= b.depth) continue;   // (an entry exists only past the depth)
-        Slot* const bucket = in_slots + b.slot_base + (uint64_t)(key - b.cell_base) * b.depth;
-        const uint32_t off = atomicAdd(&a.state->ext_count[par], m);
-        if (off > a.ext_cap - m) {   // no room: the cell keeps its bucket, the step kernels read only that
-            atomicOr(&a.state->error_flags, kErrExtensionFull);
-            bucket->pos.w = __uint_as_float(kNoExt);
-            continue;
+    const uint32_t n = min(a.state->ov[a.ov_in_slot].count, a.ov_cap);
+    const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (uint32_t)(kThreads / 32);
+    const uint32_t warp = (gridDim.x - 1u - blockIdx.x) * (uint32_t)(kThreads / 32) + (threadIdx.x >> 5);
+    const uint32_t per = min(32u, (n + warps - 1u) / warps);   // entries a warp looks at together
+    for (uint64_t first = (uint64_t)warp * per; first < n; first += (uint64_t)warps * per) {
+        // a lane looks at one entry: is it the head of its cell's chain, and which cell is that?
+        const uint32_t e = (uint32_t)first + lane;
+        int box = 0;
+        uint32_t key = 0;
+        bool head = false;
+        if (lane < per && e < n) {
+            const float4 p = ov_pos[e];
+            const uint32_t id = __float_as_uint(ov_vel[e].w);
+            if (id != kTakenId) {
+                box = box_of_particle(a.boxes, a.nboxes, id);
+                const BoxDesc& b = a.boxes[box];
+                key = b.cell_base + storage_index(b, cell_of_wrapped(b, make_float3(p.x, p.y, p.z)));
+                head = ov_head[key] == e;   // else: not the head, or handled
+                if (head) ov_head[key] = kChainDone;
+            }
         }
-        Slot* const ext = in_slots + a.total_slots + off;
-        for (uint32_t j = 0; j < b.depth; ++j) ext[j] = bucket[j];
-        uint32_t filled = b.depth, e = e0;
-        for (uint32_t t = b.depth; t < raw && e < a.ov_cap; ++t) {
-            const uint32_t before = a.ov_next_in[e];
-            const float4 pe = ov_pos[e], we = ov_vel[e];
-            if (filled < m) {
-                ext[filled].pos = pe;
-                ext[filled].vel = we;
-                ++filled;
-                ov_vel[e].w = __uint_as_float(kTakenId);
-            } else {
-                uint32_t jmax = 0, idmax = __float_as_uint(ext[0].vel.w);
-                for (uint32_t j = 1; j < m; ++j) {
-                    const uint32_t id = __float_as_uint(ext[j].vel.w);
-                    if (id > idmax) {
-                        idmax = id;
-                        jmax = j;
+        unsigned heads = __ballot_sync(kFull, head);
+        while (heads) {   // the warp handles one cell at a time
+            const int src = __ffs(heads) - 1;
+            heads &= heads - 1u;
+            const BoxDesc& b = a.boxes[__shfl_sync(kFull, box, src)];
+            const uint32_t cell = __shfl_sync(kFull, key, src);
+            const uint32_t raw = a.in_count[cell];
+            const uint32_t m = min(raw, b.cap), depth = b.depth;
+            if (raw <= depth) continue;   // (an entry exists only past the depth)
+            Slot* const bucket = in_slots + b.slot_base + (uint64_t)(cell - b.cell_base) * depth;
+            uint32_t off = 0;
+            if (lane == 0) off = atomicAdd(&a.state->ext_count[par], m);
+            off = __shfl_sync(kFull, off, 0);
+            if (off > a.ext_cap - m) {   // no room: the cell keeps its bucket, the step kernels read only that
+                if (lane == 0) {
+                    atomicAdd(&a.state->ov[a.ov_in_slot].left, raw - depth);
+                    atomicOr(&a.state->error_flags, kErrExtensionFull);
+                    bucket->pos.w = __uint_as_float(kNoExt);
+                }
+                continue;
+            }
+            Slot* const ext = in_slots + a.total_slots + off;
+            for (uint32_t j = lane; j < depth; j += 32) ext[j] = bucket[j];
+            __syncwarp();
+            uint32_t filled = depth, at = (uint32_t)first + (uint32_t)src;
+            for (uint32_t t = depth; t < raw && at < a.ov_cap; ++t) {
+                const uint32_t before = a.ov_next_in[at];
+                const float4 pe = ov_pos[at], we = ov_vel[at];
+                if (filled < m) {
+                    __syncwarp();   // every lane has read the entry
+                    if (lane == 0) {
+                        ext[filled].pos = pe;
+                        ext[filled].vel = we;
+                        ov_vel[at].w = __uint_as_float(kTakenId);
+                    }
+                    ++filled;
+                } else {   // the largest id of the set (ids are distinct) against the entry's
+                    __syncwarp();
+                    uint32_t idmax = 0, jmax = 0;
+                    for (uint32_t j = lane; j < m; j += 32) {
+                        const uint32_t id = __float_as_uint(ext[j].vel.w);
+                        if (id >= idmax) {
+                            idmax = id;
+                            jmax = j;
+                        }
+                    }
+                    const uint32_t top = __reduce_max_sync(kFull, idmax);
+                    const int owner = __ffs(__ballot_sync(kFull, idmax == top)) - 1;
+                    jmax = __shfl_sync(kFull, jmax, owner);
+                    if (lane == 0 && __float_as_uint(we.w) < top) {
+                        ov_pos[at] = ext[jmax].pos;
+                        ov_vel[at] = ext[jmax].vel;
+                        ext[jmax].pos = pe;
+                        ext[jmax].vel = we;
                     }
                 }
-                if (__float_as_uint(we.w) < idmax) {
-                    ov_pos[e] = ext[jmax].pos;
-                    ov_vel[e] = ext[jmax].vel;
-                    ext[jmax].pos = pe;
-                    ext[jmax].vel = we;
-                }
+                __syncwarp();
+                at = before;
             }
-            e = before;
+            if (lane == 0) {
+                bucket->pos.w = __uint_as_float(off);
+                if (raw > m) atomicAdd(&a.state->ov[a.ov_in_slot].left, raw - m);   // past the cap: they skip the collision
+            }
+            __syncwarp();
         }
-        bucket->pos.w = __uint_as_float(off);
     }
 }
 
@@ -1787,7 +1836,7 @@ __global__ void compact_overflow_kernel(const BoxDesc* boxes, int nboxes, const 
                                         uint64_t list_slot0, unsigned int* placed, uint32_t* out_cell,
                                         uint32_t* out_slot, uint32_t* out_prev, uint32_t* out_id)
 {
-    const uint32_t n = min(st->ov_count[parity], ov_cap);
+    const uint32_t n = min(st->ov[parity].count, ov_cap);
     const uint32_t base = offsets[cells];
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
         const uint32_t id = __float_as_uint(ov_vel[q].w);
@@ -2021,7 +2070,7 @@ static const StepFnRun kRunFns[2][2][3] = {
 bool run_kernel_takes(const StepArgs& a, int algorithm, bool table)
 {
     return algorithm == 0 && !table && !a.replay && (!a.tape_key || (a.nboxes == 1 && a.sample)) && !a.pressure &&
-           (a.ghosts || !a.total_walls) && (a.nboxes == 1 || (a.run_info && a.box_shifts)) &&
+           (a.ghosts || !a.total_walls) && a.box_shifts && (a.nboxes == 1 || a.run_info) &&
            a.boxes_n_max <= kRunMaxN;
 }
 

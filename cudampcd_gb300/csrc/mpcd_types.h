@@ -64,6 +64,8 @@ struct BoxDesc {
     uint64_t wall_base;    // first wall-ghost entry of this box (2 per column, with walls in z)
     uint32_t run_batch;    // srd_run_kernel: cells summed and finished together (4, 8 or 16)
     uint32_t depth;        // bucket slots per cell (<= cap)
+    uint32_t run_cells;    // srd_run_kernel: cells of a run (<= 32)
+    uint32_t unused[3];
 };
 
 // The step kernel copies a box descriptor into shared memory 16 bytes per thread.
@@ -90,11 +92,17 @@ struct alignas(32) SampleAcc {
     double n, vx, vy, vz;
 };
 
+// One overflow list: its entries, and those of them that the selection left to skip
+// the collision (it moved the others into their cells' extensions).
+struct alignas(8) OverflowFill {
+    unsigned int count, left;
+};
+
 // Device-resident bookkeeping shared by all launches of a handle.
 struct DeviceState {
     unsigned long long overflow_total;   // particles that found their bucket full
     unsigned int error_flags;            // kErr* bits
-    unsigned int ov_count[3];            // overflow list fill, by step modulo 3
+    OverflowFill ov[3];                  // overflow list fill, by step modulo 3
     // injected grid shifts (test hook), valid when inject_valid[i] != 0
     unsigned long long inject_step[kMaxInjectedShifts];
     float inject_shift[kMaxInjectedShifts][4];
@@ -150,7 +158,7 @@ struct StepArgs {
     float4* ov_out_pos;
     float4* ov_out_vel;
     uint32_t ov_cap;
-    uint32_t ov_in_slot, ov_out_slot, ov_zero_slot;   // indices into DeviceState::ov_count
+    uint32_t ov_in_slot, ov_out_slot, ov_zero_slot;   // indices into DeviceState::ov
     // overflow chains: per cell the list entry of the last particle that found the
     // cell's bucket full, per entry the one before it.  Heads alternate by step
     // parity and are never cleared: a step reads the head of a cell only when the
@@ -199,7 +207,7 @@ struct StepArgs {
     uint32_t run_class[4];        // runs [run_class[c], run_class[c+1]) take batches of 16, 8, 4 cells (c = 0, 1, 2)
     uint32_t boxes_n_max;         // the largest density of any box
     uint64_t total_walls;         // wall-ghost entries of all boxes
-    float4* box_shifts;           // ensembles: grid shifts of steps k and k+1 per box (drawn by the prologue)
+    float4* box_shifts;           // grid shifts of steps k and k+1 per box (drawn by the prologue of a run-kernel step)
     int32_t run_kernel;           // this step runs srd_run_kernel (the engine's choice, run_kernel_takes)
 };
 
