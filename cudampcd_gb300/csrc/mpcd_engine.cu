@@ -123,6 +123,7 @@ public:
         cudaDeviceProp prop;
         check(cudaGetDeviceProperties(&prop, (int)params_.device_id), "cudaGetDeviceProperties");
         sms_ = prop.multiProcessorCount;
+        run_grid_ = sms_ * 4;   // srd_run_kernel: 4 CTAs per SM
         set_runs();
         allocate();
         configure();
@@ -954,11 +955,24 @@ private:
 
     // Runs of srd_run_kernel: up to 32 cells of one box, {first cell, cells | box << 6},
     // listed by batch class (16, 8, then 4 cells per batch; one launch per class).
+    // The cells of a run: 32 where the sweep is long.  A box that fills the GPU's warps
+    // (32 per SM) only k < 8 times over takes the length that makes k full rounds of
+    // them, so that no warp sweeps a run more than another, and at least the cells of
+    // one pass of 32 particles.  Step us at 61 x 61 x 85, n = 7 (2.03 rounds of 32-cell
+    // runs), 33 x 47 x 29, n = 10 (0.29) and 16^3, n = 10 (0.03): 62.9 -> 57.2, 26.2 ->
+    // 17.7 and 22.8 -> 9.7 against 32-cell runs.
     void set_runs()
     {
+        const uint64_t warps = (uint64_t)run_grid_ * (kThreads / 32);
+        const uint64_t rounds = (cells_ + 32 * warps - 1) / (32 * warps);
+        const uint32_t even = rounds >= 8 ? 32u : (uint32_t)((cells_ + rounds * warps - 1) / (rounds * warps));
         run_info_.clear();
         for (BoxDesc& b : boxes_) {
-            b.run_cells = 32;
+            b.run_cells = std::min(32u, std::max(even, (32u + b.n - 1) / b.n));
+            if (const char* e = std::getenv("MPCD_GB_RUN_CELLS")) {   // tuning sweeps
+                const uint32_t v = (uint32_t)std::strtoul(e, nullptr, 10);
+                if (v >= 1 && v <= 32) b.run_cells = v;
+            }
         }
         for (int cls = 0; cls < 3; ++cls) {
             run_class_[cls] = (uint32_t)run_info_.size();
@@ -1156,7 +1170,7 @@ private:
             use_run_kernel_ghosts(a, false);
             if (sample && a.run_kernel) a.fold_samp = sample_buffer((uint64_t)i + 1);   // the other parity: step i-1's
             err = select_overflow(a, (uint64_t)i, cs);
-            if (err == cudaSuccess) err = launch_step(a, params_.algorithm, false, pbuf_, grid_, cs, &branches_);
+            if (err == cudaSuccess) err = launch_step(a, params_.algorithm, false, pbuf_, a.run_kernel ? run_grid_ : grid_, cs, &branches_);
             if (err == cudaSuccess && sample && !a.fold_samp)
                 err = launch_sample_finalize(a.samp, acc_.as<SampleAcc>(), cells_, 0, sms_ * 8, cs);
         }
@@ -1227,7 +1241,7 @@ private:
         if (sample && fold && a.run_kernel) a.fold_samp = sample_buffer(step_ + 1);
         check(select_overflow(a, step_, stream_), "overflow selection");
         if (before) check(cudaEventRecord(before, stream_), "event");
-        check(launch_step(a, params_.algorithm, use_table_, pbuf_, grid_, stream_, &branches_), "step kernel");
+        check(launch_step(a, params_.algorithm, use_table_, pbuf_, a.run_kernel ? run_grid_ : grid_, stream_, &branches_), "step kernel");
         if (after) check(cudaEventRecord(after, stream_), "event");
         last_step_table_ = use_table_;   // a replay of this step must consume the same draws
         use_table_ = false;
@@ -1286,7 +1300,7 @@ private:
             a.tape_ncell = tncell_.as<uint32_t>() + (size_t)i * cells_;
             use_run_kernel_ghosts(a, false);   // the run kernel records the tape of single-box SRD steps
             check(select_overflow(a, step_, stream_), "overflow selection");
-            check(launch_step(a, params_.algorithm, false, pbuf_, grid_, stream_), "tape step");
+            check(launch_step(a, params_.algorithm, false, pbuf_, a.run_kernel ? run_grid_ : grid_, stream_), "tape step");
             check(launch_sample_finalize(a.samp, acc_.as<SampleAcc>(), cells_, 1, sms_ * 8, stream_,
                                          tcnt_.as<uint32_t>() + (size_t)i * cells_),
                   "tape sample");
@@ -1386,7 +1400,7 @@ private:
     std::vector<mpcd_gb_params> box_params_;
     cudaStream_t own_stream_ = nullptr, stream_ = nullptr;
     RunBranches branches_;   // ensembles: side streams of the batch classes
-    int sms_ = 0, grid_ = 0;
+    int sms_ = 0, grid_ = 0, run_grid_ = 0;
     std::vector<BoxDesc> boxes_;
     uint64_t N_ = 0, cells_ = 0, tiles_ = 0, total_slots_ = 0, walls_ = 0;
     uint32_t ov_cap_ = 0, ext_cap_ = 0, pbuf_ = 0;

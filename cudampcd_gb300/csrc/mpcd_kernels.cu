@@ -2095,7 +2095,9 @@ cudaError_t launch_step(const StepArgs& a, int algorithm, bool table, uint32_t p
         for (int i = 0; i < nused; ++i) {
             const int cls = used[i];
             const StepFnRun f = a.tape_key ? kRunTapeFns[cls] : kRunFns[a.sample ? 1 : 0][a.nboxes == 1 ? 1 : 0][cls];
-            f<<<grid, kThreads, 0, fork && i > 0 ? branches->side[i - 1] : st>>>(a, a.run_class[cls],
+            const uint32_t runs = a.run_class[cls + 1] - a.run_class[cls];
+            const unsigned blocks = std::min((unsigned)grid, (runs + kRunWarps - 1) / (unsigned)kRunWarps);
+            f<<<blocks, kThreads, 0, fork && i > 0 ? branches->side[i - 1] : st>>>(a, a.run_class[cls],
                                                                                     a.run_class[cls + 1], i == 0);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
