@@ -123,7 +123,7 @@ public:
         cudaDeviceProp prop;
         check(cudaGetDeviceProperties(&prop, (int)params_.device_id), "cudaGetDeviceProperties");
         sms_ = prop.multiProcessorCount;
-        run_grid_ = sms_ * 4;   // srd_run_kernel: 4 CTAs per SM
+        run_grid_ = sms_ * run_blocks_per_sm(params_.algorithm);
         set_runs();
         allocate();
         configure();
@@ -944,7 +944,7 @@ private:
             b.tiles = (b.C + tc - 1) / tc;
             tiles += b.tiles;
             max_tile_cells_ = std::max(max_tile_cells_, tc);
-            for (uint32_t t = 0; t < b.tiles; ++t)
+            for (uint32_t t = 0; boxes_.size() > 1 && t < b.tiles; ++t)   // a single box computes its tiles
                 tile_info_.push_back({b.cell_base + t * tc, std::min(tc, b.C - t * tc) | (tc << 16), (uint32_t)r, 0u});
         }
         tiles_ = tiles;
@@ -963,28 +963,31 @@ private:
     // 17.7 and 22.8 -> 9.7 against 32-cell runs.
     void set_runs()
     {
-        const uint64_t warps = (uint64_t)run_grid_ * (kThreads / 32);
-        const uint64_t rounds = (cells_ + 32 * warps - 1) / (32 * warps);
+        const uint64_t warps = (uint64_t)run_grid_ * run_warps_per_block(params_.algorithm);
+        const uint64_t most = run_cells_max(params_.algorithm, n_max_);
+        const uint64_t rounds = (cells_ + most * warps - 1) / (most * warps);
         const uint32_t even = rounds >= 8 ? 32u : (uint32_t)((cells_ + rounds * warps - 1) / (rounds * warps));
         run_info_.clear();
+        num_runs_ = 0;
         for (BoxDesc& b : boxes_) {
-            b.run_cells = std::min(32u, std::max(even, (32u + b.n - 1) / b.n));
+            b.run_cells = std::min(run_cells_max(params_.algorithm, b.n), std::max(even, (32u + b.n - 1) / b.n));
             if (const char* e = std::getenv("MPCD_GB_RUN_CELLS")) {   // tuning sweeps
                 const uint32_t v = (uint32_t)std::strtoul(e, nullptr, 10);
-                if (v >= 1 && v <= 32) b.run_cells = v;
+                if (v >= 1 && v <= run_cells_max(params_.algorithm, b.n)) b.run_cells = v;
             }
         }
         for (int cls = 0; cls < 3; ++cls) {
-            run_class_[cls] = (uint32_t)run_info_.size();
+            run_class_[cls] = num_runs_;
             const uint32_t batch = 16u >> cls;
             for (size_t r = 0; r < boxes_.size(); ++r) {
                 const BoxDesc& b = boxes_[r];
-                if (b.run_batch != batch) continue;
-                for (uint32_t c = 0; c < b.C; c += b.run_cells)
+                if (params_.algorithm == 0 ? b.run_batch != batch : cls > 0) continue;   // extended: one class
+                num_runs_ += (b.C + b.run_cells - 1) / b.run_cells;
+                for (uint32_t c = 0; boxes_.size() > 1 && c < b.C; c += b.run_cells)   // a single box computes its runs
                     run_info_.push_back(make_uint2(b.cell_base + c, std::min(b.run_cells, b.C - c) | ((uint32_t)r << 6)));
             }
         }
-        run_class_[3] = (uint32_t)run_info_.size();
+        run_class_[3] = num_runs_;
     }
 
     void retile(double fill, uint32_t pbuf)
@@ -1000,6 +1003,7 @@ private:
     {
         check(cudaMemcpy(boxes_d_.p, boxes_.data(), sizeof(BoxDesc) * boxes_.size(), cudaMemcpyHostToDevice),
               "upload boxes");
+        if (boxes_.size() == 1) return;   // no tables
         const size_t bytes = sizeof(TileEntry) * tile_info_.size();
         if (tile_info_d_.bytes < bytes) check(tile_info_d_.alloc(bytes), "alloc tile table");
         check(cudaMemcpy(tile_info_d_.p, tile_info_.data(), bytes, cudaMemcpyHostToDevice), "upload tile table");
@@ -1091,7 +1095,7 @@ private:
         a.num_tiles = (uint32_t)tiles_;
         a.tile_info = tile_info_d_.as<TileEntry>();
         a.run_info = boxes_.size() > 1 ? run_info_d_.as<uint2>() : nullptr;
-        a.num_runs = (uint32_t)run_info_.size();
+        a.num_runs = num_runs_;
         for (int c = 0; c < 4; ++c) a.run_class[c] = run_class_[c];
         a.boxes_n_max = n_max_;
         a.total_walls = walls_;
@@ -1122,6 +1126,7 @@ private:
         a.samp = sample_buffer(k);
         a.acc = acc_.as<SampleAcc>();
         a.fold_samp = nullptr;
+        a.fold_cells = cells_;
         std::memcpy(a.ext_axis, ext_axis_, sizeof ext_axis_);
         a.draws = tables_;
         a.replay = replay ? 1 : 0;
@@ -1168,6 +1173,7 @@ private:
             a.step_base = step_base_ptr();
             a.sample = sample ? 1 : 0;
             use_run_kernel_ghosts(a, false);
+            graph_run_ = a.run_kernel;
             if (sample && a.run_kernel) a.fold_samp = sample_buffer((uint64_t)i + 1);   // the other parity: step i-1's
             err = select_overflow(a, (uint64_t)i, cs);
             if (err == cudaSuccess) err = launch_step(a, params_.algorithm, false, pbuf_, a.run_kernel ? run_grid_ : grid_, cs, &branches_);
@@ -1198,6 +1204,7 @@ private:
         const int done = reps * kGraphSteps;
         step_ += (uint64_t)done;
         last_step_table_ = false;
+        last_step_run_ = graph_run_;
         dense_valid_ = false;
         return done;
     }
@@ -1226,7 +1233,7 @@ private:
     // draws the ghosts), else none.
     void use_run_kernel_ghosts(StepArgs& a, bool table) const
     {
-        a.run_kernel = run_kernel_takes(a, params_.algorithm, table) ? 1 : 0;
+        a.run_kernel = run_kernel_takes(a, params_.algorithm, table) ? (params_.algorithm ? kRunExtended : kRunSrd) : 0;
     }
 
     // One step: the overflow selection, then the step kernel (bracketed by the
@@ -1243,6 +1250,7 @@ private:
         if (before) check(cudaEventRecord(before, stream_), "event");
         check(launch_step(a, params_.algorithm, use_table_, pbuf_, a.run_kernel ? run_grid_ : grid_, stream_, &branches_), "step kernel");
         if (after) check(cudaEventRecord(after, stream_), "event");
+        last_step_run_ = a.run_kernel;
         last_step_table_ = use_table_;   // a replay of this step must consume the same draws
         use_table_ = false;
         ++step_;
@@ -1258,7 +1266,10 @@ private:
         if (!dense_valid_) {
             if (step_ == 0) throw Error(MPCD_GB_ESTATE, "no state to read");
             StepArgs a = args(step_ - 1, true);
-            check(launch_step(a, params_.algorithm, last_step_table_, pbuf_, grid_, stream_), "replay");
+            // the extended run kernel replays its own steps (from the prologue's ghost counts and shifts)
+            if (last_step_run_ == kRunExtended) a.run_kernel = kRunExtended;
+            check(launch_step(a, params_.algorithm, last_step_table_, pbuf_, a.run_kernel ? run_grid_ : grid_, stream_),
+                  "replay");
             check(cudaStreamSynchronize(stream_), "replay");
             check_device_errors();
             dense_valid_ = true;
@@ -1304,6 +1315,7 @@ private:
             check(launch_sample_finalize(a.samp, acc_.as<SampleAcc>(), cells_, 1, sms_ * 8, stream_,
                                          tcnt_.as<uint32_t>() + (size_t)i * cells_),
                   "tape sample");
+            last_step_run_ = a.run_kernel;
             ++step_;
         }
         last_step_table_ = false;
@@ -1414,6 +1426,7 @@ private:
     DeviceBuffer mean_;   // mean fields of a read (4 floats per cell)
     bool use_table_ = false;
     bool last_step_table_ = false;
+    int32_t last_step_run_ = 0, graph_run_ = 0;   // StepArgs::run_kernel of the last step, of the step graphs
     bool dense_valid_ = false;   // dense_pos_ / dense_vel_ hold the state after step step_ - 1
     DrawTables tables_{};
     int inject_valid_[kMaxInjectedShifts] = {0, 0, 0, 0};
@@ -1422,7 +1435,7 @@ private:
     std::vector<TileEntry> tile_info_;   // tile table of the current tiling
     DeviceBuffer tile_info_d_;
     std::vector<uint2> run_info_;        // run table of srd_run_kernel
-    uint32_t run_class_[4] = {0, 0, 0, 0};
+    uint32_t run_class_[4] = {0, 0, 0, 0}, num_runs_ = 0;
     DeviceBuffer run_info_d_;
     uint32_t n_max_ = 0;
     DeviceBuffer ov_head_[2], ov_next_[2];   // overflow chains: heads by cell, links by entry (by step parity)

@@ -374,9 +374,9 @@ struct Draws<false> {   // Philox (production)
     __device__ static float thermal(const StepArgs&, const BoxDesc& b, uint64_t step, uint32_t ref, uint32_t i)
     {
         const uint4 o = draw(b, step, kThermal, ref, i >> 2);
+        const bool second = (i & 2u) != 0;   // the inputs selected, not the results: lanes of a warp differ in i
         float g0, g1;
-        if (((i & 3u) >> 1) == 0) box_muller(o.x, o.y, g0, g1);
-        else box_muller(o.z, o.w, g0, g1);
+        box_muller(second ? o.z : o.x, second ? o.w : o.y, g0, g1);
         return (i & 1u) ? g1 : g0;
     }
 };
@@ -541,7 +541,7 @@ __device__ __forceinline__ uint32_t fetch_count(const StepArgs& a, uint32_t firs
 __device__ void overflow_pass(const StepArgs& a, uint64_t step)
 {
     const uint32_t n = min(a.state->ov[a.ov_in_slot].count, a.ov_cap);
-    for (uint32_t base = blockIdx.x * kThreads; base < n; base += gridDim.x * kThreads) {
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         const uint32_t q = base + threadIdx.x;
         const float4 w = q < n ? a.ov_in_vel[q] : make_float4(0, 0, 0, 0);
         const bool active = q < n && __float_as_uint(w.w) != kTakenId;
@@ -1469,6 +1469,433 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
     }
 }
 
+// ------------------------------------------------------------------ extended run kernel
+//
+// The production step of the extended collision and its replays (Philox draws, n <=
+// kExtMaxN; the tile kernel keeps injected draws, denser boxes and the pressure
+// estimator), one box or an ensemble: one warp per run of consecutive cells
+// (storage order), alone with 9.2 KB of shared memory, no CTA-wide barrier.  A run
+// is as many cells as hold about 160 particles.  Per run, in parts when its entries
+// do not fit the buffer:
+//   lane = cell: count, source, wall ghosts (counted by the prologue), axis and gate;
+//   one bulk copy per cell brings its particles into shared memory; each particle
+//   counts its rank among the cell's ids, which gives the cell's id order;
+//   the ghosts, one lane each;
+//   4 lanes per cell: centre of mass, mean velocity, the projections on the axis and
+//   the gate, in the tile kernel's order (rank k adds to partial k mod 4, the four
+//   partials in a fixed tree), so that either kernel replays the other bit by bit;
+//   the colliding cells, about one in seven, one at a time by the whole warp: a lane
+//   per participant for its draws and terms, a lane per sum and partial for the 11
+//   ordered sums;
+//   the particles again, 32 a pass: unshift, drag, sample, streaming of step k+1 and
+//   its cell, left in the buffer; then every slot claim, then every store.
+// What bounds it is instruction issue and latency.  The tile kernel spends 33.6 warp
+// instructions a particle at n = 20: four lanes of each colliding cell draw and sum
+// while the warp's other cells wait, ranks are looked up in every pass, and five
+// CTA-wide barriers a tile stall its warps.  This kernel: 26 a particle, 64 % issue.  256 x 256 x 66, n = 20 (8.2e7 particles), us a step:
+// tile kernel 3459, this one 2656; sampled 3677 and 2954.  Its code size matters: with
+// the passes over a part unrolled it no longer fit the instruction cache and took
+// 10700 us; with the compiler's own unrolling of the inner loops 3280.
+
+constexpr uint32_t kExtBuf = 184;                  // entries (particles and ghosts) of a part
+constexpr uint32_t kExtCells = 24;                 // cells of a run at most
+constexpr int kExtThreads = 128;
+constexpr int kExtWarps = kExtThreads / 32;
+constexpr int kExtBlocks = 6;                      // CTAs per SM: 24 warps of up to 80 registers
+constexpr uint32_t kTermRow = 36;                  // 4 (sum) + (participant) then covers the banks
+static_assert(kExtBuf >= 5 * kExtMaxN, "a cell's 4n colliding particles and n ghosts fit the buffer");
+
+struct ExtShared {                   // one per warp
+    Slot buf[kExtBuf];               // by cell, ghosts after its particles; in the end the streamed state
+    union {
+        uint32_t ids[kExtBuf + 3 * kExtCells];   // of the particles, each cell's padded to a multiple of 4
+        float term[11][kTermRow];                // a colliding cell's terms, by sum and participant
+    };
+    float4 mean[kExtCells];          // mean velocity; w: entries of the collision
+    float4 com[kExtCells];           // centre of mass; w: 1 in a cell that collided
+    float4 omega[kExtCells];         // axis and gate, then the rotation; w: participants that move
+    uint64_t bar;
+    uint8_t cell[kExtBuf];           // of an entry, kExtGhost on ghosts
+    uint8_t rank[kExtBuf];           // of a particle within its cell
+    uint8_t order[kExtBuf];          // a cell's particles by rank
+};
+constexpr uint32_t kExtGhost = 0x80u;
+
+// The last lane-ordered cell whose range starts at or before t: end = inclusive ends by lane.
+__device__ __forceinline__ uint32_t cell_of_entry(uint32_t t, uint32_t end)
+{
+    uint32_t i = 0;
+#pragma unroll
+    for (uint32_t half = 16; half; half >>= 1) i += t >= __shfl_sync(kFull, end, (int)(i + half - 1)) ? half : 0u;
+    return i;
+}
+
+template <bool SAMPLE, bool SINGLE, bool REPLAY>
+__global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const StepArgs a)
+{
+    extern __shared__ __align__(128) unsigned char dyn[];
+    __shared__ __align__(16) BoxDesc shared_box[SINGLE ? 1 : kExtWarps];
+    const uint32_t lane = threadIdx.x & 31u;
+    ExtShared& sh = reinterpret_cast<ExtShared*>(dyn)[threadIdx.x >> 5];
+    BoxDesc& sbox = shared_box[SINGLE ? 0 : threadIdx.x >> 5];
+    const uint64_t step = a.step_base ? *a.step_base + a.step : a.step;   // graph replays read the base
+    const uint32_t left = a.state->ov[a.ov_in_slot].left;
+    const BoxDesc& b = SINGLE ? a.box0 : sbox;
+    float3 s = make_float3(0, 0, 0), sn = s;
+    if (SINGLE) {
+        const float4 s0 = __ldg(a.box_shifts), s1 = __ldg(a.box_shifts + 1);   // drawn by the prologue
+        s = make_float3(s0.x, s0.y, s0.z);
+        sn = make_float3(s1.x, s1.y, s1.z);
+    }
+    if (!REPLAY && blockIdx.x == 0 && threadIdx.x == 0)   // list of step k-1, refilled by step k+1
+        a.state->ov[a.ov_zero_slot] = OverflowFill{0u, 0u};
+    if (left) overflow_pass(a, step);
+    if (lane == 0) mbar_init(&sh.bar);
+    __syncwarp();
+    uint32_t phase = 0;
+    int cur_box = -1;
+    const uint32_t warps = gridDim.x * (uint32_t)kExtWarps;
+    uint32_t run = blockIdx.x * (uint32_t)kExtWarps + (threadIdx.x >> 5);
+    uint2 next = run_entry<SINGLE>(a, run);
+    uint32_t raw_next = lane < (next.y & 63u) ? a.in_count[next.x + lane] : 0u;   // counts one run ahead
+    uint64_t fold = 32ull * run + lane;   // sampled steps: the cell whose previous sample this lane folds next
+
+    for (; run < a.num_runs; run += warps) {
+        const uint2 cur = next;
+        if (!SINGLE && (int)(cur.y >> 6) != cur_box) {   // box and grid shifts
+            cur_box = (int)(cur.y >> 6);
+            __syncwarp();
+            if (lane < sizeof(BoxDesc) / 16)
+                reinterpret_cast<uint4*>(&sbox)[lane] = __ldg(reinterpret_cast<const uint4*>(a.boxes + cur_box) + lane);
+            const float4 s0 = __ldg(a.box_shifts + 2 * cur_box), s1 = __ldg(a.box_shifts + 2 * cur_box + 1);
+            s = make_float3(s0.x, s0.y, s0.z);
+            sn = make_float3(s1.x, s1.y, s1.z);
+            __syncwarp();
+        }
+        const bool sign = s.z > 0;
+        const uint32_t cells = cur.y & 63u;
+        const uint32_t c0 = cur.x - b.cell_base;   // box-local first cell
+        const bool valid = lane < cells;
+        const Slot* src_lane;
+        const uint32_t cnt = cell_source(a, b, a.in_slots, c0 + lane, raw_next, src_lane);
+        const uint32_t src_slot = (uint32_t)(src_lane - a.in_slots);
+        if (!REPLAY && valid) a.zero_count[cur.x + lane] = 0;   // counts of step k-1: step k+1 fills them
+        next = run_entry<SINGLE>(a, run + warps);
+        raw_next = lane < (next.y & 63u) ? a.in_count[next.x + lane] : 0u;
+        uint32_t ng = 0, ref;   // wall ghosts and reference index of the lane's cell
+        {
+            const uint3 cc = storage_coords(b, valid ? c0 + lane : 0u);
+            ref = ref_index(b, cc);
+            bool layer, wall;
+            wall_layer(b, cc.z, sign, layer, wall);
+            if (wall && valid)
+                ng = a.ghosts[b.wall_base + 2u * (cc.x + (uint32_t)b.L[0] * cc.y) + (cc.z == (uint32_t)sign ? 0u : 1u)].n;
+        }
+        // ends over the run's cells: entries, real particles, padded ids
+        const uint32_t padded = (cnt + 3u) & ~3u;
+        uint32_t end_e = cnt + ng, end_r = cnt, end_i = padded;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t e = __shfl_up_sync(kFull, end_e, d), r = __shfl_up_sync(kFull, end_r, d),
+                           q = __shfl_up_sync(kFull, end_i, d);
+            if ((int)lane >= d) {
+                end_e += e;
+                end_r += r;
+                end_i += q;
+            }
+        }
+
+        for (uint32_t i0 = 0; i0 < cells;) {   // cells [i0, i1) whose entries fit the buffer
+            const uint32_t e0 = __shfl_sync(kFull, end_e - (cnt + ng), (int)i0);
+            const uint32_t r0 = __shfl_sync(kFull, end_r - cnt, (int)i0);
+            const uint32_t q0 = __shfl_sync(kFull, end_i - padded, (int)i0);
+            const uint32_t i1 = min(cells, (uint32_t)__popc(__ballot_sync(kFull, lane < i0 || end_e - e0 <= kExtBuf)));
+            const uint32_t total = __shfl_sync(kFull, end_e, (int)i1 - 1) - e0;
+            const uint32_t real = __shfl_sync(kFull, end_r, (int)i1 - 1) - r0;
+            // first entry, first id and count of the lane's cell: 8, 9 and 8 bits
+            const uint32_t first_e = end_e - (cnt + ng) - e0, first_i = end_i - padded - q0;
+            const uint32_t range = (first_e & 0xFFu) | (first_i & 0x1FFu) << 8 | cnt << 17;
+            const bool mine = lane >= i0 && lane < i1;
+            fence_proxy_async();   // the buffer's earlier reads and writes, before the copies
+            __syncwarp();
+            if (lane == 0 && real) mbar_arrive_expect_tx(&sh.bar, real * (uint32_t)sizeof(Slot));
+            __syncwarp();
+            if (mine && cnt) bulk_g2s(sh.buf + first_e, a.in_slots + src_slot, cnt * (uint32_t)sizeof(Slot), &sh.bar);
+            if (mine) {
+                float gate = 1.0f;
+                const float3 ax = Draws<false>::ext_axis(a, b, step, ref, gate);
+                sh.omega[lane] = make_float4(ax.x, ax.y, ax.z, gate);
+#pragma unroll 1
+                for (uint32_t q = cnt; q < padded; ++q) sh.ids[first_i + q] = 0xFFFFFFFFu;
+            }
+            // the previous step's sample of 32 cells into the FP64 sums, while the copies are under way
+            if (SAMPLE && a.fold_samp && fold < a.fold_cells) {
+                fold_sample(a.fold_samp, a.acc, fold, 0, nullptr);
+                fold += 32ull * warps;
+            }
+            // ghosts after each cell's particles, one lane each
+            for (uint32_t g0 = 0; g0 < total - real; g0 += 32) {
+                const uint32_t t = e0 - r0 + min(g0 + lane, total - real - 1u);
+                const uint32_t i = cell_of_entry(t, end_e - end_r);
+                const uint32_t before = __shfl_sync(kFull, end_e - ng - e0, (int)i);   // entries before the cell's ghosts
+                const uint32_t j = t - __shfl_sync(kFull, end_e - end_r - ng, (int)i);
+                const uint3 cc = storage_coords(b, c0 + i);
+                bool layer, wall;
+                wall_layer(b, cc.z, sign, layer, wall);
+                float3 gx, gv;
+                Draws<false>::ghost(a, b, step, ref_index(b, cc), j, cell_centre(b, cc), fabsf(s.z), layer, sign, gx, gv);
+                if (g0 + lane < total - real) {
+                    sh.buf[before + j].pos = make_float4(gx.x, gx.y, gx.z, 0.0f);
+                    sh.buf[before + j].vel = make_float4(gv.x, gv.y, gv.z, 0.0f);
+                }
+            }
+            if (real) {
+                if (!mbar_wait_bounded(&sh.bar, phase)) {
+                    if (lane == 0) atomicOr(&a.state->error_flags, kErrWaitTimeout);
+                    mbar_wait_bounded(&sh.bar, phase);   // let copies in flight land
+                    return;
+                }
+                phase ^= 1u;
+            }
+            // the cell of every entry and the particles' ids side by side, 4 lanes per cell
+#pragma unroll 1
+            for (uint32_t r = i0; r < i1; r += 8) {
+                const uint32_t i = r + (lane >> 2);
+                const uint32_t at = __shfl_sync(kFull, range, (int)(i & 31u)), g = __shfl_sync(kFull, ng, (int)(i & 31u));
+                const uint32_t o = at & 0xFFu, n = at >> 17, end = i < i1 ? n + g : 0u;
+#pragma unroll 1
+                for (uint32_t k = lane & 3u; k < end; k += 4) {
+                    sh.cell[o + k] = (uint8_t)(i | (k < n ? 0u : kExtGhost));
+                    if (k < n) sh.ids[(at >> 8 & 0x1FFu) + k] = __float_as_uint(sh.buf[o + k].vel.w);
+                }
+            }
+            __syncwarp();
+            // ranks: the cell's ids below the particle's own
+#pragma unroll 1
+            for (uint32_t p0 = 0; p0 < total; p0 += 32) {
+                const uint32_t p = min(p0 + lane, total - 1u);
+                const uint32_t info = sh.cell[p];
+                const uint32_t at = __shfl_sync(kFull, range, (int)(info & 31u));
+                const uint32_t id = __float_as_uint(sh.buf[p].vel.w), n = at >> 17;
+                const uint4* const q = reinterpret_cast<const uint4*>(sh.ids + (at >> 8 & 0x1FFu));
+                uint32_t rank = 0;
+#pragma unroll 1
+                for (uint32_t k = 0; 4 * k < n; ++k) {
+                    const uint4 w = q[k];
+                    rank += (w.x < id) + (w.y < id) + (w.z < id) + (w.w < id);
+                }
+                if (p0 + lane < total && !(info & kExtGhost)) {
+                    sh.rank[p] = (uint8_t)rank;
+                    sh.order[(at & 0xFFu) + rank] = (uint8_t)p;
+                }
+            }
+            __syncwarp();
+
+            // collision quantities, 4 lanes per cell, 8 cells at a time
+            for (uint32_t r = i0; r < i1; r += 8) {
+                const uint32_t i = r + (lane >> 2), j = lane & 3u;
+                const bool in_part = i < i1;
+                const uint32_t o = __shfl_sync(kFull, end_e - (cnt + ng) - e0, (int)(i & 31u));
+                const uint32_t real_n = __shfl_sync(kFull, cnt, (int)(i & 31u)), g = __shfl_sync(kFull, ng, (int)(i & 31u));
+                const uint32_t n = in_part ? min(real_n + g, b.cap) : 0u;
+                const uint32_t m = n - min(g, n);   // real participants (lowest ids)
+                const uint32_t gap = o + real_n - m;   // participant k >= m: the ghost in entry gap + k
+                const bool live = n > 1;
+                const uint3 cc = storage_coords(b, c0 + (in_part ? i : 0u));
+                const float3 centre = cell_centre(b, cc);
+                const float4 axg = sh.omega[in_part ? i : i0];
+                const float3 axis = make_float3(axg.x, axg.y, axg.z);
+                float3 com = make_float3(0, 0, 0), mean = make_float3(0, 0, 0);
+#pragma unroll 1
+                for (uint32_t k = j; live && k < n; k += 4) {
+                    const uint32_t p = k < m ? sh.order[o + k] : gap + k;
+                    const float4 xp = sh.buf[p].pos, vp = sh.buf[p].vel;
+                    com.x += (xp.x - centre.x); com.y += (xp.y - centre.y); com.z += (xp.z - centre.z);
+                    mean.x += vp.x; mean.y += vp.y; mean.z += vp.z;
+                }
+                com = make_float3(group_sum(com.x, 4), group_sum(com.y, 4), group_sum(com.z, 4));
+                mean = make_float3(group_sum(mean.x, 4), group_sum(mean.y, 4), group_sum(mean.z, 4));
+                const float inv = live ? 1.0f / (float)n : 0.0f;
+                com = make_float3(com.x * inv + centre.x, com.y * inv + centre.y, com.z * inv + centre.z);
+                mean = make_float3(mean.x * inv, mean.y * inv, mean.z * inv);
+                // projections on the axis of the side below the plane through the centre of mass
+                float proj0 = 0.0f;
+                int size0 = 0;
+#pragma unroll 1
+                for (uint32_t k = j; live && k < n; k += 4) {
+                    const uint32_t p = k < m ? sh.order[o + k] : gap + k;
+                    const float4 xp = sh.buf[p].pos, vp = sh.buf[p].vel;
+                    if (dot3(make_float3(xp.x - com.x, xp.y - com.y, xp.z - com.z), axis) < 0) {
+                        proj0 += dot3(make_float3(vp.x - mean.x, vp.y - mean.y, vp.z - mean.z), axis);
+                        size0 += 1;
+                    }
+                }
+                proj0 = group_sum(proj0, 4);
+                size0 = group_sum(size0, 4);
+                const int size1 = (int)n - size0;
+                const float proj1 = live ? -proj0 / (float)size1 : 0.0f;
+                proj0 = live ? proj0 / (float)size0 : 0.0f;
+                const float prob = live ? 1 - expf(0.01f * (proj1 - proj0) * (float)size0 * (float)size1) : 0.0f;
+                const bool collide = live && axg.w < prob;
+                if (in_part && j == 0) {
+                    sh.mean[i] = make_float4(mean.x, mean.y, mean.z, __uint_as_float(n));
+                    sh.com[i] = make_float4(com.x, com.y, com.z, __uint_as_float(collide ? 1u : 0u));
+                    if (!collide) sh.omega[i] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(m));
+                }
+                __syncwarp();
+                // the colliding cells, one at a time by the whole warp
+                for (unsigned todo = __ballot_sync(kFull, collide && j == 0); todo; todo &= todo - 1u) {
+                    const int src = __ffs(todo) - 1;
+                    const uint32_t ci = r + ((uint32_t)src >> 2);
+                    const uint32_t co = __shfl_sync(kFull, o, src), cn = __shfl_sync(kFull, n, src),
+                                   cm = __shfl_sync(kFull, m, src), cgap = __shfl_sync(kFull, gap, src);
+                    const uint32_t cref = __shfl_sync(kFull, ref, (int)ci);
+                    const int s0 = __shfl_sync(kFull, size0, src), s1 = (int)cn - s0;
+                    // stochastic exchange along the axis, thermalised per side
+                    const float t0 = __shfl_sync(kFull, proj1, src) * ((float)s1 / (float)s0);
+                    const float t1 = __shfl_sync(kFull, proj0, src) * ((float)s0 / (float)s1);
+                    const float4 mv = sh.mean[ci], cv = sh.com[ci], av = sh.omega[ci];
+                    const float3 ax = make_float3(av.x, av.y, av.z);
+                    float sum0 = 0.0f, sum1 = 0.0f;   // lane 4 q + j: partial j of sum q (side means, inertia), of sum 8 + q (dL)
+                    const uint32_t q = lane >> 2;
+#pragma unroll 1
+                    for (uint32_t k0 = 0; k0 < cn; k0 += 32) {
+                        const uint32_t k = k0 + lane;
+                        if (k < cn) {
+                            const uint32_t p = k < cm ? sh.order[co + k] : cgap + k;
+                            const float4 xp = sh.buf[p].pos, vp = sh.buf[p].vel;
+                            const float3 x = make_float3(xp.x - cv.x, xp.y - cv.y, xp.z - cv.z);
+                            float3 v = make_float3(vp.x - mv.x, vp.y - mv.y, vp.z - mv.z);
+                            const bool sd = dot3(x, ax) < 0;
+                            const float vr = Draws<false>::thermal(a, b, step, cref, k) * b.tv;
+                            const float3 cr = cross3(x, v);
+                            const float kick = (vr - dot3(v, ax)) + (sd ? t0 : t1);
+                            v.x += ax.x * kick; v.y += ax.y * kick; v.z += ax.z * kick;
+                            sh.buf[p].vel = make_float4(v.x, v.y, v.z, vp.w);
+                            const float sx = x.x * x.x, sy = x.y * x.y, sz = x.z * x.z;
+                            sh.term[0][lane] = sd ? vr : 0.0f;   // adding +0 changes no partial (none is -0)
+                            sh.term[1][lane] = sd ? 0.0f : vr;
+                            sh.term[2][lane] = sy + sz;
+                            sh.term[3][lane] = sx + sz;
+                            sh.term[4][lane] = sx + sy;
+                            sh.term[5][lane] = -x.x * x.y;
+                            sh.term[6][lane] = -x.x * x.z;
+                            sh.term[7][lane] = -x.y * x.z;
+                            sh.term[8][lane] = cr.x;
+                            sh.term[9][lane] = cr.y;
+                            sh.term[10][lane] = cr.z;
+                        }
+                        __syncwarp();
+#pragma unroll 1
+                        for (uint32_t t = j; t < min(32u, cn - k0); t += 4) {
+                            sum0 += sh.term[q][t];
+                            if (q < 3) sum1 += sh.term[8 + q][t];
+                        }
+                        __syncwarp();
+                    }
+                    const float all0 = group_sum(sum0, 4);
+                    const float m0 = __shfl_sync(kFull, all0, 0) / (float)s0, m1 = __shfl_sync(kFull, all0, 4) / (float)s1;
+                    float I[6];
+#pragma unroll
+                    for (int w = 0; w < 6; ++w) I[w] = __shfl_sync(kFull, all0, 4 * (w + 2));
+                    const float3 vm0 = make_float3(ax.x * m0, ax.y * m0, ax.z * m0);
+                    const float3 vm1 = make_float3(ax.x * m1, ax.y * m1, ax.z * m1);
+#pragma unroll 1
+                    for (uint32_t k0 = 0; k0 < cn; k0 += 32) {
+                        const uint32_t k = k0 + lane;
+                        if (k < cn) {
+                            const uint32_t p = k < cm ? sh.order[co + k] : cgap + k;
+                            const float4 xp = sh.buf[p].pos;
+                            float4 vp = sh.buf[p].vel;
+                            const float3 x = make_float3(xp.x - cv.x, xp.y - cv.y, xp.z - cv.z);
+                            const float3 vm = dot3(x, ax) < 0 ? vm0 : vm1;
+                            vp.x -= vm.x; vp.y -= vm.y; vp.z -= vm.z;
+                            sh.buf[p].vel = vp;
+                            const float3 cr = cross3(x, make_float3(vp.x, vp.y, vp.z));
+                            sh.term[0][lane] = cr.x;
+                            sh.term[1][lane] = cr.y;
+                            sh.term[2][lane] = cr.z;
+                        }
+                        __syncwarp();
+                        if (q < 3)
+#pragma unroll 1
+                            for (uint32_t t = j; t < min(32u, cn - k0); t += 4) sum1 -= sh.term[q][t];
+                        __syncwarp();
+                    }
+                    const float all1 = group_sum(sum1, 4);
+                    const float3 dL = make_float3(__shfl_sync(kFull, all1, 0), __shfl_sync(kFull, all1, 4), __shfl_sync(kFull, all1, 8));
+                    float Ii[6];
+                    sym_inverse(I, 1e-5f, Ii);
+                    if (lane == 0)
+                        sh.omega[ci] = make_float4(Ii[0] * dL.x + Ii[3] * dL.y + Ii[4] * dL.z,
+                                                   Ii[3] * dL.x + Ii[1] * dL.y + Ii[5] * dL.z,
+                                                   Ii[4] * dL.x + Ii[5] * dL.y + Ii[2] * dL.z, __uint_as_float(cm));
+                }
+            }
+            __syncwarp();
+
+            // the particles, 32 a pass: finish the collision, sample, stream step k+1, claim a
+            // slot in the next cell; a pass is stored after the next one's claims are issued
+            uint32_t held_key = kNoKey, held_peers = 0, held_base = 0, held_p = 0;
+            auto store_held = [&]() {
+                const uint32_t at = __shfl_sync(kFull, held_base, __ffs(held_peers) - 1) + __popc(held_peers & lanemask_lt());
+                if (held_key == kNoKey) return;
+                const float4 xq = sh.buf[held_p].pos, vq = sh.buf[held_p].vel;
+                const uint32_t index = (uint32_t)b.slot_base + (held_key - b.cell_base) * b.depth + at;
+                if (at < b.depth) store_slot(a.out_slots + index, xq, vq);
+                else push_overflow(a, held_key, xq, vq);
+            };
+#pragma unroll 1
+            for (uint32_t p0 = 0; p0 < total; p0 += 32) {
+                const uint32_t p = min(p0 + lane, total - 1u);
+                const uint32_t info = sh.cell[p], i = info & 31u;
+                const bool active = p0 + lane < total && !(info & kExtGhost);
+                const float4 xp = sh.buf[p].pos, vp = sh.buf[p].vel;
+                const float4 k0 = sh.mean[i], k1 = sh.com[i], k2 = sh.omega[i];
+                float3 x = make_float3(xp.x, xp.y, xp.z), v = make_float3(vp.x, vp.y, vp.z);
+                if (__float_as_uint(k0.w) > 1 && sh.rank[p] < __float_as_uint(k2.w)) {
+                    const float3 xr = make_float3(x.x - k1.x, x.y - k1.y, x.z - k1.z);
+                    if (!__float_as_uint(k1.w)) { v.x -= k0.x; v.y -= k0.y; v.z -= k0.z; }
+                    v.x += k0.x; v.y += k0.y; v.z += k0.z;
+                    v.x += b.drag_dt;
+                    const float3 cr = cross3(xr, make_float3(k2.x, k2.y, k2.z));
+                    v.x -= cr.x; v.y -= cr.y; v.z -= cr.z;
+                    // com + xr rebuilds the wrapped staged position to within rounding
+                    x = pbc_near(b, make_float3((k1.x + xr.x) - s.x, (k1.y + xr.y) - s.y, (k1.z + xr.z) - s.z));
+                }
+                if (REPLAY) {
+                    if (active) {
+                        const uint64_t i3 = 3 * (uint64_t)__float_as_uint(vp.w);
+                        a.dense_pos[i3] = x.x; a.dense_pos[i3 + 1] = x.y; a.dense_pos[i3 + 2] = x.z;
+                        a.dense_vel[i3] = v.x; a.dense_vel[i3 + 1] = v.y; a.dense_vel[i3 + 2] = v.z;
+                    }
+                    continue;
+                }
+                float3 vn = v;
+                const float3 xn = stream_shift(b, x, vn, sn);
+                const uint32_t key = active ? b.cell_base + storage_index(b, cell_of_wrapped(b, xn)) : kNoKey;
+                if (SAMPLE) {
+                    const uint32_t lab = b.cell_base + storage_index(b, cell_of_wrapped(b, x));
+                    sample_add(a.samp, lab, v, active);
+                }
+                __syncwarp();   // idle lanes have read the part's last entry
+                if (active) {
+                    sh.buf[p].pos = make_float4(xn.x, xn.y, xn.z, __uint_as_float(kNoExt));
+                    sh.buf[p].vel = make_float4(vn.x, vn.y, vn.z, vp.w);
+                }
+                const unsigned peers = __match_any_sync(kFull, key);
+                uint32_t base = 0;
+                if (active && (int)lane == __ffs(peers) - 1) base = atomicAdd(a.out_count + key, (uint32_t)__popc(peers));
+                if (p0) store_held();
+                held_key = key; held_peers = peers; held_base = base; held_p = p;
+            }
+            if (!REPLAY && total) store_held();
+            __syncwarp();   // the next part rewrites this warp's shared arrays
+            i0 = i1;
+        }
+    }
+}
+
 // Before step k: every cell that received more particles than its bucket
 // holds (raw count > depth) gets its colliding set -- all raw particles, or the
 // cap lowest ids when raw > cap, whatever order the claims of step k-1 arrived
@@ -1539,7 +1966,7 @@ __global__ void __launch_bounds__(kThreads) overflow_select_kernel(const StepArg
                     if (4 * chunk + k < b.n && ((u01(u[k]) > shift_abs) ^ layer ^ sign)) ++g;
             }
             GhostSum r{0, 0, 0, g, 0u};
-            if (g) {
+            if (g && a.run_kernel == kRunSrd) {   // the extended collision draws them one by one
                 const float3 v = ghost_sum_velocity(b, step, ref, g);
                 r.sx = fixed24(v.x);
                 r.sy = fixed24(v.y);
@@ -2067,8 +2494,17 @@ static const StepFnRun kRunFns[2][2][3] = {
     {{srd_run_kernel<true, false, 16>, srd_run_kernel<true, false, 8>, srd_run_kernel<true, false, 4>},
      {srd_run_kernel<true, true, 16>, srd_run_kernel<true, true, 8>, srd_run_kernel<true, true, 4>}}};
 
+using StepFnExt = void (*)(const StepArgs);
+// [sample][single box]; replays by single box
+static const StepFnExt kExtFns[2][2] = {{ext_run_kernel<false, false, false>, ext_run_kernel<false, true, false>},
+                                        {ext_run_kernel<true, false, false>, ext_run_kernel<true, true, false>}};
+static const StepFnExt kExtReplayFns[2] = {ext_run_kernel<false, false, true>, ext_run_kernel<false, true, true>};
+
 bool run_kernel_takes(const StepArgs& a, int algorithm, bool table)
 {
+    if (algorithm == 1)
+        return !table && !a.pressure && (a.ghosts || !a.total_walls) && a.box_shifts && (a.nboxes == 1 || a.run_info) &&
+               a.boxes_n_max <= kExtMaxN;
     return algorithm == 0 && !table && !a.replay && (!a.tape_key || (a.nboxes == 1 && a.sample)) && !a.pressure &&
            (a.ghosts || !a.total_walls) && a.box_shifts && (a.nboxes == 1 || a.run_info) &&
            a.boxes_n_max <= kRunMaxN;
@@ -2077,6 +2513,12 @@ bool run_kernel_takes(const StepArgs& a, int algorithm, bool table)
 cudaError_t launch_step(const StepArgs& a, int algorithm, bool table, uint32_t pbuf, int grid, cudaStream_t st,
                         const RunBranches* branches)
 {
+    if (a.run_kernel == kRunExtended) {
+        const unsigned blocks = std::min((unsigned)grid, (a.num_runs + kExtWarps - 1) / (unsigned)kExtWarps);
+        const StepFnExt f = a.replay ? kExtReplayFns[a.nboxes == 1 ? 1 : 0] : kExtFns[a.sample ? 1 : 0][a.nboxes == 1 ? 1 : 0];
+        f<<<blocks, kExtThreads, kExtWarps * sizeof(ExtShared), st>>>(a);
+        return cudaGetLastError();
+    }
     if (a.run_kernel) {
         // one launch per batch size in use: a single box's, or an ensemble's density
         // classes, whose runs the run table lists class by class; with branches, the
@@ -2113,6 +2555,17 @@ cudaError_t launch_step(const StepArgs& a, int algorithm, bool table, uint32_t p
     kStepFns[algorithm ? 1 : 0][table ? 1 : 0][a.nboxes == 1 ? 1 : 0][a.replay ? 1 : 0]<<<grid, kThreads, smem, st>>>(
         a, pbuf);
     return cudaGetLastError();
+}
+
+int run_blocks_per_sm(int algorithm) { return algorithm ? kExtBlocks : 4; }
+int run_warps_per_block(int algorithm) { return algorithm ? kExtWarps : kRunWarps; }
+
+uint32_t run_cells_max(int algorithm, uint32_t n)
+{
+    if (algorithm == 0) return kRunCells;
+    // about 160 of the buffer's 184 entries, in rounds of 8 cells where they are as many
+    const uint32_t fit = std::max(1u, kExtBuf * 7 / (8 * n));
+    return std::min(kExtCells, fit >= 8 ? fit & ~7u : fit);
 }
 
 cudaError_t configure_step(int algorithm, uint32_t pbuf, uint32_t cells, int* blocks_per_sm)
@@ -2157,6 +2610,13 @@ cudaError_t configure_step(int algorithm, uint32_t pbuf, uint32_t cells, int* bl
                                              27);
     for (int k = 0; k < 3 && e == cudaSuccess; ++k)
         e = cudaFuncSetAttribute((const void*)kRunTapeFns[k], cudaFuncAttributePreferredSharedMemoryCarveout, 27);
+    // the extended run kernel: all of the unified array but a little as shared memory
+    for (int k = 0; k < 6 && e == cudaSuccess; ++k) {
+        const void* f = (const void*)(k < 4 ? kExtFns[k >> 1][k & 1] : kExtReplayFns[k & 1]);
+        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kExtWarps * sizeof(ExtShared)));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, f);
+    }
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, (const void*)sample_finalize_kernel);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, (const void*)overflow_select_kernel);
     if (e != cudaSuccess) return e;

@@ -64,7 +64,7 @@ struct BoxDesc {
     uint64_t wall_base;    // first wall-ghost entry of this box (2 per column, with walls in z)
     uint32_t run_batch;    // srd_run_kernel: cells summed and finished together (4, 8 or 16)
     uint32_t depth;        // bucket slots per cell (<= cap)
-    uint32_t run_cells;    // srd_run_kernel: cells of a run (<= 32)
+    uint32_t run_cells;    // run kernels: cells of a run (<= 32)
     uint32_t unused[3];
 };
 
@@ -182,6 +182,7 @@ struct StepArgs {
     // buffer) to fold into acc, or null (the engine folds it with sample_finalize_kernel)
     float4* fold_samp;
     SampleAcc* acc;
+    uint64_t fold_cells;          // cells of fold_samp (all boxes)
     float ext_axis[13][3];        // discrete axis set of the extended collision
     DrawTables draws;             // used by the injected-draw instantiation
     // adjoint tape of this step, by particle id / cell (null: not recorded):
@@ -208,9 +209,11 @@ struct StepArgs {
     uint32_t boxes_n_max;         // the largest density of any box
     uint64_t total_walls;         // wall-ghost entries of all boxes
     float4* box_shifts;           // grid shifts of steps k and k+1 per box (drawn by the prologue of a run-kernel step)
-    int32_t run_kernel;           // this step runs srd_run_kernel (the engine's choice, run_kernel_takes)
+    int32_t run_kernel;           // kRunSrd or kRunExtended: this step runs that kernel (the engine's choice, run_kernel_takes)
 };
 
+constexpr int32_t kRunSrd = 1, kRunExtended = 2;   // StepArgs::run_kernel
+constexpr uint32_t kExtMaxN = 36;                  // densities that ext_run_kernel takes
 constexpr uint32_t kTapeNone = 0xFFFFFFFFu;
 constexpr uint32_t kTapeBounce = 0x80000000u;
 
