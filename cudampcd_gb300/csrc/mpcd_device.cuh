@@ -231,6 +231,30 @@ __device__ __forceinline__ float3 stream_shift(const BoxDesc& b, float3 x, float
     return pbc(b, make_float3(x.x + s.x, x.y + s.y, x.z + s.z));
 }
 
+// stream_shift() and the storage index of the cell it leads to (box-local).  The
+// common case, a particle that neither wraps nor lands in the last 2^-20 of the box,
+// costs one compare per axis: with a = r + 1.5L, m = a - L lies in [0, L) exactly
+// when the wrap subtracts L (a difference that is then exact), and below L (1 - 2^-20)
+// the sums that follow cannot round up to L, so that the floor is a cell.
+__device__ __forceinline__ float3 stream_shift_cell(const BoxDesc& b, float3 x, float3& v, float3 s, uint32_t& cell)
+{
+    stream(b, x, v);
+    const float3 r = make_float3(x.x + s.x, x.y + s.y, x.z + s.z);
+    const float mx = (r.x + b.L15[0]) - b.Lf[0], my = (r.y + b.L15[1]) - b.Lf[1], mz = (r.z + b.L15[2]) - b.Lf[2];
+    // non-negative floats order as their bits; negative values and NaN fail
+    const bool in = (__float_as_uint(mx) < __float_as_uint(b.Lin[0])) & (__float_as_uint(my) < __float_as_uint(b.Lin[1])) &
+                    (__float_as_uint(mz) < __float_as_uint(b.Lin[2]));
+    float3 w = make_float3(mx - b.Lh[0], my - b.Lh[1], mz - b.Lh[2]);
+    uint3 c = make_uint3((uint32_t)(int)floorf(w.x + b.Lh[0]), (uint32_t)(int)floorf(w.y + b.Lh[1]),
+                         (uint32_t)(int)floorf(w.z + b.Lh[2]));
+    if (__builtin_expect(!in, 0)) {
+        w = pbc(b, r);
+        c = cell_of_wrapped(b, w);
+    }
+    cell = storage_index(b, c);
+    return w;
+}
+
 // Wall-layer test of a cell in the shifted frame (simulation_functions.cpp:137-138).
 __device__ __forceinline__ void wall_layer(const BoxDesc& b, uint32_t cz, bool sign, bool& layer, bool& ghosts)
 {

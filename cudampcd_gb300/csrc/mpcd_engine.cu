@@ -806,6 +806,7 @@ private:
             b.L2x[d] = 2.0f * b.Lf[d];
             b.L3x[d] = 3.0f * b.Lf[d];
             b.Lh[d] = b.Lf[d] * 0.5f;
+            b.Lin[d] = b.Lf[d] * (1.0f - 0x1p-20f);
             b.periodic[d] = p.periodicity[d];
             Nf *= (uint64_t)(b.L[d] - 2 * (1 - b.periodic[d]));
         }

@@ -1448,8 +1448,8 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
                     v = collided ? vc : v;
                 }
                 vn = v;
-                xn = stream_shift(b, x, vn, sn);
-                key = b.cell_base + storage_index(b, cell_of_wrapped(b, xn));
+                xn = stream_shift_cell(b, x, vn, sn, key);
+                key += b.cell_base;
                 id = __float_as_uint(vp.w);
                 const uint32_t lab = SAMPLE || TAPE ? b.cell_base + storage_index(b, cell_of_wrapped(b, x)) : 0u;
                 if (SAMPLE) sample_add(a.samp, lab, v, active);
@@ -1492,8 +1492,9 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
 // What bounds it is instruction issue and latency.  The tile kernel spends 33.6 warp
 // instructions a particle at n = 20: four lanes of each colliding cell draw and sum
 // while the warp's other cells wait, ranks are looked up in every pass, and five
-// CTA-wide barriers a tile stall its warps.  This kernel: 26 a particle, 64 % issue.  256 x 256 x 66, n = 20 (8.2e7 particles), us a step:
-// tile kernel 3459, this one 2656; sampled 3677 and 2954.  Its code size matters: with
+// CTA-wide barriers a tile stall its warps.  This kernel: 26 a particle before, 24.6 after the
+// streaming's fast wrap, 64 % issue.  256 x 256 x 66, n = 20 (8.2e7 particles), us a step:
+// tile kernel 3459, this one 2600; sampled 3677 and 2863.  Its code size matters: with
 // the passes over a part unrolled it no longer fit the instruction cache and took
 // 10700 us; with the compiler's own unrolling of the inner loops 3280.
 
@@ -1872,8 +1873,9 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                     continue;
                 }
                 float3 vn = v;
-                const float3 xn = stream_shift(b, x, vn, sn);
-                const uint32_t key = active ? b.cell_base + storage_index(b, cell_of_wrapped(b, xn)) : kNoKey;
+                uint32_t key;
+                const float3 xn = stream_shift_cell(b, x, vn, sn, key);
+                key = active ? b.cell_base + key : kNoKey;
                 if (SAMPLE) {
                     const uint32_t lab = b.cell_base + storage_index(b, cell_of_wrapped(b, x));
                     sample_add(a.samp, lab, v, active);

@@ -41,6 +41,7 @@ struct BoxDesc {
     int32_t L[3];          // container size incl. wall layers
     float Lf[3];
     float L15[3], L2x[3], L3x[3], Lh[3];   // 1.5 L, 2 L, 3 L, L / 2 (float products, as the reference forms them)
+    float Lin[3];          // L (1 - 2^-20): see stream_shift_cell
     int32_t periodic[3];
     int32_t wall_z;        // periodicity.z == 0: bounce-back walls and ghost layers in z
     int32_t channel;       // ExperimentType::channel
@@ -65,7 +66,6 @@ struct BoxDesc {
     uint32_t run_batch;    // srd_run_kernel: cells summed and finished together (4, 8 or 16)
     uint32_t depth;        // bucket slots per cell (<= cap)
     uint32_t run_cells;    // run kernels: cells of a run (<= 32)
-    uint32_t unused[3];
 };
 
 // The step kernel copies a box descriptor into shared memory 16 bytes per thread.
