@@ -1241,6 +1241,7 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
 {
     __shared__ RunShared shared_runs[kRunWarps];
     __shared__ __align__(16) BoxDesc shared_box[SINGLE ? 1 : kRunWarps];   // ensembles: the box of the warp's run
+    __shared__ float4 shared_shifts[SINGLE ? 1 : kRunWarps][2];              // and its grid shifts of steps k and k+1
     const uint32_t lane = threadIdx.x & 31u;
     RunShared& sh = shared_runs[threadIdx.x >> 5];
     BoxDesc& sbox = shared_box[SINGLE ? 0 : threadIdx.x >> 5];
@@ -1252,11 +1253,9 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
     static_assert(BATCH == 4 || BATCH == 8 || BATCH == 16, "batches of 4, 8 or 16 cells");
     // single box: geometry straight from the kernel parameters (constant bank)
     const BoxDesc& b = SINGLE ? a.box0 : sbox;
-    float3 s = make_float3(0, 0, 0), sn = s;
-    if (SINGLE) {
-        const float4 s0 = __ldg(a.box_shifts), s1 = __ldg(a.box_shifts + 1);   // drawn by the prologue
-        s = make_float3(s0.x, s0.y, s0.z);
-        sn = make_float3(s1.x, s1.y, s1.z);
+    if (SINGLE) {   // drawn by the prologue
+        if (threadIdx.x < 2) shared_shifts[0][threadIdx.x] = __ldg(a.box_shifts + threadIdx.x);
+        __syncthreads();
     }
     if (first_launch) {   // once per step (ensembles launch once per batch size)
         if (blockIdx.x == 0 && threadIdx.x == 0) {   // list of step k-1, refilled by step k+1
@@ -1280,12 +1279,10 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
             __syncwarp();
             if (lane < sizeof(BoxDesc) / 16)
                 reinterpret_cast<uint4*>(&sbox)[lane] = __ldg(reinterpret_cast<const uint4*>(a.boxes + cur_box) + lane);
-            const float4 s0 = __ldg(a.box_shifts + 2 * cur_box), s1 = __ldg(a.box_shifts + 2 * cur_box + 1);
-            s = make_float3(s0.x, s0.y, s0.z);
-            sn = make_float3(s1.x, s1.y, s1.z);
+            if (lane < 2) shared_shifts[threadIdx.x >> 5][lane] = __ldg(a.box_shifts + 2 * cur_box + lane);
             __syncwarp();
         }
-        const bool sign = s.z > 0;
+        const bool sign = shared_shifts[SINGLE ? 0 : threadIdx.x >> 5][0].z > 0;
         const uint32_t c = cur.x - b.cell_base + lane;   // box-local cell of this lane
         const bool valid = lane < (cur.y & 63u);
         // the lane's cell: its colliding particles and the slot of the first (its
@@ -1442,13 +1439,15 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
                 {   // the collision computed for every lane, kept where the cell has more than one
                     // entry (a lone particle keeps its shifted position, as in the reference)
                     float3 xc = x, vc = v;
-                    srd_collide(b, s, make_float3(cd.x, cd.y, cd.z), make_float3(ax.x, ax.y, ax.z), xc, vc);
+                    const float4 sv = shared_shifts[SINGLE ? 0 : threadIdx.x >> 5][0];
+                    srd_collide(b, make_float3(sv.x, sv.y, sv.z), make_float3(cd.x, cd.y, cd.z), make_float3(ax.x, ax.y, ax.z), xc, vc);
                     const bool collided = __float_as_uint(cd.w) > 1;
                     x = collided ? xc : x;
                     v = collided ? vc : v;
                 }
                 vn = v;
-                xn = stream_shift_cell(b, x, vn, sn, key);
+                const float4 nv = shared_shifts[SINGLE ? 0 : threadIdx.x >> 5][1];
+                xn = stream_shift_cell(b, x, vn, make_float3(nv.x, nv.y, nv.z), key);
                 key += b.cell_base;
                 id = __float_as_uint(vp.w);
                 const uint32_t lab = SAMPLE || TAPE ? b.cell_base + storage_index(b, cell_of_wrapped(b, x)) : 0u;
@@ -1494,7 +1493,7 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
 // while the warp's other cells wait, ranks are looked up in every pass, and five
 // CTA-wide barriers a tile stall its warps.  This kernel: 26 a particle before, 24.6 after the
 // streaming's fast wrap, 64 % issue.  256 x 256 x 66, n = 20 (8.2e7 particles), us a step:
-// tile kernel 3459, this one 2600; sampled 3677 and 2863.  Its code size matters: with
+// tile kernel 3459, this one 2595; sampled 3677 and 2857.  Its code size matters: with
 // the passes over a part unrolled it no longer fit the instruction cache and took
 // 10700 us; with the compiler's own unrolling of the inner loops 3280.
 
