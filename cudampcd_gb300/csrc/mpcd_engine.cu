@@ -145,6 +145,7 @@ public:
             if (branches_.join[i]) cudaEventDestroy(branches_.join[i]);
         }
         if (branches_.fork) cudaEventDestroy(branches_.fork);
+        if (flags_host_) cudaFreeHost(flags_host_);
     }
 
     // ------------------------------------------------------------ reference Backend interface
@@ -269,18 +270,20 @@ public:
     void set_device(const float* d_pos, const float* d_vel)
     {
         if (!d_pos || !d_vel) materialise();
-        if (d_pos)
-            check(cudaMemcpyAsync(dense_pos_.p, d_pos, sizeof(float) * 3 * N_, cudaMemcpyDeviceToDevice, stream_),
-                  "positions write");
-        if (d_vel)
-            check(cudaMemcpyAsync(dense_vel_.p, d_vel, sizeof(float) * 3 * N_, cudaMemcpyDeviceToDevice, stream_),
-                  "velocities write");
-        scatter_dense();
+        scatter_dense(nullptr, d_pos, d_vel);
         check_device_errors();
     }
 
     void get_device(float* d_pos, float* d_vel)
     {
+        // the first read of a state replays the step straight into the caller's buffers;
+        // later ones keep the state and copy it
+        if (d_pos && d_vel && !dense_valid_ && !direct_read_ && step_ > 0) {
+            launch_replay(d_pos, d_vel);
+            check_device_errors();
+            direct_read_ = true;
+            return;
+        }
         materialise();
         if (d_pos)
             check(cudaMemcpyAsync(d_pos, dense_pos_.p, sizeof(float) * 3 * N_, cudaMemcpyDeviceToDevice, stream_),
@@ -1031,6 +1034,7 @@ private:
         if (walls_) check(ghosts_.alloc(sizeof(GhostSum) * walls_), "alloc wall ghosts");
         check(box_shifts_.alloc(sizeof(float4) * 2 * boxes_.size()), "alloc box shifts");
         check(state_.alloc(sizeof(DeviceState)), "alloc state");
+        check(cudaMallocHost((void**)&flags_host_, sizeof *flags_host_), "alloc error flags");
         check(cudaMemset(state_.p, 0, sizeof(DeviceState)), "clear state");
         check(samp_.alloc(sizeof(float4) * cells_ * 2), "alloc sample");   // two parities
         check(cudaMemset(samp_.p, 0, samp_.bytes), "clear sample");
@@ -1206,7 +1210,7 @@ private:
         step_ += (uint64_t)done;
         last_step_table_ = false;
         last_step_run_ = graph_run_;
-        dense_valid_ = false;
+        dense_valid_ = direct_read_ = false;
         return done;
     }
 
@@ -1255,8 +1259,21 @@ private:
         last_step_table_ = use_table_;   // a replay of this step must consume the same draws
         use_table_ = false;
         ++step_;
-        dense_valid_ = false;
+        dense_valid_ = direct_read_ = false;
         return a.fold_samp != nullptr;
+    }
+
+    // Recompute the collision of the last step from its inputs into (N, 3) arrays by
+    // particle id.  A run kernel replays its own steps, from the wall ghosts and grid
+    // shifts that the step's prologue left.
+    void launch_replay(float* pos, float* vel)
+    {
+        StepArgs a = args(step_ - 1, true);
+        a.dense_pos = pos;
+        a.dense_vel = vel;
+        a.run_kernel = last_step_run_;
+        check(launch_step(a, params_.algorithm, last_step_table_, pbuf_, a.run_kernel ? run_grid_ : grid_, stream_),
+              "replay");
     }
 
     // The post-step state, by particle id, in dense_pos_ / dense_vel_: recompute
@@ -1266,12 +1283,7 @@ private:
     {
         if (!dense_valid_) {
             if (step_ == 0) throw Error(MPCD_GB_ESTATE, "no state to read");
-            StepArgs a = args(step_ - 1, true);
-            // the extended run kernel replays its own steps (from the prologue's ghost counts and shifts)
-            if (last_step_run_ == kRunExtended) a.run_kernel = kRunExtended;
-            check(launch_step(a, params_.algorithm, last_step_table_, pbuf_, a.run_kernel ? run_grid_ : grid_, stream_),
-                  "replay");
-            check(cudaStreamSynchronize(stream_), "replay");
+            launch_replay(dense_pos_.as<float>(), dense_vel_.as<float>());
             check_device_errors();
             dense_valid_ = true;
         }
@@ -1320,29 +1332,26 @@ private:
             ++step_;
         }
         last_step_table_ = false;
-        dense_valid_ = false;
+        dense_valid_ = direct_read_ = false;
         return k;
     }
 
     // Dense post-step arrays (dense_pos_, dense_vel_) -> buckets of step step_:
     // the scatter plays the epilogue of step step_ - 1 (tape_b0: bounce bits of its streaming).
-    void scatter_dense(uint32_t* tape_b0 = nullptr)
+    // The state comes from the dense arrays, or from pos and vel where they are given:
+    // the dense arrays then receive a copy.
+    void scatter_dense(uint32_t* tape_b0 = nullptr, const float* pos = nullptr, const float* vel = nullptr)
     {
         const uint64_t k = step_;
-        for (uint64_t j = k; j < k + 2; ++j) {
-            check(cudaMemsetAsync(count_[j % 3].p, 0, count_[j % 3].bytes, stream_), "clear counts");
-            check(cudaMemsetAsync((char*)state_.p + offsetof(DeviceState, ov) + sizeof(OverflowFill) * (j % 3), 0,
-                                  sizeof(OverflowFill), stream_),
-                  "clear overflow list");
-        }
-        check(cudaMemsetAsync((char*)state_.p + offsetof(DeviceState, ext_count) + sizeof(unsigned int) * (k & 1), 0,
-                              sizeof(unsigned int), stream_),
-              "clear extension");
         StepArgs a = args(k - 1);   // out_* = buckets, counts and overflow list of step k
+        a.out_count = count_[k % 3].as<uint32_t>();
         a.tape_lab = tape_b0;
-        check(launch_scatter(a, dense_pos_.as<float>(), dense_vel_.as<float>(), N_, sms_ * 8, stream_),
+        check(launch_scatter(a, pos ? pos : dense_pos_.as<float>(), vel ? vel : dense_vel_.as<float>(),
+                             pos ? dense_pos_.as<float>() : nullptr, vel ? dense_vel_.as<float>() : nullptr, N_, cells_,
+                             count_[(k + 1) % 3].as<uint32_t>(), sms_, stream_),
               "scatter");
         dense_valid_ = true;
+        direct_read_ = false;
     }
 
     void layout(uint32_t* cell, uint32_t* slot, uint32_t* prev, uint32_t* id)
@@ -1393,11 +1402,11 @@ private:
     void check_device_errors()
     {
         check(cudaGetLastError(), "launch");
-        unsigned int flags = 0;
-        check(cudaMemcpyAsync(&flags, (char*)state_.p + offsetof(DeviceState, error_flags), sizeof flags,
+        check(cudaMemcpyAsync(flags_host_, (char*)state_.p + offsetof(DeviceState, error_flags), sizeof *flags_host_,
                               cudaMemcpyDeviceToHost, stream_),
               "error flags");
         check(cudaStreamSynchronize(stream_), "step");
+        const unsigned int flags = *flags_host_;
         if (flags & kErrOverflowListFull) throw Error(MPCD_GB_EDEVICE, "cell overflow list exhausted");
         if (flags & kErrWaitTimeout) throw Error(MPCD_GB_EDEVICE, "device wait timed out");
         if (flags & kErrKeyMismatch) throw Error(MPCD_GB_EDEVICE, "particle found in the wrong cell bucket");
@@ -1428,6 +1437,8 @@ private:
     bool use_table_ = false;
     bool last_step_table_ = false;
     int32_t last_step_run_ = 0, graph_run_ = 0;   // StepArgs::run_kernel of the last step, of the step graphs
+    unsigned int* flags_host_ = nullptr;   // pinned: error flags read at the end of a call
+    bool direct_read_ = false;   // the state of this step was replayed into a caller's buffers
     bool dense_valid_ = false;   // dense_pos_ / dense_vel_ hold the state after step step_ - 1
     DrawTables tables_{};
     int inject_valid_[kMaxInjectedShifts] = {0, 0, 0, 0};

@@ -1235,7 +1235,30 @@ __device__ __forceinline__ uint2 run_entry(const StepArgs& a, uint32_t run)
     return make_uint2(a.box0.cell_base + c0, min(a.box0.run_cells, a.box0.C - c0));
 }
 
-template <bool SAMPLE, bool SINGLE, uint32_t BATCH, bool TAPE = false>
+enum RunMode : int { kPlain = 0, kTape = 1, kReplay = 2 };
+
+// A row of a dense (N, 3) array for every lane of the mask: through shared memory (96
+// floats), so that consecutive lanes write consecutive words of a row and a warp's store
+// touches a third of the sectors that a store per component does (replay of 1.49e7
+// particles in random order 1600 -> 1216 us, bound by the random writes; of 449,000 that
+// fit L2 26.7 -> 12.7).
+__device__ __forceinline__ void write_rows(float* stage, float* dense, uint32_t id, float3 r, unsigned mask)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    stage[3 * lane] = r.x;
+    stage[3 * lane + 1] = r.y;
+    stage[3 * lane + 2] = r.z;
+    __syncwarp();
+#pragma unroll
+    for (uint32_t t = 0; t < 3; ++t) {
+        const uint32_t w = 32 * t + lane, row = w / 3;
+        const uint64_t at = 3 * (uint64_t)__shfl_sync(kFull, id, (int)row) + (w - 3 * row);
+        if (mask >> row & 1u) dense[at] = stage[w];
+    }
+    __syncwarp();
+}
+
+template <bool SAMPLE, bool SINGLE, uint32_t BATCH, int MODE = kPlain>
 __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, uint32_t run_begin, uint32_t run_end,
                                                               bool first_launch)
 {
@@ -1243,6 +1266,8 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
     __shared__ __align__(16) BoxDesc shared_box[SINGLE ? 1 : kRunWarps];   // ensembles: the box of the warp's run
     __shared__ float4 shared_shifts[SINGLE ? 1 : kRunWarps][2];              // and its grid shifts of steps k and k+1
     const uint32_t lane = threadIdx.x & 31u;
+    constexpr bool TAPE = MODE == kTape, REPLAY = MODE == kReplay;
+    __shared__ float shared_rows[REPLAY ? kRunWarps : 1][96];
     RunShared& sh = shared_runs[threadIdx.x >> 5];
     BoxDesc& sbox = shared_box[SINGLE ? 0 : threadIdx.x >> 5];
     const uint64_t step = a.step_base ? *a.step_base + a.step : a.step;   // graph replays read the base
@@ -1258,7 +1283,7 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
         __syncthreads();
     }
     if (first_launch) {   // once per step (ensembles launch once per batch size)
-        if (blockIdx.x == 0 && threadIdx.x == 0) {   // list of step k-1, refilled by step k+1
+        if (!REPLAY && blockIdx.x == 0 && threadIdx.x == 0) {   // list of step k-1, refilled by step k+1
             a.state->ov[a.ov_zero_slot] = OverflowFill{0u, 0u};
         }
         if (left) overflow_pass(a, step);
@@ -1291,7 +1316,7 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
         const Slot* src_lane;
         const uint32_t cnt = cell_source(a, b, a.in_slots, c, raw_next, src_lane);
         const uint32_t src_slot = (uint32_t)(src_lane - a.in_slots);
-        if (valid) a.zero_count[cur.x + lane] = 0;   // counts of step k-1: step k+1 fills them
+        if (!REPLAY && valid) a.zero_count[cur.x + lane] = 0;   // counts of step k-1: step k+1 fills them
         // sampled steps: the previous step's sample of this lane's (lab) cell into the
         // FP64 sums, where the engine defers it to this step (every cell is one lane's)
         if (SAMPLE && !TAPE && a.fold_samp && valid) fold_sample(a.fold_samp, a.acc, cur.x + lane, 0, nullptr);
@@ -1444,6 +1469,13 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
                     const bool collided = __float_as_uint(cd.w) > 1;
                     x = collided ? xc : x;
                     v = collided ? vc : v;
+                }
+                if (REPLAY) {
+                    const unsigned rows = __ballot_sync(kFull, active);
+                    float* const stage = shared_rows[REPLAY ? threadIdx.x >> 5 : 0];
+                    write_rows(stage, a.dense_pos, __float_as_uint(vp.w), x, rows);
+                    write_rows(stage, a.dense_vel, __float_as_uint(vp.w), v, rows);
+                    continue;
                 }
                 vn = v;
                 const float4 nv = shared_shifts[SINGLE ? 0 : threadIdx.x >> 5][1];
@@ -1863,12 +1895,10 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                     // com + xr rebuilds the wrapped staged position to within rounding
                     x = pbc_near(b, make_float3((k1.x + xr.x) - s.x, (k1.y + xr.y) - s.y, (k1.z + xr.z) - s.z));
                 }
-                if (REPLAY) {
-                    if (active) {
-                        const uint64_t i3 = 3 * (uint64_t)__float_as_uint(vp.w);
-                        a.dense_pos[i3] = x.x; a.dense_pos[i3 + 1] = x.y; a.dense_pos[i3 + 2] = x.z;
-                        a.dense_vel[i3] = v.x; a.dense_vel[i3 + 1] = v.y; a.dense_vel[i3 + 2] = v.z;
-                    }
+                if (REPLAY) {   // staged in the terms' room
+                    const unsigned rows = __ballot_sync(kFull, active);
+                    write_rows(&sh.term[0][0], a.dense_pos, __float_as_uint(vp.w), x, rows);
+                    write_rows(&sh.term[0][0], a.dense_vel, __float_as_uint(vp.w), v, rows);
                     continue;
                 }
                 float3 vn = v;
@@ -2075,29 +2105,80 @@ __global__ void advance_kernel(DeviceState* state, unsigned steps)
 
 // ------------------------------------------------------------------ prologue scatter
 
+// Zero the counts of steps k and k+1 and the bookkeeping of their overflow lists and
+// of step k's extension: what a scatter into step k's buckets starts from.
+__global__ void __launch_bounds__(kThreads) clear_counts_kernel(uint32_t* c0, uint32_t* c1, uint64_t cells,
+                                                                DeviceState* state, uint64_t k)
+{
+    const uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+    if (i == 0) {
+        state->ov[k % 3] = state->ov[(k + 1) % 3] = OverflowFill{0u, 0u};
+        state->ext_count[k & 1] = 0u;
+    }
+    for (uint64_t c = i; c < cells; c += (uint64_t)gridDim.x * kThreads) {
+        c0[c] = 0u;
+        c1[c] = 0u;
+    }
+}
+
 // Stream dense post-step particles for step k (a.step = k - 1: the launch plays
 // the epilogue of step k-1), key them by the cell they then occupy and scatter
-// them into the buckets of step k (a.out_*); particle id = dense index.
-__global__ void __launch_bounds__(kThreads) scatter_kernel(StepArgs a, const float* pos, const float* vel,
-                                                           uint64_t n_total)
+// them into the buckets of step k (a.out_*); particle id = dense index.  keep_pos,
+// keep_vel (or null): where the handle keeps the dense state that it was given.
+// What bounds it is the random 32-byte store (40 G/s measured on stores alone over a
+// region past L2, 128 G/s for the claims): 1.49e7 particles in random order over 151 x
+// 203 x 97 cells take 491 us, the copy to the dense arrays included, where 373 us are
+// the stores' own; the copies and the scatter before took 411 + 117 us.  A lane has four
+// particles in flight (two in an ensemble, whose boxes it looks up), and a single box
+// draws its grid shift once per thread: 41,000 particles 14.5 -> 6.1 us.
+template <bool SINGLE>
+__global__ void __launch_bounds__(kThreads, 4) scatter_kernel(const StepArgs a, const float* pos, const float* vel,
+                                                              float* keep_pos, float* keep_vel, uint64_t n_total)
 {
-    for (uint64_t base = (uint64_t)blockIdx.x * kThreads; base < n_total; base += (uint64_t)gridDim.x * kThreads) {
-        const uint64_t i = base + threadIdx.x;
-        const bool active = i < n_total;
-        int bi = 0;
-        uint32_t key = 0;
-        float3 xs = make_float3(0, 0, 0), vs = xs;
-        if (active) {
-            bi = box_of_particle(a.boxes, a.nboxes, i);
-            const BoxDesc& b = a.boxes[bi];
-            vs = make_float3(vel[3 * i], vel[3 * i + 1], vel[3 * i + 2]);
-            const float3 v0 = vs;
-            xs = stream_shift(b, make_float3(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]), vs,
-                              grid_shift(b, bi, a.step + 1, a.state));
-            key = b.cell_base + storage_index(b, cell_of_wrapped(b, xs));
-            if (a.tape_lab) a.tape_lab[i] = (vs.x != v0.x || vs.y != v0.y || vs.z != v0.z) ? kTapeBounce : 0u;
+    constexpr int kEach = SINGLE ? 4 : 2;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t warp = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) >> 5, warps = (uint64_t)gridDim.x * (kThreads / 32);
+    float3 shift = make_float3(0, 0, 0);
+    if (SINGLE) shift = grid_shift(a.box0, 0, a.step + 1, a.state);
+    for (uint64_t base = warp * 32 * kEach; base < n_total; base += warps * 32 * kEach) {
+        float3 x[kEach], v[kEach];
+        uint32_t key[kEach], slot[kEach];
+        unsigned peers[kEach];
+        int box[kEach];
+#pragma unroll
+        for (int u = 0; u < kEach; ++u) {
+            const uint64_t i = base + 32 * u + lane, at = 3 * (i < n_total ? i : n_total - 1);
+            x[u] = make_float3(pos[at], pos[at + 1], pos[at + 2]);
+            v[u] = make_float3(vel[at], vel[at + 1], vel[at + 2]);
         }
-        store_particle(a, a.boxes[bi], xs, vs, (uint32_t)i, key, active);
+#pragma unroll
+        for (int u = 0; u < kEach; ++u) {
+            const uint64_t i = base + 32 * u + lane;
+            const bool active = i < n_total;
+            if (keep_pos && active) { keep_pos[3 * i] = x[u].x; keep_pos[3 * i + 1] = x[u].y; keep_pos[3 * i + 2] = x[u].z; }
+            if (keep_vel && active) { keep_vel[3 * i] = v[u].x; keep_vel[3 * i + 1] = v[u].y; keep_vel[3 * i + 2] = v[u].z; }
+            box[u] = SINGLE || !active ? 0 : box_of_particle(a.boxes, a.nboxes, i);
+            const BoxDesc& b = SINGLE ? a.box0 : a.boxes[box[u]];
+            const float3 v0 = v[u];
+            uint32_t cell;
+            x[u] = stream_shift_cell(b, x[u], v[u], SINGLE ? shift : grid_shift(b, box[u], a.step + 1, a.state), cell);
+            key[u] = active ? b.cell_base + cell : kNoKey;
+            if (a.tape_lab && active)
+                a.tape_lab[i] = (v[u].x != v0.x || v[u].y != v0.y || v[u].z != v0.z) ? kTapeBounce : 0u;
+            peers[u] = __match_any_sync(kFull, key[u]);
+            slot[u] = 0;
+            if (active && (int)lane == __ffs(peers[u]) - 1) slot[u] = atomicAdd(a.out_count + key[u], (uint32_t)__popc(peers[u]));
+        }
+#pragma unroll
+        for (int u = 0; u < kEach; ++u) {
+            const uint32_t at = __shfl_sync(kFull, slot[u], __ffs(peers[u]) - 1) + __popc(peers[u] & lanemask_lt());
+            if (key[u] == kNoKey) continue;
+            const BoxDesc& b = SINGLE ? a.box0 : a.boxes[box[u]];
+            const float4 xp = make_float4(x[u].x, x[u].y, x[u].z, __uint_as_float(kNoExt));
+            const float4 vp = make_float4(v[u].x, v[u].y, v[u].z, __uint_as_float((uint32_t)(base + 32 * u + lane)));
+            if (at < b.depth) store_slot(a.out_slots + ((uint32_t)b.slot_base + (key[u] - b.cell_base) * b.depth + at), xp, vp);
+            else push_overflow(a, key[u], xp, vp);
+        }
     }
 }
 
@@ -2487,8 +2568,12 @@ const StepFn kStepFns[2][2][2][2] = {
 using StepFnRun = void (*)(const StepArgs, uint32_t, uint32_t, bool);
 // [sample][single box][batch class: 16, 8, 4 cells]
 // single-box sampled steps that record the adjoint tape, by batch size
-static const StepFnRun kRunTapeFns[3] = {srd_run_kernel<true, true, 16, true>, srd_run_kernel<true, true, 8, true>,
-                                         srd_run_kernel<true, true, 4, true>};
+static const StepFnRun kRunTapeFns[3] = {srd_run_kernel<true, true, 16, kTape>, srd_run_kernel<true, true, 8, kTape>,
+                                         srd_run_kernel<true, true, 4, kTape>};
+// replays: [single box][batch class]
+static const StepFnRun kRunReplayFns[2][3] = {
+    {srd_run_kernel<false, false, 16, kReplay>, srd_run_kernel<false, false, 8, kReplay>, srd_run_kernel<false, false, 4, kReplay>},
+    {srd_run_kernel<false, true, 16, kReplay>, srd_run_kernel<false, true, 8, kReplay>, srd_run_kernel<false, true, 4, kReplay>}};
 static const StepFnRun kRunFns[2][2][3] = {
     {{srd_run_kernel<false, false, 16>, srd_run_kernel<false, false, 8>, srd_run_kernel<false, false, 4>},
      {srd_run_kernel<false, true, 16>, srd_run_kernel<false, true, 8>, srd_run_kernel<false, true, 4>}},
@@ -2537,7 +2622,8 @@ cudaError_t launch_step(const StepArgs& a, int algorithm, bool table, uint32_t p
         }
         for (int i = 0; i < nused; ++i) {
             const int cls = used[i];
-            const StepFnRun f = a.tape_key ? kRunTapeFns[cls] : kRunFns[a.sample ? 1 : 0][a.nboxes == 1 ? 1 : 0][cls];
+            const int single = a.nboxes == 1 ? 1 : 0;
+            const StepFnRun f = a.replay ? kRunReplayFns[single][cls] : a.tape_key ? kRunTapeFns[cls] : kRunFns[a.sample ? 1 : 0][single][cls];
             const uint32_t runs = a.run_class[cls + 1] - a.run_class[cls];
             const unsigned blocks = std::min((unsigned)grid, (runs + kRunWarps - 1) / (unsigned)kRunWarps);
             f<<<blocks, kThreads, 0, fork && i > 0 ? branches->side[i - 1] : st>>>(a, a.run_class[cls],
@@ -2609,8 +2695,11 @@ cudaError_t configure_step(int algorithm, uint32_t pbuf, uint32_t cells, int* bl
                 if (e == cudaSuccess)
                     e = cudaFuncSetAttribute((const void*)kRunFns[i][j][k], cudaFuncAttributePreferredSharedMemoryCarveout,
                                              27);
-    for (int k = 0; k < 3 && e == cudaSuccess; ++k)
+    for (int k = 0; k < 3 && e == cudaSuccess; ++k) {
         e = cudaFuncSetAttribute((const void*)kRunTapeFns[k], cudaFuncAttributePreferredSharedMemoryCarveout, 27);
+        for (int i = 0; i < 2 && e == cudaSuccess; ++i)
+            e = cudaFuncSetAttribute((const void*)kRunReplayFns[i][k], cudaFuncAttributePreferredSharedMemoryCarveout, 34);
+    }
     // the extended run kernel: all of the unified array but a little as shared memory
     for (int k = 0; k < 6 && e == cudaSuccess; ++k) {
         const void* f = (const void*)(k < 4 ? kExtFns[k >> 1][k & 1] : kExtReplayFns[k & 1]);
@@ -2657,10 +2746,16 @@ cudaError_t launch_advance(DeviceState* state, unsigned steps, cudaStream_t st)
     return cudaGetLastError();
 }
 
-cudaError_t launch_scatter(const StepArgs& a, const float* pos, const float* vel, uint64_t n_total, int grid,
-                           cudaStream_t st)
+cudaError_t launch_scatter(const StepArgs& a, const float* pos, const float* vel, float* keep_pos, float* keep_vel,
+                           uint64_t n_total, uint64_t cells, uint32_t* next_count, int sms, cudaStream_t st)
 {
-    scatter_kernel<<<grid, kThreads, 0, st>>>(a, pos, vel, n_total);
+    const unsigned zero = (unsigned)std::min<uint64_t>((cells + kThreads - 1) / kThreads, (uint64_t)sms * 8);
+    clear_counts_kernel<<<zero, kThreads, 0, st>>>(a.out_count, next_count, cells, a.state, a.step + 1);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const unsigned grid = (unsigned)std::min<uint64_t>((n_total + 4 * kThreads - 1) / (4 * kThreads), (uint64_t)sms * 4);
+    if (a.nboxes == 1) scatter_kernel<true><<<grid, kThreads, 0, st>>>(a, pos, vel, keep_pos, keep_vel, n_total);
+    else scatter_kernel<false><<<grid, kThreads, 0, st>>>(a, pos, vel, keep_pos, keep_vel, n_total);
     return cudaGetLastError();
 }
 

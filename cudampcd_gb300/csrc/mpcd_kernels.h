@@ -38,9 +38,11 @@ uint32_t run_cells_max(int algorithm, uint32_t n);
 bool run_kernel_takes(const StepArgs& a, int algorithm, bool table);
 // state->step_base += steps (the last node of a replayed step graph).
 cudaError_t launch_advance(DeviceState* state, unsigned steps, cudaStream_t st);
-// Key dense clean particles for step a.step + 1 and scatter them into a.out_*.
-cudaError_t launch_scatter(const StepArgs& a, const float* pos, const float* vel, uint64_t n_total, int grid,
-                           cudaStream_t st);
+// Clear the counts of steps k = a.step + 1 and k + 1 (a.out_count, next_count), key dense
+// clean particles for step k and scatter them into a.out_*; keep_pos / keep_vel (or null)
+// receive a copy of them.
+cudaError_t launch_scatter(const StepArgs& a, const float* pos, const float* vel, float* keep_pos, float* keep_vel,
+                           uint64_t n_total, uint64_t cells, uint32_t* next_count, int sms, cudaStream_t st);
 // Before a step (not a replay): the particles the reference keeps in each cell past
 // its bucket depth into the extension area after the buckets, the others left in
 // the overflow list (in_* / ov_*: the step's input buckets and list, a.in_count,
