@@ -15,9 +15,9 @@ adjoint holds the discrete events of the forward trajectory fixed:
 - ghost counts;
 - wall bounces.
 
-The state is checkpointed every `checkpoint_every` steps. The backward recomputes
-one segment at a time, then sweeps it in reverse. It returns dL/dV0 for every
-particle and dL/d(drag).
+A forward whose events fit 4 GiB keeps them all.  A longer one checkpoints the state
+every `checkpoint_every` steps, and the backward recomputes one segment at a time, then
+sweeps it in reverse. It returns dL/dV0 for every particle and dL/d(drag).
 """
 from __future__ import annotations
 

@@ -1319,7 +1319,7 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
         if (!REPLAY && valid) a.zero_count[cur.x + lane] = 0;   // counts of step k-1: step k+1 fills them
         // sampled steps: the previous step's sample of this lane's (lab) cell into the
         // FP64 sums, where the engine defers it to this step (every cell is one lane's)
-        if (SAMPLE && !TAPE && a.fold_samp && valid) fold_sample(a.fold_samp, a.acc, cur.x + lane, 0, nullptr);
+        if (SAMPLE && a.fold_samp && valid) fold_sample(a.fold_samp, a.acc, cur.x + lane, 0, TAPE ? a.fold_count : nullptr);
         next = run_entry<SINGLE>(a, run + warps < run_end ? run + warps : a.num_runs);
         raw_next = lane < (next.y & 63u) ? a.in_count[next.x + lane] : 0u;
         const uint3 cc = storage_coords(b, valid ? c : 0u);
@@ -2461,87 +2461,98 @@ __global__ void __launch_bounds__(kThreads) profile_kernel(const SampleAcc* acc,
     if (threadIdx.x == 0) profile[blockIdx.x] = (float)(red[0] * inv);
 }
 
-// Per cell of the step (storage order): clear the cell sums of mu, and store the
-// cell's rotation axis (as a collision cell) and its sampling term dU(z) w / count
-// (as a lab cell; FP64 quotient rounded to FP32) in cell_axis, so that the particle
-// passes read them instead of drawing an axis and dividing per particle.
-__global__ void __launch_bounds__(kThreads) adjoint_cells_kernel(BoxDesc b, uint64_t step, const uint32_t* lab_count,
-                                                                 const float* dU, double w, float4* cellsum,
-                                                                 float4* cell_axis)
+// Cells of a step (storage order), before its sweep adds to their sums: N_c, the axis and
+// the sampling term, so that a particle neither draws an axis nor divides.
+__device__ __forceinline__ void adjoint_cells(const BoxDesc& b, const AdjointStep& t, const float* dU, double w)
 {
-    const uint32_t Lz = (uint32_t)b.L[2];
     for (uint32_t c = blockIdx.x * kThreads + threadIdx.x; c < b.C; c += gridDim.x * kThreads) {
-        cellsum[c] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        const uint32_t cnt = lab_count[b.cell_base + c];
-        const float term = cnt ? (float)((double)dU[c % Lz] * w / (double)cnt) : 0.0f;   // z fastest
-        const float3 a = srd_axis_philox(b, step, ref_index(b, storage_coords(b, c)));
-        cell_axis[c] = make_float4(a.x, a.y, a.z, term);
+        const uint32_t cnt = t.lab_count[c], n = t.ncell[c];
+        const uint3 cc = storage_coords(b, c);
+        const float term = cnt ? (float)((double)dU[cc.z] * w / (double)cnt) : 0.0f;
+        const float3 a = srd_axis_philox(b, t.step, ref_index(b, cc));
+        t.cells[c].sum = make_float4(0.0f, 0.0f, 0.0f, n ? 1.0f / (float)n : 0.0f);
+        t.cells[c].axis = make_float4(a.x, a.y, a.z, term);
     }
 }
 
-// mu = B_{t+1} lambda + sampling term; cell sums of mu over collided particles; dL/dg partial.
-__global__ void __launch_bounds__(kThreads) adjoint_pass1_kernel(BoxDesc b, uint32_t n, float* lam,
-                                                                 const uint32_t* key, const uint32_t* lab,
-                                                                 const float4* cell_axis, float4* cellsum,
-                                                                 double* gsum)
+__global__ void __launch_bounds__(kThreads) adjoint_cells_kernel(BoxDesc b, AdjointStep t, const float* dU, double w)
 {
-    __shared__ double red[kThreads];
+    adjoint_cells(b, t, dU, w);
+}
+
+// One kernel per step of the reverse sweep, between the sums of step t + 1 (hi) and
+// those of step t (lo):
+//   HI: lambda_{t+1} = R^T (mu - s_c) + s_c for the particles collided at t + 1 (R^T:
+//       rotation by -alpha), with the sums that the launch before completed;
+//   LO: mu_t = B lambda_{t+1} + sampling term; its sums over the cells of step t; dL/dg;
+//   the cells of step t - 1 (prev), which the next launch adds to.
+// Without LO the lambda are those of the segment's first step; out (or null) then takes
+// dL/dV0 = B_0 lambda_0, the bounces of the initial streaming in b0.
+// What bounds it is the latency of three random sectors a particle (its cells' AdjointCell
+// and the atomic on one) behind the tape's ids.  One launch and one pass over lambda a
+// step instead of three launches and two: 64 x 64 x 34, n = 10, 46.4 -> 24.4 us a step (28.0 with
+// the cell read as two 16-byte loads; two to four particles a thread at once: 28 to 37).
+// A cell with one 256-bit load (the cells of step hi are read-only in a sweep).
+__device__ __forceinline__ void load_cell(const AdjointCell* c, float4& sum, float4& axis)
+{
+    load_slot(reinterpret_cast<const Slot*>(c), sum, axis);
+}
+
+template <bool HI, bool LO>
+__global__ void __launch_bounds__(kThreads, 6) adjoint_sweep_kernel(BoxDesc b, uint32_t n, float4* lam, AdjointStep hi,
+                                                                    AdjointStep lo, AdjointStep prev, const float* dU,
+                                                                    double w, double* gsum, const uint32_t* b0, float* out)
+{
+    if (LO && prev.cells) adjoint_cells(b, prev, dU, w);
     double gl = 0;
+#pragma unroll 2
     for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
-        float3 m = make_float3(lam[3 * i], lam[3 * i + 1], lam[3 * i + 2]);
-        const uint32_t l = lab[i];
-        if (l & kTapeBounce) m = make_float3(-m.x, -m.y, -m.z);
-        const uint32_t c = l & ~kTapeBounce;
-        m.x += __ldg(&cell_axis[c - b.cell_base].w);
-        lam[3 * i] = m.x; lam[3 * i + 1] = m.y; lam[3 * i + 2] = m.z;
-        const uint32_t k = key[i];
-        if (k != kTapeNone) {
-            atomicAdd(cellsum + k, make_float4(m.x, m.y, m.z, 0.0f));
-            gl += (double)m.x;
+        const float4 l4 = lam[i];
+        float3 m = make_float3(l4.x, l4.y, l4.z);
+        const uint32_t kh = HI ? hi.key[i] : kTapeNone;
+        const uint32_t l = LO ? lo.lab[i] : 0u, kl = LO ? lo.key[i] : kTapeNone;
+        if (HI && kh != kTapeNone) {
+            float4 cs, ax;
+            load_cell(hi.cells + (kh - b.cell_base), cs, ax);
+            const float3 sc = make_float3(cs.x * cs.w, cs.y * cs.w, cs.z * cs.w);
+            const float3 a = make_float3(ax.x, ax.y, ax.z);
+            const float3 wv = make_float3(m.x - sc.x, m.y - sc.y, m.z - sc.z);
+            const float d = dot3(wv, a);
+            const float3 para = make_float3(a.x * d, a.y * d, a.z * d);
+            const float3 perp = make_float3(wv.x - para.x, wv.y - para.y, wv.z - para.z);
+            const float3 cr = cross3(wv, a);
+            m = make_float3((para.x + b.cos_a * perp.x) - b.sin_a * cr.x + sc.x,
+                            (para.y + b.cos_a * perp.y) - b.sin_a * cr.y + sc.y,
+                            (para.z + b.cos_a * perp.z) - b.sin_a * cr.z + sc.z);
+        }
+        if (LO) {
+            if (l & kTapeBounce) m = make_float3(-m.x, -m.y, -m.z);
+            m.x += __ldcg(&lo.cells[(l & ~kTapeBounce) - b.cell_base].axis.w);
+            if (kl != kTapeNone) {
+                atomicAdd(&lo.cells[kl - b.cell_base].sum, make_float4(m.x, m.y, m.z, 0.0f));
+                gl += (double)m.x;
+            }
+        }
+        if (!LO && out) {
+            const float f = (b0[i] & kTapeBounce) ? -1.0f : 1.0f;
+            out[3 * (uint64_t)i] = f * m.x;
+            out[3 * (uint64_t)i + 1] = f * m.y;
+            out[3 * (uint64_t)i + 2] = f * m.z;
+        } else {
+            lam[i] = make_float4(m.x, m.y, m.z, 0.0f);
         }
     }
-    red[threadIdx.x] = gl;
-    __syncthreads();
-    for (int o = kThreads / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+    if (LO) {
+        __shared__ double red[kThreads / 32];
+#pragma unroll
+        for (int o = 16; o; o >>= 1) gl += __shfl_xor_sync(kFull, gl, o);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = gl;
         __syncthreads();
-    }
-    if (threadIdx.x == 0) atomicAdd(gsum, red[0]);
-}
-
-// lambda = R^T (mu - s_c) + s_c for collided particles (R^T: rotation by -alpha).
-__global__ void __launch_bounds__(kThreads) adjoint_pass2_kernel(BoxDesc b, uint32_t n, float* lam,
-                                                                 const uint32_t* key, const uint32_t* ncell,
-                                                                 const float4* cellsum, const float4* cell_axis)
-{
-    for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
-        const uint32_t k = key[i];
-        if (k == kTapeNone) continue;
-        const float inv = 1.0f / (float)ncell[k];
-        const float4 cs = cellsum[k];
-        const float3 sc = make_float3(cs.x * inv, cs.y * inv, cs.z * inv);
-        const float4 ax = __ldg(&cell_axis[k - b.cell_base]);
-        const float3 a = make_float3(ax.x, ax.y, ax.z);
-        const float3 wv = make_float3(lam[3 * i] - sc.x, lam[3 * i + 1] - sc.y, lam[3 * i + 2] - sc.z);
-        const float d = dot3(wv, a);
-        const float3 para = make_float3(a.x * d, a.y * d, a.z * d);
-        const float3 perp = make_float3(wv.x - para.x, wv.y - para.y, wv.z - para.z);
-        const float3 cr = cross3(wv, a);
-        lam[3 * i] = (para.x + b.cos_a * perp.x) - b.sin_a * cr.x + sc.x;
-        lam[3 * i + 1] = (para.y + b.cos_a * perp.y) - b.sin_a * cr.y + sc.y;
-        lam[3 * i + 2] = (para.z + b.cos_a * perp.z) - b.sin_a * cr.z + sc.z;
-    }
-}
-
-// dL/dV0 = B_0 lambda_0.
-__global__ void __launch_bounds__(kThreads) adjoint_finish_kernel(uint32_t n, const float* lam, const uint32_t* b0,
-                                                                  float* out)
-{
-    for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
-        const float f = (b0[i] & kTapeBounce) ? -1.0f : 1.0f;
-        out[3 * i] = f * lam[3 * i];
-        out[3 * i + 1] = f * lam[3 * i + 1];
-        out[3 * i + 2] = f * lam[3 * i + 2];
+        if (threadIdx.x == 0) {
+            double g = 0;
+            for (int q = 0; q < kThreads / 32; ++q) g += red[q];
+            atomicAdd(gsum, g);
+        }
     }
 }
 
@@ -2721,22 +2732,22 @@ cudaError_t launch_profile(const SampleAcc* acc, const BoxDesc& b, uint64_t samp
     return cudaGetLastError();
 }
 
-cudaError_t launch_adjoint_step(const BoxDesc& b, uint64_t step, uint64_t samples, float* lam, const uint32_t* key,
-                                const uint32_t* lab, const uint32_t* ncell, const uint32_t* lab_count,
-                                const float* dU, float4* cellsum, double* gsum, int grid, cudaStream_t st)
+cudaError_t launch_adjoint_cells(const BoxDesc& b, const AdjointStep& t, uint64_t samples, const float* dU, int grid,
+                                 cudaStream_t st)
 {
     const double w = 1.0 / ((double)samples * (double)b.L[0] * (double)b.L[1]);
-    float4* const cell_axis = cellsum + b.C;
-    adjoint_cells_kernel<<<grid, kThreads, 0, st>>>(b, step, lab_count, dU, w, cellsum, cell_axis);
-    adjoint_pass1_kernel<<<grid, kThreads, 0, st>>>(b, b.N, lam, key, lab, cell_axis, cellsum, gsum);
-    adjoint_pass2_kernel<<<grid, kThreads, 0, st>>>(b, b.N, lam, key, ncell, cellsum, cell_axis);
+    adjoint_cells_kernel<<<grid, kThreads, 0, st>>>(b, t, dU, w);
     return cudaGetLastError();
 }
 
-cudaError_t launch_adjoint_finish(uint32_t n, const float* lam, const uint32_t* b0, float* out, int grid,
-                                  cudaStream_t st)
+cudaError_t launch_adjoint_sweep(const BoxDesc& b, uint64_t samples, float4* lam, const AdjointStep* hi,
+                                 const AdjointStep* lo, const AdjointStep* prev, const float* dU, double* gsum,
+                                 const uint32_t* b0, float* out, int grid, cudaStream_t st)
 {
-    adjoint_finish_kernel<<<grid, kThreads, 0, st>>>(n, lam, b0, out);
+    const double w = 1.0 / ((double)samples * (double)b.L[0] * (double)b.L[1]);
+    const AdjointStep none{};
+    auto f = hi ? (lo ? adjoint_sweep_kernel<true, true> : adjoint_sweep_kernel<true, false>) : adjoint_sweep_kernel<false, true>;
+    f<<<grid, kThreads, 0, st>>>(b, b.N, lam, hi ? *hi : none, lo ? *lo : none, prev ? *prev : none, dU, w, gsum, b0, out);
     return cudaGetLastError();
 }
 

@@ -57,15 +57,15 @@ cudaError_t launch_sample_finalize(float4* samp, SampleAcc* acc, uint64_t cells,
 cudaError_t launch_mean_fields(const SampleAcc* acc, const BoxDesc& b, double inverse, float* density, float* velocity,
                                cudaStream_t st);
 // Adjoint of the sampled x-velocity profile (single box, SRD): U(z) from the sample
-// sums of `samples` steps; one reverse step (both passes) at absolute step `step`;
-// dL/dV0 from the final adjoint and the bounce bits of the initial streaming.
+// sums of `samples` steps; the cells of a step before its sweep; one launch of the
+// reverse sweep: the end of step hi (or null) and the start of step lo (or null), the
+// cells of step prev on the way (or null); the last launch writes dL/dV0 to out.
 cudaError_t launch_profile(const SampleAcc* acc, const BoxDesc& b, uint64_t samples, float* profile, cudaStream_t st);
-// cellsum: 2 C entries (the cell sums of mu, then each cell's axis and sampling term).
-cudaError_t launch_adjoint_step(const BoxDesc& b, uint64_t step, uint64_t samples, float* lam, const uint32_t* key,
-                                const uint32_t* lab, const uint32_t* ncell, const uint32_t* lab_count,
-                                const float* dU, float4* cellsum, double* gsum, int grid, cudaStream_t st);
-cudaError_t launch_adjoint_finish(uint32_t n, const float* lam, const uint32_t* b0, float* out, int grid,
-                                  cudaStream_t st);
+cudaError_t launch_adjoint_cells(const BoxDesc& b, const AdjointStep& t, uint64_t samples, const float* dU, int grid,
+                                 cudaStream_t st);
+cudaError_t launch_adjoint_sweep(const BoxDesc& b, uint64_t samples, float4* lam, const AdjointStep* hi,
+                                 const AdjointStep* lo, const AdjointStep* prev, const float* dU, double* gsum,
+                                 const uint32_t* b0, float* out, int grid, cudaStream_t st);
 // Layout dump, after the step's overflow selection: cells in storage order, stable
 // order within a cell (decoupled look-back scan of the counts, then one thread per
 // cell), then the overflow list's particles that do not collide, in any order;

@@ -183,6 +183,7 @@ struct StepArgs {
     float4* fold_samp;
     SampleAcc* acc;
     uint64_t fold_cells;          // cells of fold_samp (all boxes)
+    uint32_t* fold_count;         // taped steps: lab counts of the folded sample
     float ext_axis[13][3];        // discrete axis set of the extended collision
     DrawTables draws;             // used by the injected-draw instantiation
     // adjoint tape of this step, by particle id / cell (null: not recorded):
@@ -216,5 +217,19 @@ constexpr int32_t kRunSrd = 1, kRunExtended = 2;   // StepArgs::run_kernel
 constexpr uint32_t kExtMaxN = 36;                  // densities that ext_run_kernel takes
 constexpr uint32_t kTapeNone = 0xFFFFFFFFu;
 constexpr uint32_t kTapeBounce = 0x80000000u;
+
+// Adjoint sweep, a cell at one step: the sums of mu over its collided particles and
+// 1 / N_c in sum.w; the rotation axis (as a collision cell), and in axis.w its sampling
+// term dU(z) / (samples Lx Ly count) (as a lab cell).
+struct alignas(32) AdjointCell {
+    float4 sum, axis;
+};
+
+// One step of the adjoint tape (by particle id / storage cell) and its cells.
+struct AdjointStep {
+    uint64_t step;
+    const uint32_t *key, *lab, *ncell, *lab_count;
+    AdjointCell* cells;
+};
 
 }  // namespace mpcd_gb

@@ -228,8 +228,10 @@ int32_t mpcd_gb_set_drag(mpcd_gb_handle *h, float drag);
  * dL/d(drag) (host double).  Collision cells, grid shifts, rotation axes, ghost counts
  * and wall bounces are held fixed at those of the forward trajectory: each checkpoint
  * segment is recomputed (its draws replayed from the Philox counters) and then swept
- * in reverse.  Afterwards the handle's particle state is that of an intermediate step;
- * set the particles again before stepping on. */
+ * in reverse.  A forward whose events fit 4 GiB (8 bytes per particle and per cell a step)
+ * keeps them instead of checkpoints, and nothing is recomputed.  Afterwards the handle's
+ * particle state is that of some step of the forward; set the particles again before
+ * stepping on. */
 int32_t mpcd_gb_profile_forward(mpcd_gb_handle *h, int32_t steps, int32_t checkpoint_every, float *d_profile);
 int32_t mpcd_gb_profile_backward(mpcd_gb_handle *h, const float *d_grad_profile, float *d_grad_velocities,
                                  double *grad_drag);
