@@ -1044,8 +1044,8 @@ private:
             check(count_[k].alloc(sizeof(uint32_t) * cells_), "alloc counts");
             check(cudaMemset(count_[k].p, 0, count_[k].bytes), "clear counts");
         }
-        if (walls_) check(ghosts_.alloc(sizeof(GhostSum) * walls_), "alloc wall ghosts");
-        check(box_shifts_.alloc(sizeof(float4) * 2 * boxes_.size()), "alloc box shifts");
+        if (walls_) check(ghosts_.alloc(sizeof(GhostSum) * walls_ * 2), "alloc wall ghosts");   // two parities
+        check(box_shifts_.alloc(sizeof(float4) * 4 * boxes_.size()), "alloc box shifts");
         check(state_.alloc(sizeof(DeviceState)), "alloc state");
         check(cudaMallocHost((void**)&flags_host_, sizeof *flags_host_), "alloc error flags");
         check(cudaMemset(state_.p, 0, sizeof(DeviceState)), "clear state");
@@ -1117,8 +1117,8 @@ private:
         for (int c = 0; c < 4; ++c) a.run_class[c] = run_class_[c];
         a.boxes_n_max = n_max_;
         a.total_walls = walls_;
-        a.ghosts = ghosts_.as<GhostSum>();
-        a.box_shifts = box_shifts_.as<float4>();
+        a.ghosts = walls_ ? ghosts_.as<GhostSum>() + (k & 1) * walls_ : nullptr;
+        a.box_shifts = box_shifts_.as<float4>() + (k & 1) * 2 * boxes_.size();
         a.total_slots = total_slots_;
         a.ext_cap = ext_cap_;
         a.step = k;

@@ -109,6 +109,13 @@ __device__ __forceinline__ void store_slot(Slot* dst, float4 p, float4 v)
                  : "memory");
 }
 
+// Programmatic dependent launch: a kernel launched so (launch_overlapped) may start while
+// the one before it in the stream runs, once every block of that one has called
+// let_next_start(); wait_for_previous() returns when it has completed and its writes are
+// visible.  Both do nothing after an ordinary launch.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ unsigned lanemask_lt()
 {
     unsigned m;
@@ -1270,32 +1277,32 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
     __shared__ float shared_rows[REPLAY ? kRunWarps : 1][96];
     RunShared& sh = shared_runs[threadIdx.x >> 5];
     BoxDesc& sbox = shared_box[SINGLE ? 0 : threadIdx.x >> 5];
-    const uint64_t step = a.step_base ? *a.step_base + a.step : a.step;   // graph replays read the base
-
-    const uint32_t left = a.state->ov[a.ov_in_slot].left;
     constexpr uint32_t kBatchCells = BATCH;
     constexpr uint32_t kBatchLanes = 32 / BATCH;   // lanes per cell in the sums
     static_assert(BATCH == 4 || BATCH == 8 || BATCH == 16, "batches of 4, 8 or 16 cells");
     // single box: geometry straight from the kernel parameters (constant bank)
     const BoxDesc& b = SINGLE ? a.box0 : sbox;
-    if (SINGLE) {   // drawn by the prologue
-        if (threadIdx.x < 2) shared_shifts[0][threadIdx.x] = __ldg(a.box_shifts + threadIdx.x);
-        __syncthreads();
-    }
-    if (first_launch) {   // once per step (ensembles launch once per batch size)
-        if (!REPLAY && blockIdx.x == 0 && threadIdx.x == 0) {   // list of step k-1, refilled by step k+1
-            a.state->ov[a.ov_zero_slot] = OverflowFill{0u, 0u};
-        }
-        if (left) overflow_pass(a, step);
-    }
-    int cur_box = -1;
+    wait_for_previous();   // the prologue, and with it the step before
+    let_next_start();      // the next prologue, which draws while this sweeps
     const uint32_t warps = gridDim.x * (uint32_t)kRunWarps;
     uint32_t run = run_begin + blockIdx.x * (uint32_t)kRunWarps + (threadIdx.x >> 5);
     uint2 next = run_entry<SINGLE>(a, run < run_end ? run : a.num_runs);
     uint32_t raw_next = lane < (next.y & 63u) ? a.in_count[next.x + lane] : 0u;   // counts one run ahead
+    const uint64_t step = a.step_base ? *a.step_base + a.step : a.step;   // graph replays read the base
+    const uint32_t left = a.state->ov[a.ov_in_slot].left;
+    if (SINGLE) {   // drawn by the prologue
+        if (threadIdx.x < 2) shared_shifts[0][threadIdx.x] = a.box_shifts[threadIdx.x];
+        __syncthreads();
+    }
     if (SINGLE && lane < kBatchCells && raw_next)   // the first batch of the first run
         prefetch_l2(a.in_slots + b.slot_base + (uint64_t)(next.x - b.cell_base + lane) * b.depth,
                     min(raw_next, b.depth) * (uint32_t)sizeof(Slot));
+    if (first_launch) {   // once per step (ensembles launch once per batch size)
+        if (!REPLAY && blockIdx.x == 0 && threadIdx.x == 0)   // list of step k-1, refilled by step k+1
+            a.state->ov[a.ov_zero_slot] = OverflowFill{0u, 0u};
+        if (left) overflow_pass(a, step);
+    }
+    int cur_box = -1;
 
     for (; run < run_end; run += warps) {
         const uint2 cur = next;
@@ -1570,12 +1577,14 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
     const uint32_t lane = threadIdx.x & 31u;
     ExtShared& sh = reinterpret_cast<ExtShared*>(dyn)[threadIdx.x >> 5];
     BoxDesc& sbox = shared_box[SINGLE ? 0 : threadIdx.x >> 5];
+    wait_for_previous();   // the prologue, and with it the step before
+    let_next_start();      // the next prologue, which draws while this sweeps
     const uint64_t step = a.step_base ? *a.step_base + a.step : a.step;   // graph replays read the base
     const uint32_t left = a.state->ov[a.ov_in_slot].left;
     const BoxDesc& b = SINGLE ? a.box0 : sbox;
     float3 s = make_float3(0, 0, 0), sn = s;
     if (SINGLE) {
-        const float4 s0 = __ldg(a.box_shifts), s1 = __ldg(a.box_shifts + 1);   // drawn by the prologue
+        const float4 s0 = a.box_shifts[0], s1 = a.box_shifts[1];   // drawn by the prologue
         s = make_float3(s0.x, s0.y, s0.z);
         sn = make_float3(s1.x, s1.y, s1.z);
     }
@@ -2006,9 +2015,14 @@ __global__ void __launch_bounds__(kThreads) overflow_select_kernel(const StepArg
             a.ghosts[wg] = r;
         }
     }
+    // The draws depend on no earlier launch, and the arrays they fill alternate by step
+    // parity (the step before reads the others), so they run beside the step kernel
+    // before this prologue; the selection needs its claims.
+    wait_for_previous();
     const uint32_t par = (uint32_t)(a.step & 1u);
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.state->ext_count[par ^ 1u] = 0;
     const uint32_t n = min(a.state->ov[a.ov_in_slot].count, a.ov_cap);
+    if (n == 0) let_next_start();   // (with entries to place, the step kernel starts when all are placed)
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.state->ext_count[par ^ 1u] = 0;
     const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (uint32_t)(kThreads / 32);
     const uint32_t warp = (gridDim.x - 1u - blockIdx.x) * (uint32_t)(kThreads / 32) + (threadIdx.x >> 5);
     const uint32_t per = min(32u, (n + warps - 1u) / warps);   // entries a warp looks at together
@@ -2597,6 +2611,24 @@ static const StepFnExt kExtFns[2][2] = {{ext_run_kernel<false, false, false>, ex
                                         {ext_run_kernel<true, false, false>, ext_run_kernel<true, true, false>}};
 static const StepFnExt kExtReplayFns[2] = {ext_run_kernel<false, false, true>, ext_run_kernel<false, true, true>};
 
+// Launch that may overlap the end of the kernel before it in the stream (a kernel that
+// calls wait_for_previous before it reads what that one wrote).
+template <class... P, class... A>
+static cudaError_t launch_overlapped(void (*f)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t st, A... args)
+{
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = attr;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, f, static_cast<P>(args)...);
+}
+
 bool run_kernel_takes(const StepArgs& a, int algorithm, bool table)
 {
     if (algorithm == 1)
@@ -2613,6 +2645,7 @@ cudaError_t launch_step(const StepArgs& a, int algorithm, bool table, uint32_t p
     if (a.run_kernel == kRunExtended) {
         const unsigned blocks = std::min((unsigned)grid, (a.num_runs + kExtWarps - 1) / (unsigned)kExtWarps);
         const StepFnExt f = a.replay ? kExtReplayFns[a.nboxes == 1 ? 1 : 0] : kExtFns[a.sample ? 1 : 0][a.nboxes == 1 ? 1 : 0];
+        if (a.nboxes == 1 && !a.replay) return launch_overlapped(f, blocks, kExtThreads, kExtWarps * sizeof(ExtShared), st, a);
         f<<<blocks, kExtThreads, kExtWarps * sizeof(ExtShared), st>>>(a);
         return cudaGetLastError();
     }
@@ -2637,6 +2670,11 @@ cudaError_t launch_step(const StepArgs& a, int algorithm, bool table, uint32_t p
             const StepFnRun f = a.replay ? kRunReplayFns[single][cls] : a.tape_key ? kRunTapeFns[cls] : kRunFns[a.sample ? 1 : 0][single][cls];
             const uint32_t runs = a.run_class[cls + 1] - a.run_class[cls];
             const unsigned blocks = std::min((unsigned)grid, (runs + kRunWarps - 1) / (unsigned)kRunWarps);
+            if (a.nboxes == 1 && !a.replay) {   // (an ensemble's classes fork and join)
+                e = launch_overlapped(f, blocks, kThreads, 0, st, a, a.run_class[cls], a.run_class[cls + 1], i == 0);
+                if (e != cudaSuccess) return e;
+                continue;
+            }
             f<<<blocks, kThreads, 0, fork && i > 0 ? branches->side[i - 1] : st>>>(a, a.run_class[cls],
                                                                                     a.run_class[cls + 1], i == 0);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -2773,6 +2811,8 @@ cudaError_t launch_scatter(const StepArgs& a, const float* pos, const float* vel
 cudaError_t launch_overflow_select(const StepArgs& a, Slot* in_slots, float4* ov_pos, float4* ov_vel,
                                    uint32_t* ov_head, int grid, cudaStream_t st)
 {
+    if (a.nboxes == 1)
+        return launch_overlapped(overflow_select_kernel, (unsigned)grid, kThreads, 0, st, a, in_slots, ov_pos, ov_vel, ov_head);
     overflow_select_kernel<<<grid, kThreads, 0, st>>>(a, in_slots, ov_pos, ov_vel, ov_head);
     return cudaGetLastError();
 }

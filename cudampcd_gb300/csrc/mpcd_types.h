@@ -200,7 +200,8 @@ struct StepArgs {
     // (bounce-backs and collisions in the wall-layer cells) into state->wall_impulse
     int32_t pressure;
     // srd_run_kernel steps: the wall ghosts of step k, drawn by the step's
-    // prologue (overflow_select_kernel), entry wall_base + 2 (x + Lx y) + top
+    // prologue (overflow_select_kernel), entry wall_base + 2 (x + Lx y) + top; the
+    // array of the step's parity
     GhostSum* ghosts;
     // runs of up to 32 consecutive cells of one box (srd_run_kernel): per run
     // {first global cell, cells | box << 6}; a single box computes them
