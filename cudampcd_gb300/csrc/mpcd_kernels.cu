@@ -104,7 +104,7 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 // One bucket slot (32 bytes, a full sector) with a single 256-bit store.
 __device__ __forceinline__ void store_slot(Slot* dst, float4 p, float4 v)
 {
-    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "f"(p.x), "f"(p.y), "f"(p.z),
+    asm volatile("st.global.L1::no_allocate.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "f"(p.x), "f"(p.y), "f"(p.z),
                  "f"(p.w), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
                  : "memory");
 }
@@ -1203,8 +1203,10 @@ __global__ void __launch_bounds__(kThreads, 4) step_kernel(const StepArgs a, uin
 //   a batch of 4, 8 or 16 cells (about 80 particles) at a time with 32 / batch
 //   lanes per cell and four loads in flight each, so that the group's slots are
 //   still in L1 from the sums.  Each batch asks L2 for the next batch's buckets.
+//   STAGED (ensembles): a ring of 160 particles per warp in shared memory instead, which
+//   asynchronous copies fill a batch ahead; sums and finish both read it.
 // The arithmetic is step_kernel's (the same helpers), so a replay of this step
-// by step_kernel (the getters) reproduces it bit for bit.
+// by either kernel (the getters) reproduces it bit for bit.
 
 constexpr uint32_t kRunCells = 32;
 // Cells summed together: BATCH = 4, 8 or 16, about 80 particles per batch (the
@@ -1217,6 +1219,24 @@ struct RunShared {                   // one per warp
     float4 axis[kRunCells];          // rotation axis
     long long gsum[kRunCells][3];    // exact velocity sums of the cell's ghosts
 };
+
+// A warp's particles in flight (STAGED), run particle t in place t mod kRing.
+constexpr uint32_t kRing = 160;
+constexpr uint32_t kRingMaxN = 32;   // 31 particles of an unfinished pass and a cell's 4n fit
+static_assert(kRing % 32 == 0 && 31 + 4 * kRingMaxN <= kRing, "a pass and a cell fit the ring");
+struct RunRing {
+    float4 pos[kRing], vel[kRing];
+};
+
+// 16 bytes of global memory into shared memory, asynchronously (committed in groups).
+__device__ __forceinline__ void copy_async16(void* dst, const void* src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// All groups but the last `N` have landed.
+template <int N>
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // Bring `bytes` (a multiple of 16, 16-byte aligned) of global memory into L2.
 __device__ __forceinline__ void prefetch_l2(const void* src, uint32_t bytes)
@@ -1265,17 +1285,18 @@ __device__ __forceinline__ void write_rows(float* stage, float* dense, uint32_t 
     __syncwarp();
 }
 
-template <bool SAMPLE, bool SINGLE, uint32_t BATCH, int MODE = kPlain>
+template <bool SAMPLE, bool SINGLE, uint32_t BATCH, int MODE = kPlain, bool STAGED = !SINGLE>
 __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, uint32_t run_begin, uint32_t run_end,
                                                               bool first_launch)
 {
-    __shared__ RunShared shared_runs[kRunWarps];
+    extern __shared__ __align__(128) unsigned char dyn[];   // RunShared of every warp, then RunRing of every warp
     __shared__ __align__(16) BoxDesc shared_box[SINGLE ? 1 : kRunWarps];   // ensembles: the box of the warp's run
     __shared__ float4 shared_shifts[SINGLE ? 1 : kRunWarps][2];              // and its grid shifts of steps k and k+1
     const uint32_t lane = threadIdx.x & 31u;
     constexpr bool TAPE = MODE == kTape, REPLAY = MODE == kReplay;
-    __shared__ float shared_rows[REPLAY ? kRunWarps : 1][96];
-    RunShared& sh = shared_runs[threadIdx.x >> 5];
+    RunShared& sh = reinterpret_cast<RunShared*>(dyn)[threadIdx.x >> 5];
+    RunRing& ring = reinterpret_cast<RunRing*>(dyn + kRunWarps * sizeof(RunShared))[STAGED ? threadIdx.x >> 5 : 0];
+    __shared__ float shared_rows[REPLAY && !STAGED ? kRunWarps : 1][96];
     BoxDesc& sbox = shared_box[SINGLE ? 0 : threadIdx.x >> 5];
     constexpr uint32_t kBatchCells = BATCH;
     constexpr uint32_t kBatchLanes = 32 / BATCH;   // lanes per cell in the sums
@@ -1294,7 +1315,7 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
         if (threadIdx.x < 2) shared_shifts[0][threadIdx.x] = a.box_shifts[threadIdx.x];
         __syncthreads();
     }
-    if (SINGLE && lane < kBatchCells && raw_next)   // the first batch of the first run
+    if (!STAGED && SINGLE && lane < kBatchCells && raw_next)   // the first batch of the first run
         prefetch_l2(a.in_slots + b.slot_base + (uint64_t)(next.x - b.cell_base + lane) * b.depth,
                     min(raw_next, b.depth) * (uint32_t)sizeof(Slot));
     if (first_launch) {   // once per step (ensembles launch once per batch size)
@@ -1375,6 +1396,28 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
         const uint32_t rel = src_slot - (incl - cnt);
         uint32_t summed = 0;           // cells [0, summed) have their means in sh.cell
         bool next_prefetched = false;  // the next run's first batch was asked of L2
+        // STAGED: cells [summed, a_end) are the batch to sum next, cells [a_end, b_end) the
+        // one after, their copies under way; gpos: the pass's place in the ring
+        uint32_t a_end = 0, b_end = 0, gpos = 0;
+        const uint32_t in_ring = (incl - cnt) % kRing, len = cur.y & 63u;
+        auto fetch = [&](uint32_t g0, bool need = false) {   // copy another batch, once it fits beside the particles from g0 on (need: what of it fits)
+            if (b_end > a_end || b_end >= len) return;
+            const uint32_t fit = __popc(__ballot_sync(kFull, lane >= b_end && lane < min(b_end + kBatchCells, len) && incl - g0 <= kRing));
+            if (fit == 0 || (!need && fit < min(kBatchCells, len - b_end))) return;
+            const uint32_t q = lane / kBatchLanes, L = (b_end + q) & 31u;
+            uint32_t n = __shfl_sync(kFull, cnt, (int)L), place = __shfl_sync(kFull, in_ring, (int)L) + lane % kBatchLanes;
+            const Slot* src = a.in_slots + __shfl_sync(kFull, src_slot, (int)L);
+            n = q < fit ? n : 0u;
+            for (uint32_t t = lane % kBatchLanes; t < n; t += kBatchLanes, place += kBatchLanes) {
+                const uint32_t w = place >= kRing ? place - kRing : place;
+                copy_async16(&ring.pos[w], &src[t].pos);
+                copy_async16(&ring.vel[w], &src[t].vel);
+            }
+            copy_async_commit();
+            if (a_end == summed) a_end += fit;
+            b_end += fit;
+        };
+        if (STAGED && total) fetch(0, true);
         // 32 particles at a time, across batch boundaries
         for (uint32_t g0 = 0; g0 < total; g0 += 32) {
             // lanes past the run's last particle redo that particle and write nothing
@@ -1386,10 +1429,28 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
             const uint32_t hi = __popc(__ballot_sync(kFull, incl <= min(g0 + 31u, total - 1u)));
             // exact sums and means of every cell up to hi, a batch of BATCH cells at a
             // time (kBatchLanes lanes per cell); each batch asks L2 for the next one's buckets
+            if (STAGED) {
+                __syncwarp();   // every lane has read the particles of the pass before
+                fetch(g0);
+            }
             while (summed <= hi) {
                 const uint32_t c8 = summed;
-                summed += kBatchCells;
-                if (c8 + kBatchCells < (cur.y & 63u)) {
+                uint32_t c_end = c8 + kBatchCells;
+                if (STAGED) {
+                    if (a_end == summed) {   // fits: the cell starts within this pass
+                        fetch(g0, true);
+                        if (a_end == summed) {   // (impossible while a cell holds at most 4 kRingMaxN)
+                            if (lane == 0) atomicOr(&a.state->error_flags, kErrKeyMismatch);
+                            return;
+                        }
+                    }
+                    if (b_end > a_end) copy_async_wait<1>();
+                    else copy_async_wait<0>();
+                    __syncwarp();
+                    summed = c_end = a_end;
+                    a_end = b_end;
+                    fetch(g0);
+                } else if (summed += kBatchCells, c8 + kBatchCells < (cur.y & 63u)) {
                     if (lane >= c8 + kBatchCells && lane < c8 + 2 * kBatchCells && cnt)
                         prefetch_l2(a.in_slots + src_slot, cnt * (uint32_t)sizeof(Slot));
                 } else {
@@ -1399,15 +1460,23 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
                                     min(raw_next, b.depth) * (uint32_t)sizeof(Slot));
                 }
                 const uint32_t L = c8 + lane / kBatchLanes, jl = lane % kBatchLanes;
-                const uint32_t cntL = __shfl_sync(kFull, cnt, (int)L), mL = __shfl_sync(kFull, m, (int)L);
-                const Slot* src = a.in_slots + __shfl_sync(kFull, src_slot, (int)L);
+                uint32_t cntL = __shfl_sync(kFull, cnt, (int)(L & 31u));
+                const uint32_t mL = __shfl_sync(kFull, m, (int)(L & 31u));
+                const Slot* src = STAGED ? nullptr : a.in_slots + __shfl_sync(kFull, src_slot, (int)L);
+                const uint32_t place = STAGED ? __shfl_sync(kFull, in_ring, (int)(L & 31u)) : 0u;
+                if (STAGED && L >= c_end) cntL = 0;
+                auto velocity = [&](uint32_t t) -> float4 {
+                    if (!STAGED) return __ldg(&src[t].vel);
+                    const uint32_t w = place + t;
+                    return ring.vel[w >= kRing ? w - kRing : w];
+                };
                 long long sx = 0, sy = 0, sz = 0;
                 float mx = 0.0f;
                 for (uint32_t j = jl; j < cntL; j += 4 * kBatchLanes) {   // four loads in flight per lane
                     float4 v[4];
 #pragma unroll
                     for (uint32_t u = 0; u < 4; ++u)
-                        v[u] = j + u * kBatchLanes < cntL ? __ldg(&src[j + u * kBatchLanes].vel) : make_float4(0, 0, 0, 0);
+                        v[u] = j + u * kBatchLanes < cntL ? velocity(j + u * kBatchLanes) : make_float4(0, 0, 0, 0);
                     int px = 0, py = 0, pz = 0;
 #pragma unroll
                     for (uint32_t u = 0; u < 4; ++u) {
@@ -1422,7 +1491,7 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
                 if (__any_sync(kFull, mx >= kNarrowLimit)) {   // a speed of 32 or more in the batch: 64-bit sums
                     sx = sy = sz = 0;
                     for (uint32_t j = jl; j < cntL; j += kBatchLanes) {
-                        const float4 v = __ldg(&src[j].vel);
+                        const float4 v = velocity(j);
                         sx += fixed24(v.x);
                         sy += fixed24(v.y);
                         sz += fixed24(v.z);
@@ -1434,7 +1503,7 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
                     sy += __shfl_xor_sync(kFull, sy, (int)o);
                     sz += __shfl_xor_sync(kFull, sz, (int)o);
                 }
-                if (jl == 0) {
+                if (jl == 0 && (!STAGED || L < c_end)) {
                     sx += sh.gsum[L][0];
                     sy += sh.gsum[L][1];
                     sz += sh.gsum[L][2];
@@ -1459,12 +1528,17 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
                 for (uint32_t half = 16; half; half >>= 1)
                     i += t >= __shfl_sync(kFull, incl, (int)(i + half - 1)) ? half : 0u;
             }
-            const uint32_t slot = __shfl_sync(kFull, rel, (int)(i & 31u)) + t;
+            const uint32_t slot = STAGED ? 0u : __shfl_sync(kFull, rel, (int)(i & 31u)) + t;
             uint32_t key = 0, id = 0;
             float3 xn = make_float3(0, 0, 0), vn = xn;
             {
                 float4 xp, vp;
-                load_slot(a.in_slots + slot, xp, vp);
+                if (STAGED) {
+                    xp = ring.pos[gpos + (t - g0)];
+                    vp = ring.vel[gpos + (t - g0)];
+                } else {
+                    load_slot(a.in_slots + slot, xp, vp);
+                }
                 const float4 cd = sh.cell[i];
                 const float4 ax = sh.axis[i];
                 float3 x = make_float3(xp.x, xp.y, xp.z), v = make_float3(vp.x, vp.y, vp.z);
@@ -1479,9 +1553,12 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
                 }
                 if (REPLAY) {
                     const unsigned rows = __ballot_sync(kFull, active);
-                    float* const stage = shared_rows[REPLAY ? threadIdx.x >> 5 : 0];
+                    // staged in the places of the pass, which every lane has read
+                    float* const stage = STAGED ? &ring.pos[gpos].x : shared_rows[REPLAY && !STAGED ? threadIdx.x >> 5 : 0];
+                    __syncwarp();
                     write_rows(stage, a.dense_pos, __float_as_uint(vp.w), x, rows);
                     write_rows(stage, a.dense_vel, __float_as_uint(vp.w), v, rows);
+                    gpos = gpos + 32 == kRing ? 0u : gpos + 32;
                     continue;
                 }
                 vn = v;
@@ -1498,6 +1575,7 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
                 }
             }
             store_particle(a, b, xn, vn, id, key, active);
+            gpos = gpos + 32 == kRing ? 0u : gpos + 32;
         }
         // a run whose last cells are empty: the next run's first batch
         if (SINGLE && !next_prefetched && lane < kBatchCells && raw_next)
@@ -2591,19 +2669,34 @@ const StepFn kStepFns[2][2][2][2] = {
 }  // namespace
 
 using StepFnRun = void (*)(const StepArgs, uint32_t, uint32_t, bool);
-// [sample][single box][batch class: 16, 8, 4 cells]
-// single-box sampled steps that record the adjoint tape, by batch size
-static const StepFnRun kRunTapeFns[3] = {srd_run_kernel<true, true, 16, kTape>, srd_run_kernel<true, true, 8, kTape>,
-                                         srd_run_kernel<true, true, 4, kTape>};
-// replays: [single box][batch class]
-static const StepFnRun kRunReplayFns[2][3] = {
-    {srd_run_kernel<false, false, 16, kReplay>, srd_run_kernel<false, false, 8, kReplay>, srd_run_kernel<false, false, 4, kReplay>},
-    {srd_run_kernel<false, true, 16, kReplay>, srd_run_kernel<false, true, 8, kReplay>, srd_run_kernel<false, true, 4, kReplay>}};
-static const StepFnRun kRunFns[2][2][3] = {
-    {{srd_run_kernel<false, false, 16>, srd_run_kernel<false, false, 8>, srd_run_kernel<false, false, 4>},
-     {srd_run_kernel<false, true, 16>, srd_run_kernel<false, true, 8>, srd_run_kernel<false, true, 4>}},
-    {{srd_run_kernel<true, false, 16>, srd_run_kernel<true, false, 8>, srd_run_kernel<true, false, 4>},
-     {srd_run_kernel<true, true, 16>, srd_run_kernel<true, true, 8>, srd_run_kernel<true, true, 4>}}};
+// [batch class: 16, 8, 4 cells, and 4 cells unstaged (n > kRingMaxN)], single box or not
+template <bool SAMPLE, bool SINGLE, int MODE>
+static StepFnRun run_fn(int cls, bool staged)
+{
+    if (cls == 0) return srd_run_kernel<SAMPLE, SINGLE, 16, MODE>;
+    if (cls == 1) return srd_run_kernel<SAMPLE, SINGLE, 8, MODE>;
+    return SINGLE || staged ? srd_run_kernel<SAMPLE, SINGLE, 4, MODE> : srd_run_kernel<SAMPLE, SINGLE, 4, MODE, false>;
+}
+
+// The instance of a batch class: a replay, a step that records the adjoint tape (one
+// sampled box), or a plain step.
+static StepFnRun run_fn(int cls, bool staged, bool sample, bool single, bool replay, bool tape)
+{
+    if (replay) return single ? run_fn<false, true, kReplay>(cls, staged) : run_fn<false, false, kReplay>(cls, staged);
+    if (tape) return run_fn<true, true, kTape>(cls, staged);
+    if (sample) return single ? run_fn<true, true, kPlain>(cls, staged) : run_fn<true, false, kPlain>(cls, staged);
+    return single ? run_fn<false, true, kPlain>(cls, staged) : run_fn<false, false, kPlain>(cls, staged);
+}
+
+// Ensembles stage their particles through the ring, a single box does not: us a step,
+// unstaged and staged, 64 uneven channels 1144 and 978 (sampled 1399 and 1196); 500 x 500
+// x 22, n = 20 1478 and 1544 (1780 and 1862); 300 x 300 x 102, n = 10 1572 and 1552 (1900
+// and 1931).  Staging spares the finish its slot loads, of which only 30 % hit L1, but
+// leaves the copies less lead than the L2 prefetch of a single box's sweep.  Batches that
+// fit the ring only in part wait for room (copied in part: 1056 and 1726).
+static bool run_staged(bool single, int cls, uint32_t n_max) { return !single && (cls < 2 || n_max <= kRingMaxN); }
+
+static size_t run_smem(bool staged) { return kRunWarps * (sizeof(RunShared) + (staged ? sizeof(RunRing) : 0)); }
 
 using StepFnExt = void (*)(const StepArgs);
 // [sample][single box]; replays by single box
@@ -2666,16 +2759,16 @@ cudaError_t launch_step(const StepArgs& a, int algorithm, bool table, uint32_t p
         }
         for (int i = 0; i < nused; ++i) {
             const int cls = used[i];
-            const int single = a.nboxes == 1 ? 1 : 0;
-            const StepFnRun f = a.replay ? kRunReplayFns[single][cls] : a.tape_key ? kRunTapeFns[cls] : kRunFns[a.sample ? 1 : 0][single][cls];
+            const bool staged = run_staged(a.nboxes == 1, cls, a.boxes_n_max);
+            const StepFnRun f = run_fn(cls, staged, a.sample, a.nboxes == 1, a.replay, a.tape_key != nullptr);
             const uint32_t runs = a.run_class[cls + 1] - a.run_class[cls];
             const unsigned blocks = std::min((unsigned)grid, (runs + kRunWarps - 1) / (unsigned)kRunWarps);
             if (a.nboxes == 1 && !a.replay) {   // (an ensemble's classes fork and join)
-                e = launch_overlapped(f, blocks, kThreads, 0, st, a, a.run_class[cls], a.run_class[cls + 1], i == 0);
+                e = launch_overlapped(f, blocks, kThreads, run_smem(staged), st, a, a.run_class[cls], a.run_class[cls + 1], i == 0);
                 if (e != cudaSuccess) return e;
                 continue;
             }
-            f<<<blocks, kThreads, 0, fork && i > 0 ? branches->side[i - 1] : st>>>(a, a.run_class[cls],
+            f<<<blocks, kThreads, run_smem(staged), fork && i > 0 ? branches->side[i - 1] : st>>>(a, a.run_class[cls],
                                                                                     a.run_class[cls + 1], i == 0);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
@@ -2736,18 +2829,15 @@ cudaError_t configure_step(int algorithm, uint32_t pbuf, uint32_t cells, int* bl
     // load the kernels that step graphs capture before any capture begins
     cudaFuncAttributes attr;
     e = cudaFuncGetAttributes(&attr, (const void*)advance_kernel);
-    // the run kernel: about a quarter of the unified array as shared memory (4
-    // CTAs of 14 KB), the rest L1, which holds each batch's slots between its two passes
-    for (int i = 0; i < 2; ++i)
-        for (int j = 0; j < 2; ++j)
-            for (int k = 0; k < 3; ++k)
-                if (e == cudaSuccess)
-                    e = cudaFuncSetAttribute((const void*)kRunFns[i][j][k], cudaFuncAttributePreferredSharedMemoryCarveout,
-                                             27);
-    for (int k = 0; k < 3 && e == cudaSuccess; ++k) {
-        e = cudaFuncSetAttribute((const void*)kRunTapeFns[k], cudaFuncAttributePreferredSharedMemoryCarveout, 27);
-        for (int i = 0; i < 2 && e == cudaSuccess; ++i)
-            e = cudaFuncSetAttribute((const void*)kRunReplayFns[i][k], cudaFuncAttributePreferredSharedMemoryCarveout, 34);
+    // the run kernel: staged, nearly all of the unified array as shared memory (4 CTAs of
+    // 56 KB); unstaged about a quarter (14 KB), the rest L1, which then holds each
+    // batch's slots between its two passes
+    for (int v = 0; v < 64 && e == cudaSuccess; ++v) {
+        const int cls = v & 3;
+        const bool staged = cls < 3 && !(v & 8) && !((v & 32) && !(v & 16));   // (single boxes and their taped steps are not)
+        const void* f = (const void*)run_fn(std::min(cls, 2), staged, v & 4, v & 8, v & 16, v & 32);
+        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)run_smem(staged));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, staged ? 100 : 27);
     }
     // the extended run kernel: all of the unified array but a little as shared memory
     for (int k = 0; k < 6 && e == cudaSuccess; ++k) {
