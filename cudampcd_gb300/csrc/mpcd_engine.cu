@@ -1251,7 +1251,7 @@ private:
     // draws the ghosts), else none.
     void use_run_kernel_ghosts(StepArgs& a, bool table) const
     {
-        a.run_kernel = run_kernel_takes(a, params_.algorithm, table) ? (params_.algorithm ? kRunExtended : kRunSrd) : 0;
+        a.run_kernel = !tile_kernel_ && run_kernel_takes(a, params_.algorithm, table) ? (params_.algorithm ? kRunExtended : kRunSrd) : 0;
     }
 
     // One step: the overflow selection, then the step kernel (bracketed by the
@@ -1464,6 +1464,8 @@ private:
 
     StepGraph graph_[2];                    // [sampling]
     bool graphs_ = std::getenv("MPCD_GB_GRAPHS") == nullptr || std::getenv("MPCD_GB_GRAPHS")[0] != '0';
+    // test hook: every step on the tile kernel
+    bool tile_kernel_ = std::getenv("MPCD_GB_TILE_KERNEL") != nullptr && std::getenv("MPCD_GB_TILE_KERNEL")[0] == '1';
     unsigned long long graph_base_host_ = 0;
     mpcd_gb_params params_;                 // box 0 (algorithm and device of every box)
     std::vector<mpcd_gb_params> box_params_;

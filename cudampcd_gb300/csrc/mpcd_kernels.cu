@@ -1187,9 +1187,9 @@ __global__ void __launch_bounds__(kThreads, 4) step_kernel(const StepArgs a, uin
 
 // ------------------------------------------------------------------ SRD run kernel
 //
-// The production SRD step of one box or an ensemble (Philox draws; replays and the
-// pressure estimator take step_kernel; TAPE: a sampled single-box step that records
-// the adjoint tape, as step_kernel does): one warp per run of 32
+// The production SRD step of one box or an ensemble and its replays (Philox draws; with
+// the pressure estimator or, kTape, the adjoint tape of a sampled step for one box; the
+// tile kernel keeps injected draws and n > 64): one warp per run of up to 32
 // consecutive cells (storage order), lane l owning cell l of the run.  No
 // CTA-wide barrier and no staging: each warp works alone on its runs with 1.5
 // KB of shared memory of its own, and reads the particles straight from their
@@ -1262,7 +1262,35 @@ __device__ __forceinline__ uint2 run_entry(const StepArgs& a, uint32_t run)
     return make_uint2(a.box0.cell_base + c0, min(a.box0.run_cells, a.box0.C - c0));
 }
 
-enum RunMode : int { kPlain = 0, kTape = 1, kReplay = 2 };
+enum RunMode : int { kPlain = 0, kTape = 1, kReplay = 2, kPressure = 3 };
+
+// Pressure estimator: a thread's outward impulses on the bottom and top wall.  FP64: a
+// wall's impulse is a small difference of many.
+struct WallImpulse {
+    double bottom = 0.0, top = 0.0;
+    __device__ __forceinline__ void add(uint32_t side, double outward)   // side: 1 bottom, 2 top
+    {
+        if (side == 1u) bottom += outward;
+        if (side == 2u) top += outward;
+    }
+    // Bounce-back of a particle with z velocity v.
+    __device__ __forceinline__ void bounce(float v) { add(v > 0.0f ? 2u : 1u, 2.0 * fabs((double)v)); }
+    __device__ __forceinline__ void collect(DeviceState* state) const
+    {
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            double v = w ? top : bottom;
+            for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+            if ((threadIdx.x & 31u) == 0 && v != 0.0) atomicAdd(&state->wall_impulse[w], v);
+        }
+    }
+};
+
+// Wall layer of a cell for the estimator: 1 bottom, 2 top, 0 neither.
+__device__ __forceinline__ uint32_t wall_side(const BoxDesc& b, uint32_t z)
+{
+    return !b.wall_z ? 0u : z <= 1u ? 1u : z + 2u >= (uint32_t)b.L[2] ? 2u : 0u;
+}
 
 // A row of a dense (N, 3) array for every lane of the mask: through shared memory (96
 // floats), so that consecutive lanes write consecutive words of a row and a warp's store
@@ -1293,7 +1321,8 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
     __shared__ __align__(16) BoxDesc shared_box[SINGLE ? 1 : kRunWarps];   // ensembles: the box of the warp's run
     __shared__ float4 shared_shifts[SINGLE ? 1 : kRunWarps][2];              // and its grid shifts of steps k and k+1
     const uint32_t lane = threadIdx.x & 31u;
-    constexpr bool TAPE = MODE == kTape, REPLAY = MODE == kReplay;
+    constexpr bool TAPE = MODE == kTape, REPLAY = MODE == kReplay, PRESSURE = MODE == kPressure;
+    WallImpulse impulse;
     RunShared& sh = reinterpret_cast<RunShared*>(dyn)[threadIdx.x >> 5];
     RunRing& ring = reinterpret_cast<RunRing*>(dyn + kRunWarps * sizeof(RunShared))[STAGED ? threadIdx.x >> 5 : 0];
     __shared__ float shared_rows[REPLAY && !STAGED ? kRunWarps : 1][96];
@@ -1379,6 +1408,7 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
                 const float3 ax = srd_axis_philox(b, step, ref_index(b, cc));
                 axw = make_float4(ax.x, ax.y, ax.z, 0.0f);
             }
+            if (PRESSURE) axw.w = __uint_as_float(wall_side(b, cc.z));
             sh.axis[lane] = axw;
         }
         __syncwarp();
@@ -1565,6 +1595,16 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
                 const float4 nv = shared_shifts[SINGLE ? 0 : threadIdx.x >> 5][1];
                 xn = stream_shift_cell(b, x, vn, make_float3(nv.x, nv.y, nv.z), key);
                 key += b.cell_base;
+                if (PRESSURE) {
+                    const uint32_t side = active ? __float_as_uint(ax.w) : 0u;
+                    const bool hit = active && b.wall_z && vn.z != v.z;
+                    if (__any_sync(kFull, side != 0 || hit)) {   // (a branch: FP64 is slow even where no lane needs it)
+                        // collision in a wall layer: the ghosts took up minus the particle's change
+                        const double change = (double)v.z - (double)vp.z;
+                        impulse.add(side, side == 1u ? change : -change);
+                        if (hit) impulse.bounce(v.z);
+                    }
+                }
                 id = __float_as_uint(vp.w);
                 const uint32_t lab = SAMPLE || TAPE ? b.cell_base + storage_index(b, cell_of_wrapped(b, x)) : 0u;
                 if (SAMPLE) sample_add(a.samp, lab, v, active);
@@ -1583,13 +1623,14 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
                         min(raw_next, b.depth) * (uint32_t)sizeof(Slot));
         __syncwarp();   // the next run rewrites this warp's shared arrays
     }
+    if (PRESSURE) impulse.collect(a.state);
 }
 
 // ------------------------------------------------------------------ extended run kernel
 //
 // The production step of the extended collision and its replays (Philox draws, n <=
-// kExtMaxN; the tile kernel keeps injected draws, denser boxes and the pressure
-// estimator), one box or an ensemble: one warp per run of consecutive cells
+// kExtMaxN; the tile kernel keeps injected draws and denser boxes; one box with the
+// pressure estimator too), one box or an ensemble: one warp per run of consecutive cells
 // (storage order), alone with 9.2 KB of shared memory, no CTA-wide barrier.  A run
 // is as many cells as hold about 160 particles.  Per run, in parts when its entries
 // do not fit the buffer:
@@ -1629,7 +1670,7 @@ struct ExtShared {                   // one per warp
         float term[11][kTermRow];                // a colliding cell's terms, by sum and participant
     };
     float4 mean[kExtCells];          // mean velocity; w: entries of the collision
-    float4 com[kExtCells];           // centre of mass; w: 1 in a cell that collided
+    float4 com[kExtCells];           // centre of mass; w: 1 in a cell that collided | wall side << 1 (pressure)
     float4 omega[kExtCells];         // axis and gate, then the rotation; w: participants that move
     uint64_t bar;
     uint8_t cell[kExtBuf];           // of an entry, kExtGhost on ghosts
@@ -1647,12 +1688,14 @@ __device__ __forceinline__ uint32_t cell_of_entry(uint32_t t, uint32_t end)
     return i;
 }
 
-template <bool SAMPLE, bool SINGLE, bool REPLAY>
+template <bool SAMPLE, bool SINGLE, int MODE>
 __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const StepArgs a)
 {
     extern __shared__ __align__(128) unsigned char dyn[];
     __shared__ __align__(16) BoxDesc shared_box[SINGLE ? 1 : kExtWarps];
     const uint32_t lane = threadIdx.x & 31u;
+    constexpr bool REPLAY = MODE == kReplay, PRESSURE = MODE == kPressure;
+    WallImpulse impulse;
     ExtShared& sh = reinterpret_cast<ExtShared*>(dyn)[threadIdx.x >> 5];
     BoxDesc& sbox = shared_box[SINGLE ? 0 : threadIdx.x >> 5];
     wait_for_previous();   // the prologue, and with it the step before
@@ -1824,6 +1867,8 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                 const float3 centre = cell_centre(b, cc);
                 const float4 axg = sh.omega[in_part ? i : i0];
                 const float3 axis = make_float3(axg.x, axg.y, axg.z);
+                const uint32_t side = PRESSURE ? wall_side(b, cc.z) : 0u;
+                float real_vz = 0.0f;   // of the lane's real participants
                 float3 com = make_float3(0, 0, 0), mean = make_float3(0, 0, 0);
 #pragma unroll 1
                 for (uint32_t k = j; live && k < n; k += 4) {
@@ -1831,7 +1876,10 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                     const float4 xp = sh.buf[p].pos, vp = sh.buf[p].vel;
                     com.x += (xp.x - centre.x); com.y += (xp.y - centre.y); com.z += (xp.z - centre.z);
                     mean.x += vp.x; mean.y += vp.y; mean.z += vp.z;
+                    if (PRESSURE && k < m) real_vz += vp.z;
                 }
+                if (PRESSURE && __any_sync(kFull, side != 0))   // (a branch: FP64 is slow even where no lane needs it)
+                    impulse.add(side, side == 1u ? -(double)real_vz : (double)real_vz);   // before the collision
                 com = make_float3(group_sum(com.x, 4), group_sum(com.y, 4), group_sum(com.z, 4));
                 mean = make_float3(group_sum(mean.x, 4), group_sum(mean.y, 4), group_sum(mean.z, 4));
                 const float inv = live ? 1.0f / (float)n : 0.0f;
@@ -1858,7 +1906,7 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                 const bool collide = live && axg.w < prob;
                 if (in_part && j == 0) {
                     sh.mean[i] = make_float4(mean.x, mean.y, mean.z, __uint_as_float(n));
-                    sh.com[i] = make_float4(com.x, com.y, com.z, __uint_as_float(collide ? 1u : 0u));
+                    sh.com[i] = make_float4(com.x, com.y, com.z, __uint_as_float((collide ? 1u : 0u) | side << 1));
                     if (!collide) sh.omega[i] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(m));
                 }
                 __syncwarp();
@@ -1972,15 +2020,17 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                 const float4 xp = sh.buf[p].pos, vp = sh.buf[p].vel;
                 const float4 k0 = sh.mean[i], k1 = sh.com[i], k2 = sh.omega[i];
                 float3 x = make_float3(xp.x, xp.y, xp.z), v = make_float3(vp.x, vp.y, vp.z);
+                uint32_t side = 0;   // pressure: the wall of a particle that collided beside it
                 if (__float_as_uint(k0.w) > 1 && sh.rank[p] < __float_as_uint(k2.w)) {
                     const float3 xr = make_float3(x.x - k1.x, x.y - k1.y, x.z - k1.z);
-                    if (!__float_as_uint(k1.w)) { v.x -= k0.x; v.y -= k0.y; v.z -= k0.z; }
+                    if (!(__float_as_uint(k1.w) & 1u)) { v.x -= k0.x; v.y -= k0.y; v.z -= k0.z; }
                     v.x += k0.x; v.y += k0.y; v.z += k0.z;
                     v.x += b.drag_dt;
                     const float3 cr = cross3(xr, make_float3(k2.x, k2.y, k2.z));
                     v.x -= cr.x; v.y -= cr.y; v.z -= cr.z;
                     // com + xr rebuilds the wrapped staged position to within rounding
                     x = pbc_near(b, make_float3((k1.x + xr.x) - s.x, (k1.y + xr.y) - s.y, (k1.z + xr.z) - s.z));
+                    if (PRESSURE && active) side = __float_as_uint(k1.w) >> 1;
                 }
                 if (REPLAY) {   // staged in the terms' room
                     const unsigned rows = __ballot_sync(kFull, active);
@@ -1992,6 +2042,13 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                 uint32_t key;
                 const float3 xn = stream_shift_cell(b, x, vn, sn, key);
                 key = active ? b.cell_base + key : kNoKey;
+                if (PRESSURE) {
+                    const bool hit = active && b.wall_z && vn.z != v.z;
+                    if (__any_sync(kFull, side != 0 || hit)) {
+                        impulse.add(side, side == 1u ? (double)v.z : -(double)v.z);   // after the collision
+                        if (hit) impulse.bounce(v.z);
+                    }
+                }
                 if (SAMPLE) {
                     const uint32_t lab = b.cell_base + storage_index(b, cell_of_wrapped(b, x));
                     sample_add(a.samp, lab, v, active);
@@ -2012,6 +2069,7 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
             i0 = i1;
         }
     }
+    if (PRESSURE) impulse.collect(a.state);
 }
 
 // Before step k: every cell that received more particles than its bucket
@@ -2680,8 +2738,9 @@ static StepFnRun run_fn(int cls, bool staged)
 
 // The instance of a batch class: a replay, a step that records the adjoint tape (one
 // sampled box), or a plain step.
-static StepFnRun run_fn(int cls, bool staged, bool sample, bool single, bool replay, bool tape)
+static StepFnRun run_fn(int cls, bool staged, bool sample, bool single, bool replay, bool tape, bool pressure)
 {
+    if (pressure && !replay) return sample ? run_fn<true, true, kPressure>(cls, staged) : run_fn<false, true, kPressure>(cls, staged);
     if (replay) return single ? run_fn<false, true, kReplay>(cls, staged) : run_fn<false, false, kReplay>(cls, staged);
     if (tape) return run_fn<true, true, kTape>(cls, staged);
     if (sample) return single ? run_fn<true, true, kPlain>(cls, staged) : run_fn<true, false, kPlain>(cls, staged);
@@ -2700,9 +2759,10 @@ static size_t run_smem(bool staged) { return kRunWarps * (sizeof(RunShared) + (s
 
 using StepFnExt = void (*)(const StepArgs);
 // [sample][single box]; replays by single box
-static const StepFnExt kExtFns[2][2] = {{ext_run_kernel<false, false, false>, ext_run_kernel<false, true, false>},
-                                        {ext_run_kernel<true, false, false>, ext_run_kernel<true, true, false>}};
-static const StepFnExt kExtReplayFns[2] = {ext_run_kernel<false, false, true>, ext_run_kernel<false, true, true>};
+static const StepFnExt kExtFns[2][2] = {{ext_run_kernel<false, false, kPlain>, ext_run_kernel<false, true, kPlain>},
+                                        {ext_run_kernel<true, false, kPlain>, ext_run_kernel<true, true, kPlain>}};
+static const StepFnExt kExtReplayFns[2] = {ext_run_kernel<false, false, kReplay>, ext_run_kernel<false, true, kReplay>};
+static const StepFnExt kExtPressureFns[2] = {ext_run_kernel<false, true, kPressure>, ext_run_kernel<true, true, kPressure>};   // [sample]
 
 // Launch that may overlap the end of the kernel before it in the stream (a kernel that
 // calls wait_for_previous before it reads what that one wrote).
@@ -2725,9 +2785,10 @@ static cudaError_t launch_overlapped(void (*f)(P...), unsigned grid, unsigned th
 bool run_kernel_takes(const StepArgs& a, int algorithm, bool table)
 {
     if (algorithm == 1)
-        return !table && !a.pressure && (a.ghosts || !a.total_walls) && a.box_shifts && (a.nboxes == 1 || a.run_info) &&
+        return !table && (!a.pressure || a.nboxes == 1) && (a.ghosts || !a.total_walls) && a.box_shifts && (a.nboxes == 1 || a.run_info) &&
                a.boxes_n_max <= kExtMaxN;
-    return algorithm == 0 && !table && !a.replay && (!a.tape_key || (a.nboxes == 1 && a.sample)) && !a.pressure &&
+    return algorithm == 0 && !table && !a.replay && (!a.tape_key || (a.nboxes == 1 && a.sample)) &&
+           (!a.pressure || (a.nboxes == 1 && !a.tape_key)) &&
            (a.ghosts || !a.total_walls) && a.box_shifts && (a.nboxes == 1 || a.run_info) &&
            a.boxes_n_max <= kRunMaxN;
 }
@@ -2737,7 +2798,8 @@ cudaError_t launch_step(const StepArgs& a, int algorithm, bool table, uint32_t p
 {
     if (a.run_kernel == kRunExtended) {
         const unsigned blocks = std::min((unsigned)grid, (a.num_runs + kExtWarps - 1) / (unsigned)kExtWarps);
-        const StepFnExt f = a.replay ? kExtReplayFns[a.nboxes == 1 ? 1 : 0] : kExtFns[a.sample ? 1 : 0][a.nboxes == 1 ? 1 : 0];
+        const StepFnExt f = a.replay ? kExtReplayFns[a.nboxes == 1 ? 1 : 0]
+                            : a.pressure ? kExtPressureFns[a.sample ? 1 : 0] : kExtFns[a.sample ? 1 : 0][a.nboxes == 1 ? 1 : 0];
         if (a.nboxes == 1 && !a.replay) return launch_overlapped(f, blocks, kExtThreads, kExtWarps * sizeof(ExtShared), st, a);
         f<<<blocks, kExtThreads, kExtWarps * sizeof(ExtShared), st>>>(a);
         return cudaGetLastError();
@@ -2760,7 +2822,7 @@ cudaError_t launch_step(const StepArgs& a, int algorithm, bool table, uint32_t p
         for (int i = 0; i < nused; ++i) {
             const int cls = used[i];
             const bool staged = run_staged(a.nboxes == 1, cls, a.boxes_n_max);
-            const StepFnRun f = run_fn(cls, staged, a.sample, a.nboxes == 1, a.replay, a.tape_key != nullptr);
+            const StepFnRun f = run_fn(cls, staged, a.sample, a.nboxes == 1, a.replay, a.tape_key != nullptr, a.pressure);
             const uint32_t runs = a.run_class[cls + 1] - a.run_class[cls];
             const unsigned blocks = std::min((unsigned)grid, (runs + kRunWarps - 1) / (unsigned)kRunWarps);
             if (a.nboxes == 1 && !a.replay) {   // (an ensemble's classes fork and join)
@@ -2832,16 +2894,18 @@ cudaError_t configure_step(int algorithm, uint32_t pbuf, uint32_t cells, int* bl
     // the run kernel: staged, nearly all of the unified array as shared memory (4 CTAs of
     // 56 KB); unstaged about a quarter (14 KB), the rest L1, which then holds each
     // batch's slots between its two passes
-    for (int v = 0; v < 64 && e == cudaSuccess; ++v) {
+    for (int v = 0; v < 128 && e == cudaSuccess; ++v) {
         const int cls = v & 3;
-        const bool staged = cls < 3 && !(v & 8) && !((v & 32) && !(v & 16));   // (single boxes and their taped steps are not)
-        const void* f = (const void*)run_fn(std::min(cls, 2), staged, v & 4, v & 8, v & 16, v & 32);
+        const bool sample = v & 4, replay = v & 16, tape = v & 32, pressure = v & 64;
+        const bool single = (v & 8) || ((tape || pressure) && !replay);   // (taped and pressure steps are a single box's)
+        const bool staged = cls < 3 && !single;
+        const void* f = (const void*)run_fn(std::min(cls, 2), staged, sample, single, replay, tape, pressure);
         e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)run_smem(staged));
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, staged ? 100 : 27);
     }
     // the extended run kernel: all of the unified array but a little as shared memory
-    for (int k = 0; k < 6 && e == cudaSuccess; ++k) {
-        const void* f = (const void*)(k < 4 ? kExtFns[k >> 1][k & 1] : kExtReplayFns[k & 1]);
+    for (int k = 0; k < 8 && e == cudaSuccess; ++k) {
+        const void* f = (const void*)(k < 4 ? kExtFns[k >> 1][k & 1] : k < 6 ? kExtReplayFns[k & 1] : kExtPressureFns[k & 1]);
         e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kExtWarps * sizeof(ExtShared)));
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, f);

@@ -30,10 +30,10 @@ cudaError_t launch_step(const StepArgs& a, int algorithm, bool table, uint32_t p
 int run_blocks_per_sm(int algorithm);
 int run_warps_per_block(int algorithm);
 uint32_t run_cells_max(int algorithm, uint32_t n);
-// Whether srd_run_kernel can run this step (SRD, Philox draws, no replay or
-// pressure estimator, the adjoint tape only for one sampled box, n <= 64 in every
+// Whether srd_run_kernel can run this step (SRD, Philox draws, no replay, the adjoint
+// tape and the pressure estimator only for one box and not both, n <= 64 in every
 // box, a run table for ensembles and the wall-ghost array when boxes have walls);
-// or ext_run_kernel (extended, Philox draws, no pressure estimator, n <= kExtMaxN;
+// or ext_run_kernel (extended, Philox draws, n <= kExtMaxN;
 // also the replay of a step that it ran); the caller then sets a.run_kernel, which launch_step and the step's prologue follow.
 bool run_kernel_takes(const StepArgs& a, int algorithm, bool table);
 // state->step_base += steps (the last node of a replayed step graph).
