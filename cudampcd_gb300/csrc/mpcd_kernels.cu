@@ -1635,8 +1635,8 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
 // is as many cells as hold about 160 particles.  Per run, in parts when its entries
 // do not fit the buffer:
 //   lane = cell: count, source, wall ghosts (counted by the prologue), axis and gate;
-//   one bulk copy per cell brings its particles into shared memory; each particle
-//   counts its rank among the cell's ids, which gives the cell's id order;
+//   asynchronous copies bring the particles into shared memory; each counts its rank
+//   among its cell's ids, which gives the cell's id order;
 //   the ghosts, one lane each;
 //   4 lanes per cell: centre of mass, mean velocity, the projections on the axis and
 //   the gate, in the tile kernel's order (rank k adds to partial k mod 4, the four
@@ -1649,11 +1649,11 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
 // What bounds it is instruction issue and latency.  The tile kernel spends 33.6 warp
 // instructions a particle at n = 20: four lanes of each colliding cell draw and sum
 // while the warp's other cells wait, ranks are looked up in every pass, and five
-// CTA-wide barriers a tile stall its warps.  This kernel: 26 a particle before, 24.6 after the
-// streaming's fast wrap, 64 % issue.  256 x 256 x 66, n = 20 (8.2e7 particles), us a step:
-// tile kernel 3459, this one 2595; sampled 3677 and 2857.  Its code size matters: with
+// CTA-wide barriers a tile stall its warps.  This kernel's first version
+// took 26, at 64 % issue.  256 x 256 x 66, n = 20 (8.2e7 particles), us a step: tile kernel
+// 3459, this one 2508; sampled 3677 and 2763.  Its code size matters: with
 // the passes over a part unrolled it no longer fit the instruction cache and took
-// 10700 us; with the compiler's own unrolling of the inner loops 3280.
+// 10700 us; with the compiler's own unrolling of the inner loops 3280 (rolled 2773).
 
 constexpr uint32_t kExtBuf = 184;                  // entries (particles and ghosts) of a part
 constexpr uint32_t kExtCells = 24;                 // cells of a run at most
@@ -1671,13 +1671,12 @@ struct ExtShared {                   // one per warp
     };
     float4 mean[kExtCells];          // mean velocity; w: entries of the collision
     float4 com[kExtCells];           // centre of mass; w: 1 in a cell that collided | wall side << 1 (pressure)
-    float4 omega[kExtCells];         // axis and gate, then the rotation; w: participants that move
-    uint64_t bar;
-    uint8_t cell[kExtBuf];           // of an entry, kExtGhost on ghosts
-    uint8_t rank[kExtBuf];           // of a particle within its cell
+    float4 omega[kExtCells];         // axis and gate, then (in a cell that collided) the rotation
+    uint8_t cell[kExtBuf];           // of an entry, with kExtGhost or kExtIdle
     uint8_t order[kExtBuf];          // a cell's particles by rank
 };
-constexpr uint32_t kExtGhost = 0x80u;
+constexpr uint32_t kExtGhost = 0x80u;   // a ghost
+constexpr uint32_t kExtIdle = 0x40u;    // a particle past its cell's participants (4n, ghosts included)
 
 // The last lane-ordered cell whose range starts at or before t: end = inclusive ends by lane.
 __device__ __forceinline__ uint32_t cell_of_entry(uint32_t t, uint32_t end)
@@ -1712,9 +1711,6 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
     if (!REPLAY && blockIdx.x == 0 && threadIdx.x == 0)   // list of step k-1, refilled by step k+1
         a.state->ov[a.ov_zero_slot] = OverflowFill{0u, 0u};
     if (left) overflow_pass(a, step);
-    if (lane == 0) mbar_init(&sh.bar);
-    __syncwarp();
-    uint32_t phase = 0;
     int cur_box = -1;
     const uint32_t warps = gridDim.x * (uint32_t)kExtWarps;
     uint32_t run = blockIdx.x * (uint32_t)kExtWarps + (threadIdx.x >> 5);
@@ -1778,11 +1774,22 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
             const uint32_t first_e = end_e - (cnt + ng) - e0, first_i = end_i - padded - q0;
             const uint32_t range = (first_e & 0xFFu) | (first_i & 0x1FFu) << 8 | cnt << 17;
             const bool mine = lane >= i0 && lane < i1;
-            fence_proxy_async();   // the buffer's earlier reads and writes, before the copies
-            __syncwarp();
-            if (lane == 0 && real) mbar_arrive_expect_tx(&sh.bar, real * (uint32_t)sizeof(Slot));
-            __syncwarp();
-            if (mine && cnt) bulk_g2s(sh.buf + first_e, a.in_slots + src_slot, cnt * (uint32_t)sizeof(Slot), &sh.bar);
+            // the particles, 4 lanes per cell (one bulk copy per cell, which the lanes issue one
+            // after another, measured 2493 us plain and 2795 sampled at 256 x 256 x 66, n = 20
+            // and 180 at 100^3, n = 5, against 2508, 2763 and 176)
+#pragma unroll 1
+            for (uint32_t r = i0; r < i1; r += 8) {
+                const uint32_t i = r + (lane >> 2);
+                const uint32_t at = __shfl_sync(kFull, range, (int)(i & 31u));
+                const Slot* const from = a.in_slots + __shfl_sync(kFull, src_slot, (int)(i & 31u));
+                const uint32_t n = i < i1 ? at >> 17 : 0u;
+#pragma unroll 1
+                for (uint32_t k = lane & 3u; k < n; k += 4) {
+                    copy_async16(&sh.buf[(at & 0xFFu) + k].pos, &from[k].pos);
+                    copy_async16(&sh.buf[(at & 0xFFu) + k].vel, &from[k].vel);
+                }
+            }
+            copy_async_commit();
             if (mine) {
                 float gate = 1.0f;
                 const float3 ax = Draws<false>::ext_axis(a, b, step, ref, gate);
@@ -1811,14 +1818,8 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                     sh.buf[before + j].vel = make_float4(gv.x, gv.y, gv.z, 0.0f);
                 }
             }
-            if (real) {
-                if (!mbar_wait_bounded(&sh.bar, phase)) {
-                    if (lane == 0) atomicOr(&a.state->error_flags, kErrWaitTimeout);
-                    mbar_wait_bounded(&sh.bar, phase);   // let copies in flight land
-                    return;
-                }
-                phase ^= 1u;
-            }
+            copy_async_wait<0>();
+            __syncwarp();
             // the cell of every entry and the particles' ids side by side, 4 lanes per cell
 #pragma unroll 1
             for (uint32_t r = i0; r < i1; r += 8) {
@@ -1844,14 +1845,17 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
 #pragma unroll 1
                 for (uint32_t k = 0; 4 * k < n; ++k) {
                     const uint4 w = q[k];
-                    rank += (w.x < id) + (w.y < id) + (w.z < id) + (w.w < id);
+                    // (predicated adds: the compiler's own selects and sums cost 2 % of the step)
+                    asm("{.reg .pred a,b,c,d; setp.lt.u32 a,%1,%5; setp.lt.u32 b,%2,%5; setp.lt.u32 c,%3,%5; setp.lt.u32 d,%4,%5; @a add.u32 %0,%0,1; @b add.u32 %0,%0,1; @c add.u32 %0,%0,1; @d add.u32 %0,%0,1;}" : "+r"(rank) : "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w), "r"(id));
                 }
-                if (p0 + lane < total && !(info & kExtGhost)) {
-                    sh.rank[p] = (uint8_t)rank;
-                    sh.order[(at & 0xFFu) + rank] = (uint8_t)p;
-                }
+                if (p0 + lane < total && !(info & kExtGhost)) sh.order[(at & 0xFFu) + rank] = (uint8_t)p;
             }
             __syncwarp();
+            if (__any_sync(kFull, mine && cnt + ng > b.cap)) {   // more than 4n entries: the highest ids do not collide
+                if (mine && cnt + ng > b.cap)
+                    for (uint32_t k = b.cap - min(ng, b.cap); k < cnt; ++k) sh.cell[sh.order[first_e + k]] |= (uint8_t)kExtIdle;
+                __syncwarp();
+            }
 
             // collision quantities, 4 lanes per cell, 8 cells at a time
             for (uint32_t r = i0; r < i1; r += 8) {
@@ -1907,7 +1911,6 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                 if (in_part && j == 0) {
                     sh.mean[i] = make_float4(mean.x, mean.y, mean.z, __uint_as_float(n));
                     sh.com[i] = make_float4(com.x, com.y, com.z, __uint_as_float((collide ? 1u : 0u) | side << 1));
-                    if (!collide) sh.omega[i] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(m));
                 }
                 __syncwarp();
                 // the colliding cells, one at a time by the whole warp
@@ -1996,7 +1999,7 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                     if (lane == 0)
                         sh.omega[ci] = make_float4(Ii[0] * dL.x + Ii[3] * dL.y + Ii[4] * dL.z,
                                                    Ii[3] * dL.x + Ii[1] * dL.y + Ii[5] * dL.z,
-                                                   Ii[4] * dL.x + Ii[5] * dL.y + Ii[2] * dL.z, __uint_as_float(cm));
+                                                   Ii[4] * dL.x + Ii[5] * dL.y + Ii[2] * dL.z, 0.0f);
                 }
             }
             __syncwarp();
@@ -2018,16 +2021,20 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                 const uint32_t info = sh.cell[p], i = info & 31u;
                 const bool active = p0 + lane < total && !(info & kExtGhost);
                 const float4 xp = sh.buf[p].pos, vp = sh.buf[p].vel;
-                const float4 k0 = sh.mean[i], k1 = sh.com[i], k2 = sh.omega[i];
+                const float4 k0 = sh.mean[i], k1 = sh.com[i];
                 float3 x = make_float3(xp.x, xp.y, xp.z), v = make_float3(vp.x, vp.y, vp.z);
                 uint32_t side = 0;   // pressure: the wall of a particle that collided beside it
-                if (__float_as_uint(k0.w) > 1 && sh.rank[p] < __float_as_uint(k2.w)) {
+                if (__float_as_uint(k0.w) > 1 && !(info & kExtIdle)) {
                     const float3 xr = make_float3(x.x - k1.x, x.y - k1.y, x.z - k1.z);
-                    if (!(__float_as_uint(k1.w) & 1u)) { v.x -= k0.x; v.y -= k0.y; v.z -= k0.z; }
+                    const bool collided = __float_as_uint(k1.w) & 1u;   // (its velocities are comoving already)
+                    if (!collided) { v.x -= k0.x; v.y -= k0.y; v.z -= k0.z; }
                     v.x += k0.x; v.y += k0.y; v.z += k0.z;
                     v.x += b.drag_dt;
-                    const float3 cr = cross3(xr, make_float3(k2.x, k2.y, k2.z));
-                    v.x -= cr.x; v.y -= cr.y; v.z -= cr.z;
+                    if (collided) {
+                        const float4 k2 = sh.omega[i];
+                        const float3 cr = cross3(xr, make_float3(k2.x, k2.y, k2.z));
+                        v.x -= cr.x; v.y -= cr.y; v.z -= cr.z;
+                    }
                     // com + xr rebuilds the wrapped staged position to within rounding
                     x = pbc_near(b, make_float3((k1.x + xr.x) - s.x, (k1.y + xr.y) - s.y, (k1.z + xr.z) - s.z));
                     if (PRESSURE && active) side = __float_as_uint(k1.w) >> 1;
@@ -2859,6 +2866,41 @@ uint32_t run_cells_max(int algorithm, uint32_t n)
     return std::min(kExtCells, fit >= 8 ? fit & ~7u : fit);
 }
 
+// Attributes of the run kernels and of what else step graphs capture (a kernel is loaded
+// before any capture begins), once per process and device.
+static cudaError_t configure_run_kernels(int dev)
+{
+    static std::mutex mu;
+    static bool ready[64] = {};
+    std::lock_guard<std::mutex> lock(mu);
+    if (ready[dev & 63]) return cudaSuccess;
+    cudaFuncAttributes attr;
+    cudaError_t e = cudaFuncGetAttributes(&attr, (const void*)advance_kernel);
+    // the run kernel: staged, nearly all of the unified array as shared memory (4 CTAs of
+    // 56 KB); unstaged about a quarter (14 KB), the rest L1, which then holds each
+    // batch's slots between its two passes
+    for (int v = 0; v < 128 && e == cudaSuccess; ++v) {
+        const int cls = v & 3;
+        const bool sample = v & 4, replay = v & 16, tape = v & 32, pressure = v & 64;
+        const bool single = (v & 8) || ((tape || pressure) && !replay);   // (taped and pressure steps are a single box's)
+        const bool staged = cls < 3 && !single;
+        const void* f = (const void*)run_fn(std::min(cls, 2), staged, sample, single, replay, tape, pressure);
+        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)run_smem(staged));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, staged ? 100 : 27);
+    }
+    // the extended run kernel: all of the unified array but a little as shared memory
+    for (int k = 0; k < 8 && e == cudaSuccess; ++k) {
+        const void* f = (const void*)(k < 4 ? kExtFns[k >> 1][k & 1] : k < 6 ? kExtReplayFns[k & 1] : kExtPressureFns[k & 1]);
+        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kExtWarps * sizeof(ExtShared)));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, f);
+    }
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, (const void*)sample_finalize_kernel);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, (const void*)overflow_select_kernel);
+    ready[dev & 63] = e == cudaSuccess;
+    return e;
+}
+
 cudaError_t configure_step(int algorithm, uint32_t pbuf, uint32_t cells, int* blocks_per_sm)
 {
     // The shared-memory limit is an attribute of the kernel function, shared by
@@ -2888,31 +2930,7 @@ cudaError_t configure_step(int algorithm, uint32_t pbuf, uint32_t cells, int* bl
             granted[slot] = smem;
         }
     }
-    // load the kernels that step graphs capture before any capture begins
-    cudaFuncAttributes attr;
-    e = cudaFuncGetAttributes(&attr, (const void*)advance_kernel);
-    // the run kernel: staged, nearly all of the unified array as shared memory (4 CTAs of
-    // 56 KB); unstaged about a quarter (14 KB), the rest L1, which then holds each
-    // batch's slots between its two passes
-    for (int v = 0; v < 128 && e == cudaSuccess; ++v) {
-        const int cls = v & 3;
-        const bool sample = v & 4, replay = v & 16, tape = v & 32, pressure = v & 64;
-        const bool single = (v & 8) || ((tape || pressure) && !replay);   // (taped and pressure steps are a single box's)
-        const bool staged = cls < 3 && !single;
-        const void* f = (const void*)run_fn(std::min(cls, 2), staged, sample, single, replay, tape, pressure);
-        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)run_smem(staged));
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, staged ? 100 : 27);
-    }
-    // the extended run kernel: all of the unified array but a little as shared memory
-    for (int k = 0; k < 8 && e == cudaSuccess; ++k) {
-        const void* f = (const void*)(k < 4 ? kExtFns[k >> 1][k & 1] : k < 6 ? kExtReplayFns[k & 1] : kExtPressureFns[k & 1]);
-        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kExtWarps * sizeof(ExtShared)));
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, f);
-    }
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, (const void*)sample_finalize_kernel);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, (const void*)overflow_select_kernel);
-    if (e != cudaSuccess) return e;
+    if ((e = configure_run_kernels(dev)) != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         blocks_per_sm, (const void*)kStepFns[algorithm ? 1 : 0][0][1][0], kThreads, smem);
 }
