@@ -279,7 +279,7 @@ public:
         // the first read of a state replays the step straight into the caller's buffers;
         // later ones keep the state and copy it
         if (d_pos && d_vel && !dense_valid_ && !direct_read_ && step_ > 0) {
-            launch_replay(d_pos, d_vel);
+            launch_replay(d_pos, d_vel, gathers());
             check_device_errors();
             direct_read_ = true;
             return;
@@ -1279,15 +1279,32 @@ private:
     // Recompute the collision of the last step from its inputs into (N, 3) arrays by
     // particle id.  A run kernel replays its own steps, from the wall ghosts and grid
     // shifts that the step's prologue left.
-    void launch_replay(float* pos, float* vel)
+    // gather: in two passes, with the (then unused) dense arrays as scratch.
+    void launch_replay(float* pos, float* vel, bool gather = false)
     {
         StepArgs a = args(step_ - 1, true);
         a.dense_pos = pos;
         a.dense_vel = vel;
         a.run_kernel = last_step_run_;
+        if (gather) {
+            a.map = dense_pos_.as<uint32_t>();
+            a.map_cells = dense_vel_.as<AdjointCell>();
+        }
         check(launch_step(a, params_.algorithm, last_step_table_, pbuf_, a.run_kernel ? run_grid_ : grid_, stream_),
               "replay");
+        if (gather) check(launch_gather(a, N_, sms_, stream_), "replay");
     }
+
+    // Whether a replay into a caller's buffers gathers: an SRD box whose rows (24 bytes a
+    // particle) are more than 20 MB; the map (4 bytes a particle) and the cells (32 bytes)
+    // then fit the dense arrays.  One step with particles in and out, rows scattered in one
+    // pass and gathered in two: 0.6 M particles 110 and 116 us, 0.9 M 143 and 134, 2.2 M 233
+    // and 216, 5.2 M 589 and 536, 10.5 M 1189 and 1014, 40 M 5054 and 4934.
+    bool gathers() const
+    {
+        return boxes_.size() == 1 && last_step_run_ == kRunSrd && 24 * N_ > kGatherBytes && 12 * N_ >= sizeof(AdjointCell) * cells_;
+    }
+    static constexpr uint64_t kGatherBytes = 20u << 20;
 
     // The post-step state, by particle id, in dense_pos_ / dense_vel_: recompute
     // the collision of the last step from its inputs (same draws, same

@@ -567,6 +567,7 @@ __device__ void overflow_pass(const StepArgs& a, uint64_t step)
                 const uint64_t i3 = 3 * (uint64_t)id;
                 a.dense_pos[i3] = x.x; a.dense_pos[i3 + 1] = x.y; a.dense_pos[i3 + 2] = x.z;
                 a.dense_vel[i3] = v.x; a.dense_vel[i3 + 1] = v.y; a.dense_vel[i3 + 2] = v.z;
+                if (a.map) a.map[id] = kNoSlot;   // done: the gather passes it by
             } else {
                 vs = v;
                 xs = stream_shift(b, x, vs, grid_shift(b, bi, step + 1, a.state));
@@ -1262,7 +1263,7 @@ __device__ __forceinline__ uint2 run_entry(const StepArgs& a, uint32_t run)
     return make_uint2(a.box0.cell_base + c0, min(a.box0.run_cells, a.box0.C - c0));
 }
 
-enum RunMode : int { kPlain = 0, kTape = 1, kReplay = 2, kPressure = 3 };
+enum RunMode : int { kPlain = 0, kTape = 1, kReplay = 2, kPressure = 3, kMap = 4 };
 
 // Pressure estimator: a thread's outward impulses on the bottom and top wall.  FP64: a
 // wall's impulse is a small difference of many.
@@ -1321,7 +1322,7 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
     __shared__ __align__(16) BoxDesc shared_box[SINGLE ? 1 : kRunWarps];   // ensembles: the box of the warp's run
     __shared__ float4 shared_shifts[SINGLE ? 1 : kRunWarps][2];              // and its grid shifts of steps k and k+1
     const uint32_t lane = threadIdx.x & 31u;
-    constexpr bool TAPE = MODE == kTape, REPLAY = MODE == kReplay, PRESSURE = MODE == kPressure;
+    constexpr bool TAPE = MODE == kTape, MAP = MODE == kMap, REPLAY = MODE == kReplay || MAP, PRESSURE = MODE == kPressure;
     WallImpulse impulse;
     RunShared& sh = reinterpret_cast<RunShared*>(dyn)[threadIdx.x >> 5];
     RunRing& ring = reinterpret_cast<RunRing*>(dyn + kRunWarps * sizeof(RunShared))[STAGED ? threadIdx.x >> 5 : 0];
@@ -1410,6 +1411,7 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
             }
             if (PRESSURE) axw.w = __uint_as_float(wall_side(b, cc.z));
             sh.axis[lane] = axw;
+            if (MAP && valid) a.map_cells[cur.x + lane].axis = axw;
         }
         __syncwarp();
 
@@ -1539,6 +1541,7 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
                     sz += sh.gsum[L][2];
                     const float3 mean = mL > 1 ? srd_mean(sx, sy, sz, mL) : make_float3(0, 0, 0);
                     sh.cell[L] = make_float4(mean.x, mean.y, mean.z, __uint_as_float(mL));
+                    if (MAP && L < (cur.y & 63u)) a.map_cells[cur.x + L].sum = sh.cell[L];
                 }
             }
             __syncwarp();   // the means are written
@@ -1559,6 +1562,11 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
                     i += t >= __shfl_sync(kFull, incl, (int)(i + half - 1)) ? half : 0u;
             }
             const uint32_t slot = STAGED ? 0u : __shfl_sync(kFull, rel, (int)(i & 31u)) + t;
+            if (MAP) {   // where each particle lies, by id
+                const uint32_t pid = __float_as_uint(__ldg(&a.in_slots[slot].vel.w));
+                if (active) a.map[pid] = slot;
+                continue;
+            }
             uint32_t key = 0, id = 0;
             float3 xn = make_float3(0, 0, 0), vn = xn;
             {
@@ -2278,6 +2286,44 @@ __global__ void __launch_bounds__(kThreads) clear_counts_kernel(uint32_t* c0, ui
     }
 }
 
+// Second pass of a replay that gathers (one SRD box): the first, srd_run_kernel<kMap>,
+// left every particle's slot by id and every cell's mean velocity, entries and axis; here
+// a lane takes particle ids in order, finds its slot and, from the position in it, its
+// cell, and writes the post-collision rows one after another.
+// A replay that scatters its rows is bound by partial random writes once the dense arrays
+// outgrow L2 (1.25 sectors a row, two rows, at 40 G sectors/s); this one by one random
+// 32-byte read and one of a cell.  1.49e7 particles in random order: 1216 us in one pass,
+// 363 + 593 in two.
+__global__ void __launch_bounds__(kThreads, 4) gather_kernel(const StepArgs a, uint32_t n)
+{
+    constexpr int kEach = 4;
+    const BoxDesc& b = a.box0;
+    const float4 s4 = a.box_shifts[0];
+    const float3 s = make_float3(s4.x, s4.y, s4.z);
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t warp = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) >> 5, warps = (uint64_t)gridDim.x * (kThreads / 32);
+    for (uint64_t base = warp * 32 * kEach; base < n; base += warps * 32 * kEach) {
+        uint32_t slot[kEach];
+        float4 xp[kEach], vp[kEach];
+#pragma unroll
+        for (int u = 0; u < kEach; ++u) slot[u] = base + 32 * u + lane < n ? a.map[base + 32 * u + lane] : kNoSlot;
+#pragma unroll
+        for (int u = 0; u < kEach; ++u) load_slot(a.in_slots + (slot[u] == kNoSlot ? 0u : slot[u]), xp[u], vp[u]);
+#pragma unroll
+        for (int u = 0; u < kEach; ++u) {
+            float3 x = make_float3(xp[u].x, xp[u].y, xp[u].z), v = make_float3(vp[u].x, vp[u].y, vp[u].z);
+            if (slot[u] == kNoSlot) continue;
+            float4 mean, axis;
+            load_slot(reinterpret_cast<const Slot*>(a.map_cells + b.cell_base + storage_index(b, cell_of_wrapped(b, x))), mean, axis);
+            if (__float_as_uint(mean.w) > 1)
+                srd_collide(b, s, make_float3(mean.x, mean.y, mean.z), make_float3(axis.x, axis.y, axis.z), x, v);
+            const uint64_t i3 = 3 * (base + 32 * u + lane);
+            a.dense_pos[i3] = x.x; a.dense_pos[i3 + 1] = x.y; a.dense_pos[i3 + 2] = x.z;
+            a.dense_vel[i3] = v.x; a.dense_vel[i3 + 1] = v.y; a.dense_vel[i3 + 2] = v.z;
+        }
+    }
+}
+
 // Stream dense post-step particles for step k (a.step = k - 1: the launch plays
 // the epilogue of step k-1), key them by the cell they then occupy and scatter
 // them into the buckets of step k (a.out_*); particle id = dense index.  keep_pos,
@@ -2748,6 +2794,7 @@ static StepFnRun run_fn(int cls, bool staged)
 static StepFnRun run_fn(int cls, bool staged, bool sample, bool single, bool replay, bool tape, bool pressure)
 {
     if (pressure && !replay) return sample ? run_fn<true, true, kPressure>(cls, staged) : run_fn<false, true, kPressure>(cls, staged);
+    if (replay && tape) return run_fn<false, true, kMap>(cls, staged);   // a replay in two passes (gather_kernel)
     if (replay) return single ? run_fn<false, true, kReplay>(cls, staged) : run_fn<false, false, kReplay>(cls, staged);
     if (tape) return run_fn<true, true, kTape>(cls, staged);
     if (sample) return single ? run_fn<true, true, kPlain>(cls, staged) : run_fn<true, false, kPlain>(cls, staged);
@@ -2829,7 +2876,7 @@ cudaError_t launch_step(const StepArgs& a, int algorithm, bool table, uint32_t p
         for (int i = 0; i < nused; ++i) {
             const int cls = used[i];
             const bool staged = run_staged(a.nboxes == 1, cls, a.boxes_n_max);
-            const StepFnRun f = run_fn(cls, staged, a.sample, a.nboxes == 1, a.replay, a.tape_key != nullptr, a.pressure);
+            const StepFnRun f = run_fn(cls, staged, a.sample, a.nboxes == 1, a.replay, a.replay ? a.map != nullptr : a.tape_key != nullptr, a.pressure);
             const uint32_t runs = a.run_class[cls + 1] - a.run_class[cls];
             const unsigned blocks = std::min((unsigned)grid, (runs + kRunWarps - 1) / (unsigned)kRunWarps);
             if (a.nboxes == 1 && !a.replay) {   // (an ensemble's classes fork and join)
@@ -2882,7 +2929,7 @@ static cudaError_t configure_run_kernels(int dev)
     for (int v = 0; v < 128 && e == cudaSuccess; ++v) {
         const int cls = v & 3;
         const bool sample = v & 4, replay = v & 16, tape = v & 32, pressure = v & 64;
-        const bool single = (v & 8) || ((tape || pressure) && !replay);   // (taped and pressure steps are a single box's)
+        const bool single = (v & 8) || tape || (pressure && !replay);   // (taped, mapped and pressure steps are a single box's)
         const bool staged = cls < 3 && !single;
         const void* f = (const void*)run_fn(std::min(cls, 2), staged, sample, single, replay, tape, pressure);
         e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)run_smem(staged));
@@ -3031,6 +3078,12 @@ cudaError_t launch_init(const BoxDesc* boxes, int nboxes, float* pos, float* vel
                         cudaStream_t st)
 {
     init_kernel<<<grid, kThreads, 0, st>>>(boxes, nboxes, pos, vel, n_total);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_gather(const StepArgs& a, uint64_t n, int sms, cudaStream_t st)
+{
+    gather_kernel<<<sms * 4, kThreads, 0, st>>>(a, (uint32_t)n);
     return cudaGetLastError();
 }
 

@@ -83,6 +83,8 @@ cudaError_t launch_cell_offsets_static(const StepArgs& a, const uint32_t* count,
 // Initial particles (uniform positions, Maxwell-Boltzmann velocities).
 cudaError_t launch_init(const BoxDesc* boxes, int nboxes, float* pos, float* vel, uint64_t n_total, int grid,
                         cudaStream_t st);
+// Second pass of a replay with a.map and a.map_cells: rows of particles 0 .. n - 1.
+cudaError_t launch_gather(const StepArgs& a, uint64_t n, int sms, cudaStream_t st);
 cudaError_t launch_momentum_partial(const float* vel, uint64_t begin, uint64_t end, double* partial, int grid,
                                     cudaStream_t st);
 cudaError_t launch_subtract(float* vel, uint64_t begin, uint64_t end, float mx, float my, float mz, int grid,

@@ -134,6 +134,15 @@ struct DrawTables {
     uint32_t gmax, pmax;
 };
 
+// What a pass over particles needs of a cell, one sector.  Replays that gather: the mean
+// velocity and, as bits, the entries in sum, the rotation axis in axis.
+// Adjoint sweep, a cell at one step: the sums of mu over its collided particles and
+// 1 / N_c in sum.w; the rotation axis (as a collision cell), and in axis.w its sampling
+// term dU(z) / (samples Lx Ly count) (as a lab cell).
+struct alignas(32) AdjointCell {
+    float4 sum, axis;
+};
+
 struct StepArgs {
     BoxDesc box0;                 // the only box of a single-box launch (kernel-parameter space)
     const BoxDesc* boxes;
@@ -175,6 +184,9 @@ struct StepArgs {
     int32_t replay;
     float* dense_pos;
     float* dense_vel;
+    // a replay that gathers (one SRD box): the slot of every particle by id, and the cells
+    uint32_t* map;
+    AdjointCell* map_cells;
     DeviceState* state;
     int32_t sample;               // accumulate the lab-grid sample of clean(k+1)
     float4* samp;                 // [global lab cells, storage order] (sum vx, vy, vz, count)
@@ -216,15 +228,9 @@ struct StepArgs {
 
 constexpr int32_t kRunSrd = 1, kRunExtended = 2;   // StepArgs::run_kernel
 constexpr uint32_t kExtMaxN = 36;                  // densities that ext_run_kernel takes
+constexpr uint32_t kNoSlot = 0xFFFFFFFFu;          // StepArgs::map of a particle that is in no slot
 constexpr uint32_t kTapeNone = 0xFFFFFFFFu;
 constexpr uint32_t kTapeBounce = 0x80000000u;
-
-// Adjoint sweep, a cell at one step: the sums of mu over its collided particles and
-// 1 / N_c in sum.w; the rotation axis (as a collision cell), and in axis.w its sampling
-// term dU(z) / (samples Lx Ly count) (as a lab cell).
-struct alignas(32) AdjointCell {
-    float4 sum, axis;
-};
 
 // One step of the adjoint tape (by particle id / storage cell) and its cells.
 struct AdjointStep {
