@@ -8,6 +8,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 import re
+import sys
 
 import numpy as np
 
@@ -127,6 +128,7 @@ class Handle:
         arr = (Params * max(1, len(plist)))(*plist)
         self.params = plist[0] if plist else None
         self.h = C.c_void_p()
+        self._results = []
         rc = self._lib.mpcd_gb_ensemble_create(C.cast(arr, C.c_void_p), len(plist), C.byref(self.h))
         if rc != 0:
             raise GbError(f"mpcd_gb_create failed ({rc}): {self._lib.mpcd_gb_last_error(None).decode()}")
@@ -169,9 +171,24 @@ class Handle:
     def step_and_sample(self, n=1):
         self._check(self._lib.mpcd_gb_step_and_sample(self.h, n))
 
+    def _result(self, n):
+        """A float32 array of n entries for a result, in memory of an earlier one that nothing
+        refers to any more where there is such (mapped already: fresh memory costs page faults).
+        The handle keeps at most four, of up to 80 MiB each and
+        128 MiB in all."""
+        for buf in self._results:
+            if buf.size == n and sys.getrefcount(buf) == 3:   # the list's, the loop's and the call's
+                return buf[:]
+        self._results = [b for b in self._results if sys.getrefcount(b) > 3 or b.size == n]
+        buf = np.empty(n, np.float32)
+        if len(self._results) < 4 and buf.nbytes <= 80 << 20 and buf.nbytes + sum(b.nbytes for b in self._results) <= 1 << 27:
+            self._results.append(buf)
+            return buf[:]
+        return buf
+
     def sample_mean(self):
-        d = np.zeros(self.C, np.float32)
-        v = np.zeros(3 * self.C, np.float32)
+        d = self._result(self.C)
+        v = self._result(3 * self.C)
         self._check(self._lib.mpcd_gb_get_sample_mean(self.h, d, v))
         return d, v.reshape(-1, 3)
 

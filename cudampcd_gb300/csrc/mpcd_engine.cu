@@ -198,8 +198,10 @@ public:
         float* d_velocity = d_density + cells_;
         // cpu_backend.cpp:218 / cuda_backend_impl.cu:210: divide by the counter, S-1 for S samples
         const double inverse = 1.0 / (double)sample_counter_;
-        for (const BoxDesc& b : boxes_)   // lab cells of every box, each in reference order
-            check(launch_mean_fields(acc_.as<SampleAcc>(), b, inverse, d_density, d_velocity, stream_), "mean fields");
+        // lab cells of every box, each in reference order
+        check(launch_mean_fields(acc_.as<SampleAcc>(), boxes_d_.as<BoxDesc>(), (int)boxes_.size(), cells_, inverse, d_density,
+                                 d_velocity, stream_),
+              "mean fields");
         check(cudaMemcpyAsync(density, d_density, sizeof(float) * cells_, cudaMemcpyDeviceToHost, stream_),
               "sample read");
         check(cudaMemcpyAsync(velocity, d_velocity, sizeof(float) * 3 * cells_, cudaMemcpyDeviceToHost, stream_),

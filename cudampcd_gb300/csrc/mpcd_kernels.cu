@@ -2396,16 +2396,22 @@ __global__ void sample_finalize_kernel(float4* samp, SampleAcc* acc, uint64_t ce
         fold_sample(samp, acc, c, snapshot, lab_count);
 }
 
-// Mean fields of one box in reference order (x fastest) from the FP64 sums, which
+// Mean fields of every box in reference order (x fastest) from the FP64 sums, which
 // are kept in storage order: density n / S and velocity v / S per lab cell
 // (cpu_backend.cpp:218, `inverse` = 1 / S).
-__global__ void mean_fields_kernel(const SampleAcc* acc, BoxDesc b, double inverse, float* density, float* velocity)
+__global__ void mean_fields_kernel(const SampleAcc* acc, const BoxDesc* boxes, int nboxes, uint64_t cells, double inverse,
+                                   float* density, float* velocity)
 {
-    const uint32_t Lx = (uint32_t)b.L[0], Ly = (uint32_t)b.L[1], Lz = (uint32_t)b.L[2];
-    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < b.C; r += gridDim.x * blockDim.x) {
-        const uint32_t x = r % Lx, yz = r / Lx, y = yz % Ly, z = yz / Ly;
+    for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < cells; g += (uint64_t)gridDim.x * blockDim.x) {
+        int lo = 0, hi = nboxes - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (boxes[mid].cell_base <= g) lo = mid; else hi = mid - 1;
+        }
+        const BoxDesc& b = boxes[lo];
+        const uint32_t Lx = (uint32_t)b.L[0], Ly = (uint32_t)b.L[1], Lz = (uint32_t)b.L[2];
+        const uint32_t r = (uint32_t)(g - b.cell_base), x = r % Lx, yz = r / Lx, y = yz % Ly, z = yz / Ly;
         const SampleAcc q = acc[b.cell_base + z + Lz * (x + Lx * y)];
-        const uint64_t g = b.cell_base + (uint64_t)r;
         density[g] = (float)(q.n * inverse);
         velocity[3 * g + 0] = (float)(q.vx * inverse);
         velocity[3 * g + 1] = (float)(q.vy * inverse);
@@ -3043,11 +3049,11 @@ cudaError_t launch_sample_finalize(float4* samp, SampleAcc* acc, uint64_t cells,
     return cudaGetLastError();
 }
 
-cudaError_t launch_mean_fields(const SampleAcc* acc, const BoxDesc& b, double inverse, float* density, float* velocity,
-                               cudaStream_t st)
+cudaError_t launch_mean_fields(const SampleAcc* acc, const BoxDesc* boxes, int nboxes, uint64_t cells, double inverse,
+                               float* density, float* velocity, cudaStream_t st)
 {
-    const unsigned grid = (unsigned)std::min<uint64_t>((b.C + kThreads - 1) / kThreads, 4096);
-    mean_fields_kernel<<<grid, kThreads, 0, st>>>(acc, b, inverse, density, velocity);
+    const unsigned grid = (unsigned)std::min<uint64_t>((cells + kThreads - 1) / kThreads, 4096);
+    mean_fields_kernel<<<grid, kThreads, 0, st>>>(acc, boxes, nboxes, cells, inverse, density, velocity);
     return cudaGetLastError();
 }
 

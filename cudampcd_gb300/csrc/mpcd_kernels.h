@@ -52,10 +52,10 @@ cudaError_t launch_overflow_select(const StepArgs& a, Slot* in_slots, float4* ov
 // Lab-grid sample of one step into the FP64 running sums (and clear the step sums).
 cudaError_t launch_sample_finalize(float4* samp, SampleAcc* acc, uint64_t cells, int snapshot, int grid,
                                    cudaStream_t st, uint32_t* lab_count = nullptr);
-// Density and velocity means of one box in reference order (x fastest) from the
+// Density and velocity means of every box in reference order (x fastest) from the
 // FP64 sums (storage order), divided by the sample count: inverse = 1 / samples.
-cudaError_t launch_mean_fields(const SampleAcc* acc, const BoxDesc& b, double inverse, float* density, float* velocity,
-                               cudaStream_t st);
+cudaError_t launch_mean_fields(const SampleAcc* acc, const BoxDesc* boxes, int nboxes, uint64_t cells, double inverse,
+                               float* density, float* velocity, cudaStream_t st);
 // Adjoint of the sampled x-velocity profile (single box, SRD): U(z) from the sample
 // sums of `samples` steps; the cells of a step before its sweep; one launch of the
 // reverse sweep: the end of step hi (or null) and the start of step lo (or null), the

@@ -19,22 +19,34 @@ using mpcd::CollisionKernel;
 using mpcd::ExperimentType;
 using mpcd::MPCDAlgorithm;
 using mpcd::SimulationParameters;
+using mpcd::api::ResultPool;
 using mpcd::api::SimulationHandle;
 
 namespace {
 
+// A vector lent to numpy; its memory goes back to the pool with the array.
+struct Lent {
+    std::vector<float> data;
+    std::shared_ptr<ResultPool> pool;
+};
+
 // Hand a vector to numpy without a copy; the capsule owns it.
-py::array_t<float> to_numpy(std::vector<float>&& v, std::vector<py::ssize_t> shape, std::vector<py::ssize_t> strides)
+py::array_t<float> to_numpy(std::vector<float>&& v, std::shared_ptr<ResultPool> pool, std::vector<py::ssize_t> shape,
+                            std::vector<py::ssize_t> strides)
 {
-    auto* owned = new std::vector<float>(std::move(v));
-    py::capsule owner(owned, [](void* p) { delete static_cast<std::vector<float>*>(p); });
-    return py::array_t<float>(shape, strides, owned->data(), owner);
+    auto* lent = new Lent{std::move(v), std::move(pool)};
+    py::capsule owner(lent, [](void* p) {
+        auto* l = static_cast<Lent*>(p);
+        l->pool->give(std::move(l->data));
+        delete l;
+    });
+    return py::array_t<float>(shape, strides, lent->data.data(), owner);
 }
 
-py::array_t<float> vectors_to_numpy(std::vector<float>&& v)
+py::array_t<float> vectors_to_numpy(std::vector<float>&& v, std::shared_ptr<ResultPool> pool)
 {
     const py::ssize_t n = static_cast<py::ssize_t>(v.size() / 3);
-    return to_numpy(std::move(v), {n, 3}, {3 * (py::ssize_t)sizeof(float), (py::ssize_t)sizeof(float)});
+    return to_numpy(std::move(v), std::move(pool), {n, 3}, {3 * (py::ssize_t)sizeof(float), (py::ssize_t)sizeof(float)});
 }
 
 std::vector<float> from_numpy(py::array_t<float, py::array::c_style | py::array::forcecast> a)
@@ -64,45 +76,46 @@ PYBIND11_MODULE(_pympcd, m)
         .def(
             "get_mean_fields",
             [](SimulationHandle& self) {
-                std::vector<float> density, velocity;
+                auto const& p = self.getParameters();
+                const size_t cells = (size_t)p.volume_size[0] * (size_t)p.volume_size[1] * (size_t)p.volume_size[2];
+                std::vector<float> density = self.results()->take(cells), velocity = self.results()->take(3 * cells);
                 {
                     py::gil_scoped_release release;
                     self.getSampleMean(density, velocity);
                 }
-                auto const& p = self.getParameters();
                 const py::ssize_t x = (py::ssize_t)p.volume_size[0], y = (py::ssize_t)p.volume_size[1],
                                   z = (py::ssize_t)p.volume_size[2], sf = (py::ssize_t)sizeof(float);
                 // Same shape and strides as the reference binding (bindings.cpp:62-72),
                 // including its y stride of Ly (exact for Lx == Ly).
                 std::vector<py::ssize_t> shape = {x, y, z}, strides = {sf, y * sf, x * y * sf};
-                auto d = to_numpy(std::move(density), shape, strides);
+                auto d = to_numpy(std::move(density), self.results(), shape, strides);
                 for (auto& s : strides) s *= 3;
                 strides.push_back(sf);
                 shape.push_back(3);
-                auto v = to_numpy(std::move(velocity), shape, strides);
+                auto v = to_numpy(std::move(velocity), self.results(), shape, strides);
                 return py::make_tuple(d, v);
             },
             "Mean density and velocity fields (voxel arrays) of the accumulated sample.")
         .def(
             "get_particle_positions",
             [](SimulationHandle const& self) {
-                std::vector<float> out;
+                std::vector<float> out = self.results()->take(3 * self.getNParticles());
                 {
                     py::gil_scoped_release release;
                     self.getParticlePositions(out);
                 }
-                return vectors_to_numpy(std::move(out));
+                return vectors_to_numpy(std::move(out), self.results());
             },
             "Particle positions, (N, 3) float32, by particle id (a fixed order).")
         .def(
             "get_particle_velocities",
             [](SimulationHandle const& self) {
-                std::vector<float> out;
+                std::vector<float> out = self.results()->take(3 * self.getNParticles());
                 {
                     py::gil_scoped_release release;
                     self.getParticleVelocities(out);
                 }
-                return vectors_to_numpy(std::move(out));
+                return vectors_to_numpy(std::move(out), self.results());
             },
             "Particle velocities, (N, 3) float32, by particle id.")
         .def(

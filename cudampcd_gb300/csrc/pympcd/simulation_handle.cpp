@@ -19,7 +19,10 @@ SimulationHandle::SimulationHandle(SimulationParameters const& params, std::stri
 {
 }
 
-SimulationHandle::~SimulationHandle() = default;
+SimulationHandle::~SimulationHandle()
+{
+    if (results_) results_->close();
+}
 SimulationHandle::SimulationHandle(SimulationHandle&&) noexcept = default;
 SimulationHandle& SimulationHandle::operator=(SimulationHandle&&) noexcept = default;
 
