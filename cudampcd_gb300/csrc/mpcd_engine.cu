@@ -813,7 +813,24 @@ private:
         if (!std::isfinite(p.drag)) throw Error(MPCD_GB_EINVAL, "drag must be finite");
     }
 
-    static BoxDesc make_box(const mpcd_gb_params& p)
+    // Bucket depth: n + 4 sqrt(n) + 2 (a Poisson(n) cell exceeds it in about 1 of
+    // 10^4..10^5 cells), at most the reference's 4n.  deep, where there is room: a whole number
+    // of 128-byte lines, and up to n = 12 n + 6 sqrt(n) + 2, which leaves the step's prologue
+    // without a selection: dilute fluids cluster (a lone particle keeps its shift), and at n
+    // <= 7 thousands of cells a step pass the shallow depth.  Step us at 100 x 100 x 60 after
+    // 3000 steps, shallow and deep: n = 4 152 and 108, n = 5 141 and 88, n = 6 126 and 89, n =
+    // 8 97 and 92, n = 10 113 and 106; 61 x 61 x 85, n = 7 64 and 57.
+    static uint32_t bucket_depth(uint32_t n, bool deep)
+    {
+        const double root = std::sqrt((double)n);
+        const uint32_t shallow = std::min(4 * n, n + (uint32_t)std::ceil(4.0 * root) + 2u);
+        if (!deep) return shallow;
+        const uint32_t want = n <= 12 ? n + (uint32_t)std::ceil(6.0 * root) + 2u : shallow;
+        return std::min(4 * n, (want + 3u) & ~3u);
+    }
+    static constexpr uint64_t kDeepBytes = 32ull << 30;   // both bucket sets, up to which they are deep
+
+    static BoxDesc make_box(const mpcd_gb_params& p, bool deep)
     {
         BoxDesc b{};
         uint64_t Nf = p.n;
@@ -839,9 +856,7 @@ private:
         b.cos_a = cosf((float)((M_PI * 120) / 180));
         b.n = p.n;
         b.cap = 4 * p.n;
-        // bucket depth: n + 4 sqrt(n) + 2 (a Poisson(n) cell exceeds it in about 1 of
-        // 10^4..10^5 cells), at most the reference's 4n
-        b.depth = std::min(b.cap, p.n + (uint32_t)std::ceil(4.0 * std::sqrt((double)p.n)) + 2u);
+        b.depth = bucket_depth(p.n, deep);
         if (const char* e = std::getenv("MPCD_GB_BUCKET_DEPTH")) {   // test hook: force spills
             const uint32_t v = (uint32_t)std::strtoul(e, nullptr, 10);
             if (v >= 1) b.depth = std::min(b.cap, v);
@@ -863,8 +878,11 @@ private:
         boxes_.clear();
         uint64_t cells = 0, slots = 0, particles = 0, walls = 0;
         uint32_t n_max = 0;
+        double deep_bytes = 0.0;
+        for (const mpcd_gb_params& p : box_params_)
+            deep_bytes += 2.0 * sizeof(Slot) * bucket_depth(p.n, true) * p.volume_size[0] * p.volume_size[1] * p.volume_size[2];
         for (const mpcd_gb_params& p : box_params_) {
-            BoxDesc b = make_box(p);
+            BoxDesc b = make_box(p, deep_bytes <= (double)kDeepBytes);
             if (cells + b.C >= (1ull << 31)) throw Error(MPCD_GB_EINVAL, "too many cells in the ensemble");
             b.cell_base = (uint32_t)cells;
             b.slot_base = slots;

@@ -3,8 +3,9 @@
 // Particles live in per-cell buckets: cell c of a box owns `depth` slots of 32
 // bytes each, one DRAM sector: pos = (x, y, z, 0), vel = (vx, vy, vz, id).  The
 // reference's cell table is 4n deep (cap, backend_context.cu:24): up to cap
-// particles of a cell collide.  depth = min(cap, n + ceil(4 sqrt(n)) + 2) holds
-// all but about one cell in 10^4..10^5 at equilibrium; the particles of a cell
+// particles of a cell collide.  depth = min(cap, n + ceil(4 sqrt(n)) + 2), or somewhat
+// deeper where there is room (Engine::bucket_depth), holds all but about one cell in
+// 10^4..10^5 at equilibrium; the particles of a cell
 // past its depth go to the overflow list, and the step's prologue
 // (overflow_select_kernel) copies such a cell's colliding set -- its cap lowest
 // ids -- into a contiguous extension area after the buckets, records the
