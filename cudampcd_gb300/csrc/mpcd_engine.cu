@@ -815,17 +815,18 @@ private:
 
     // Bucket depth: n + 4 sqrt(n) + 2 (a Poisson(n) cell exceeds it in about 1 of
     // 10^4..10^5 cells), at most the reference's 4n.  deep, where there is room: a whole number
-    // of 128-byte lines, and up to n = 12 n + 6 sqrt(n) + 2, which leaves the step's prologue
-    // without a selection: dilute fluids cluster (a lone particle keeps its shift), and at n
+    // of 128-byte lines, and n + 6 sqrt(n) + 2 (5 sqrt(n) past n = 12), which leaves the
+    // step's prologue without a selection: dilute fluids cluster (a lone particle keeps its shift), and at n
     // <= 7 thousands of cells a step pass the shallow depth.  Step us at 100 x 100 x 60 after
     // 3000 steps, shallow and deep: n = 4 152 and 108, n = 5 141 and 88, n = 6 126 and 89, n =
-    // 8 97 and 92, n = 10 113 and 106; 61 x 61 x 85, n = 7 64 and 57.
+    // 8 97 and 92, n = 10 113 and 106; 61 x 61 x 85, n = 7 64 and 57; 100 x 100 x 42, n = 20 131
+    // and 127.
     static uint32_t bucket_depth(uint32_t n, bool deep)
     {
         const double root = std::sqrt((double)n);
         const uint32_t shallow = std::min(4 * n, n + (uint32_t)std::ceil(4.0 * root) + 2u);
         if (!deep) return shallow;
-        const uint32_t want = n <= 12 ? n + (uint32_t)std::ceil(6.0 * root) + 2u : shallow;
+        const uint32_t want = n + (uint32_t)std::ceil((n <= 12 ? 6.0 : 5.0) * root) + 2u;
         return std::min(4 * n, (want + 3u) & ~3u);
     }
     static constexpr uint64_t kDeepBytes = 32ull << 30;   // both bucket sets, up to which they are deep

@@ -163,18 +163,28 @@ __device__ __forceinline__ int box_of_particle(const BoxDesc* boxes, int nboxes,
     return lo;
 }
 
-// Claim a slot in `count[key]` for every active lane; lanes that share a key
-// are served by one atomic (warp-aggregated).  Returns the slot.
-__device__ __forceinline__ uint32_t claim_slot(uint32_t* count, uint32_t key, bool active)
-{
-    // idle lanes share a key no cell has, so that the whole warp takes one path
-    const unsigned peers = __match_any_sync(kFull, active ? key : 0xFFFFFFFFu);
-    const int leader = __ffs(peers) - 1;
-    uint32_t base = 0;
-    if (active && (int)(threadIdx.x & 31) == leader) base = atomicAdd(count + key, (uint32_t)__popc(peers));
-    base = __shfl_sync(kFull, base, leader);
-    return base + (uint32_t)__popc(peers & lanemask_lt());
-}
+// Claims of slots in `count[key]` for every active lane; lanes that share a key are
+// served by one atomic (warp-aggregated).  The claim is issued first, so that work may
+// follow while the atomic is under way, and slot() then gives the lane's slot.
+struct SlotClaim {
+    unsigned peers;
+    int leader;
+    uint32_t base;
+
+    __device__ __forceinline__ SlotClaim(uint32_t* count, uint32_t key, bool active)
+    {
+        // idle lanes share a key no cell has, so that the whole warp takes one path
+        peers = __match_any_sync(kFull, active ? key : 0xFFFFFFFFu);
+        leader = __ffs(peers) - 1;
+        base = 0;
+        if (active && (int)(threadIdx.x & 31u) == leader) base = atomicAdd(count + key, (uint32_t)__popc(peers));
+    }
+
+    __device__ __forceinline__ uint32_t slot() const
+    {
+        return __shfl_sync(kFull, base, leader) + (uint32_t)__popc(peers & lanemask_lt());
+    }
+};
 
 // Fold one step's sample of lab cell c into the FP64 running sums: the cell's mean
 // velocity (0 for an empty cell, as averageReduceOnly) and its count, snapshot or
@@ -223,16 +233,22 @@ __device__ __forceinline__ void push_overflow(const StepArgs& a, uint32_t key, f
 // Put one particle (already streamed and shifted for the next collision, in
 // cell `key`) into its bucket, or into the overflow list when the bucket is full.
 // pos.w = kNoExt: a cell the selection does not reach keeps reading its bucket.
-__device__ __forceinline__ void store_particle(const StepArgs& a, const BoxDesc& b, float3 xs, float3 vs, uint32_t id,
-                                               uint32_t key, bool active)
+__device__ __forceinline__ void place_particle(const StepArgs& a, const BoxDesc& b, float3 xs, float3 vs, uint32_t id,
+                                               uint32_t key, uint32_t slot, bool active)
 {
-    const uint32_t slot = claim_slot(a.out_count, key, active);
     const float4 xp = make_float4(xs.x, xs.y, xs.z, __uint_as_float(kNoExt));
     const float4 vp = make_float4(vs.x, vs.y, vs.z, __uint_as_float(id));
     // the slot's index in 32 bits: every bucket slot index is below 2^32 (the engine checks)
     const uint32_t index = (uint32_t)b.slot_base + (key - b.cell_base) * b.depth + slot;
     if (active && slot < b.depth) store_slot(a.out_slots + index, xp, vp);
     if (__builtin_expect(active && slot >= b.depth, 0)) push_overflow(a, key, xp, vp);
+}
+
+__device__ __forceinline__ void store_particle(const StepArgs& a, const BoxDesc& b, float3 xs, float3 vs, uint32_t id,
+                                               uint32_t key, bool active)
+{
+    const SlotClaim claim(a.out_count, key, active);
+    place_particle(a, b, xs, vs, id, key, claim.slot(), active);
 }
 
 // The colliding particles of box-local cell `local` (raw count `raw`): returns
@@ -1376,8 +1392,12 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
         const uint32_t src_slot = (uint32_t)(src_lane - a.in_slots);
         if (!REPLAY && valid) a.zero_count[cur.x + lane] = 0;   // counts of step k-1: step k+1 fills them
         // sampled steps: the previous step's sample of this lane's (lab) cell into the
-        // FP64 sums, where the engine defers it to this step (every cell is one lane's)
-        if (SAMPLE && a.fold_samp && valid) fold_sample(a.fold_samp, a.acc, cur.x + lane, 0, TAPE ? a.fold_count : nullptr);
+        // FP64 sums, where the engine defers it to this step (every cell is one lane's);
+        // its loads wait beside another wait of the run (at the top of the run a sampled
+        // step of 10 x 10 x 102, n = 10 took 10.7 us, so 10.0)
+        auto fold = [&]() {
+            if (SAMPLE && a.fold_samp && valid) fold_sample(a.fold_samp, a.acc, cur.x + lane, 0, TAPE ? a.fold_count : nullptr);
+        };
         next = run_entry<SINGLE>(a, run + warps < run_end ? run + warps : a.num_runs);
         raw_next = lane < (next.y & 63u) ? a.in_count[next.x + lane] : 0u;
         const uint3 cc = storage_coords(b, valid ? c : 0u);
@@ -1450,6 +1470,7 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
             b_end += fit;
         };
         if (STAGED && total) fetch(0, true);
+        if (STAGED) fold();   // while the first copies are under way
         // 32 particles at a time, across batch boundaries
         for (uint32_t g0 = 0; g0 < total; g0 += 32) {
             // lanes past the run's last particle redo that particle and write nothing
@@ -1622,9 +1643,12 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
                     a.tape_lab[id] = lab | (bounced ? kTapeBounce : 0u);
                 }
             }
-            store_particle(a, b, xn, vn, id, key, active);
+            const SlotClaim claim(a.out_count, key, active);
+            if (!STAGED && g0 == 0) fold();   // while the claims are under way
+            place_particle(a, b, xn, vn, id, key, claim.slot(), active);
             gpos = gpos + 32 == kRing ? 0u : gpos + 32;
         }
+        if (!STAGED && total == 0) fold();
         // a run whose last cells are empty: the next run's first batch
         if (SINGLE && !next_prefetched && lane < kBatchCells && raw_next)
             prefetch_l2(a.in_slots + b.slot_base + (uint64_t)(next.x - b.cell_base + lane) * b.depth,
