@@ -1683,7 +1683,8 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
 // while the warp's other cells wait, ranks are looked up in every pass, and five
 // CTA-wide barriers a tile stall its warps.  This kernel's first version
 // took 26, at 64 % issue.  256 x 256 x 66, n = 20 (8.2e7 particles), us a step: tile kernel
-// 3459, this one 2508; sampled 3677 and 2763.  Its code size matters: with
+// 3459, this one 2417; sampled 3677 and 2668 (2503 and 2758 with 32-byte slots in shared
+// memory, whose 16-byte reads meet in half of the banks).  Its code size matters: with
 // the passes over a part unrolled it no longer fit the instruction cache and took
 // 10700 us; with the compiler's own unrolling of the inner loops 3280 (rolled 2773).
 
@@ -1696,7 +1697,7 @@ constexpr uint32_t kTermRow = 36;                  // 4 (sum) + (participant) th
 static_assert(kExtBuf >= 5 * kExtMaxN, "a cell's 4n colliding particles and n ghosts fit the buffer");
 
 struct ExtShared {                   // one per warp
-    Slot buf[kExtBuf];               // by cell, ghosts after its particles; in the end the streamed state
+    float4 pos[kExtBuf], vel[kExtBuf];   // by cell, ghosts after its particles; in the end the streamed state
     union {
         uint32_t ids[kExtBuf + 3 * kExtCells];   // of the particles, each cell's padded to a multiple of 4
         float term[11][kTermRow];                // a colliding cell's terms, by sum and participant
@@ -1817,8 +1818,8 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                 const uint32_t n = i < i1 ? at >> 17 : 0u;
 #pragma unroll 1
                 for (uint32_t k = lane & 3u; k < n; k += 4) {
-                    copy_async16(&sh.buf[(at & 0xFFu) + k].pos, &from[k].pos);
-                    copy_async16(&sh.buf[(at & 0xFFu) + k].vel, &from[k].vel);
+                    copy_async16(&sh.pos[(at & 0xFFu) + k], &from[k].pos);
+                    copy_async16(&sh.vel[(at & 0xFFu) + k], &from[k].vel);
                 }
             }
             copy_async_commit();
@@ -1846,8 +1847,8 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                 float3 gx, gv;
                 Draws<false>::ghost(a, b, step, ref_index(b, cc), j, cell_centre(b, cc), fabsf(s.z), layer, sign, gx, gv);
                 if (g0 + lane < total - real) {
-                    sh.buf[before + j].pos = make_float4(gx.x, gx.y, gx.z, 0.0f);
-                    sh.buf[before + j].vel = make_float4(gv.x, gv.y, gv.z, 0.0f);
+                    sh.pos[before + j] = make_float4(gx.x, gx.y, gx.z, 0.0f);
+                    sh.vel[before + j] = make_float4(gv.x, gv.y, gv.z, 0.0f);
                 }
             }
             copy_async_wait<0>();
@@ -1861,7 +1862,7 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
 #pragma unroll 1
                 for (uint32_t k = lane & 3u; k < end; k += 4) {
                     sh.cell[o + k] = (uint8_t)(i | (k < n ? 0u : kExtGhost));
-                    if (k < n) sh.ids[(at >> 8 & 0x1FFu) + k] = __float_as_uint(sh.buf[o + k].vel.w);
+                    if (k < n) sh.ids[(at >> 8 & 0x1FFu) + k] = __float_as_uint(sh.vel[o + k].w);
                 }
             }
             __syncwarp();
@@ -1871,7 +1872,7 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                 const uint32_t p = min(p0 + lane, total - 1u);
                 const uint32_t info = sh.cell[p];
                 const uint32_t at = __shfl_sync(kFull, range, (int)(info & 31u));
-                const uint32_t id = __float_as_uint(sh.buf[p].vel.w), n = at >> 17;
+                const uint32_t id = __float_as_uint(sh.vel[p].w), n = at >> 17;
                 const uint4* const q = reinterpret_cast<const uint4*>(sh.ids + (at >> 8 & 0x1FFu));
                 uint32_t rank = 0;
 #pragma unroll 1
@@ -1909,7 +1910,7 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
 #pragma unroll 1
                 for (uint32_t k = j; live && k < n; k += 4) {
                     const uint32_t p = k < m ? sh.order[o + k] : gap + k;
-                    const float4 xp = sh.buf[p].pos, vp = sh.buf[p].vel;
+                    const float4 xp = sh.pos[p], vp = sh.vel[p];
                     com.x += (xp.x - centre.x); com.y += (xp.y - centre.y); com.z += (xp.z - centre.z);
                     mean.x += vp.x; mean.y += vp.y; mean.z += vp.z;
                     if (PRESSURE && k < m) real_vz += vp.z;
@@ -1927,7 +1928,7 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
 #pragma unroll 1
                 for (uint32_t k = j; live && k < n; k += 4) {
                     const uint32_t p = k < m ? sh.order[o + k] : gap + k;
-                    const float4 xp = sh.buf[p].pos, vp = sh.buf[p].vel;
+                    const float4 xp = sh.pos[p], vp = sh.vel[p];
                     if (dot3(make_float3(xp.x - com.x, xp.y - com.y, xp.z - com.z), axis) < 0) {
                         proj0 += dot3(make_float3(vp.x - mean.x, vp.y - mean.y, vp.z - mean.z), axis);
                         size0 += 1;
@@ -1965,7 +1966,7 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                         const uint32_t k = k0 + lane;
                         if (k < cn) {
                             const uint32_t p = k < cm ? sh.order[co + k] : cgap + k;
-                            const float4 xp = sh.buf[p].pos, vp = sh.buf[p].vel;
+                            const float4 xp = sh.pos[p], vp = sh.vel[p];
                             const float3 x = make_float3(xp.x - cv.x, xp.y - cv.y, xp.z - cv.z);
                             float3 v = make_float3(vp.x - mv.x, vp.y - mv.y, vp.z - mv.z);
                             const bool sd = dot3(x, ax) < 0;
@@ -1973,7 +1974,7 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                             const float3 cr = cross3(x, v);
                             const float kick = (vr - dot3(v, ax)) + (sd ? t0 : t1);
                             v.x += ax.x * kick; v.y += ax.y * kick; v.z += ax.z * kick;
-                            sh.buf[p].vel = make_float4(v.x, v.y, v.z, vp.w);
+                            sh.vel[p] = make_float4(v.x, v.y, v.z, vp.w);
                             const float sx = x.x * x.x, sy = x.y * x.y, sz = x.z * x.z;
                             sh.term[0][lane] = sd ? vr : 0.0f;   // adding +0 changes no partial (none is -0)
                             sh.term[1][lane] = sd ? 0.0f : vr;
@@ -2007,12 +2008,12 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                         const uint32_t k = k0 + lane;
                         if (k < cn) {
                             const uint32_t p = k < cm ? sh.order[co + k] : cgap + k;
-                            const float4 xp = sh.buf[p].pos;
-                            float4 vp = sh.buf[p].vel;
+                            const float4 xp = sh.pos[p];
+                            float4 vp = sh.vel[p];
                             const float3 x = make_float3(xp.x - cv.x, xp.y - cv.y, xp.z - cv.z);
                             const float3 vm = dot3(x, ax) < 0 ? vm0 : vm1;
                             vp.x -= vm.x; vp.y -= vm.y; vp.z -= vm.z;
-                            sh.buf[p].vel = vp;
+                            sh.vel[p] = vp;
                             const float3 cr = cross3(x, make_float3(vp.x, vp.y, vp.z));
                             sh.term[0][lane] = cr.x;
                             sh.term[1][lane] = cr.y;
@@ -2042,7 +2043,7 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
             auto store_held = [&]() {
                 const uint32_t at = __shfl_sync(kFull, held_base, __ffs(held_peers) - 1) + __popc(held_peers & lanemask_lt());
                 if (held_key == kNoKey) return;
-                const float4 xq = sh.buf[held_p].pos, vq = sh.buf[held_p].vel;
+                const float4 xq = sh.pos[held_p], vq = sh.vel[held_p];
                 const uint32_t index = (uint32_t)b.slot_base + (held_key - b.cell_base) * b.depth + at;
                 if (at < b.depth) store_slot(a.out_slots + index, xq, vq);
                 else push_overflow(a, held_key, xq, vq);
@@ -2052,7 +2053,7 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                 const uint32_t p = min(p0 + lane, total - 1u);
                 const uint32_t info = sh.cell[p], i = info & 31u;
                 const bool active = p0 + lane < total && !(info & kExtGhost);
-                const float4 xp = sh.buf[p].pos, vp = sh.buf[p].vel;
+                const float4 xp = sh.pos[p], vp = sh.vel[p];
                 const float4 k0 = sh.mean[i], k1 = sh.com[i];
                 float3 x = make_float3(xp.x, xp.y, xp.z), v = make_float3(vp.x, vp.y, vp.z);
                 uint32_t side = 0;   // pressure: the wall of a particle that collided beside it
@@ -2094,8 +2095,8 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                 }
                 __syncwarp();   // idle lanes have read the part's last entry
                 if (active) {
-                    sh.buf[p].pos = make_float4(xn.x, xn.y, xn.z, __uint_as_float(kNoExt));
-                    sh.buf[p].vel = make_float4(vn.x, vn.y, vn.z, vp.w);
+                    sh.pos[p] = make_float4(xn.x, xn.y, xn.z, __uint_as_float(kNoExt));
+                    sh.vel[p] = make_float4(vn.x, vn.y, vn.z, vp.w);
                 }
                 const unsigned peers = __match_any_sync(kFull, key);
                 uint32_t base = 0;
