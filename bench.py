@@ -585,7 +585,7 @@ def run_gpu_arm(args, rank, world, local_rank):
                          "frac": achieved / peak, "peak_kind": peak_kind,
                          "traffic": bpp * N if bpp else None, "traffic_source": src,
                          "algorithmic_bytes_per_particle": ALGO_BYTES_PER_PARTICLE,
-                         "kernel": "srd_run_kernel" if algorithm == 0 else "step_kernel<EXTENDED, Philox>",
+                         "kernel": "srd_run_kernel" if algorithm == 0 else "ext_run_kernel",
                          "kernel_ms": per_launch_ms},
             "e2e": e2e,
             "clocks": clocks.summary(),

@@ -96,6 +96,13 @@ class GbError(RuntimeError):
     pass
 
 
+def _references(arrays):
+    return [sys.getrefcount(a) for a in arrays]
+
+
+_IDLE = _references([np.empty(0, np.float32)])[0]   # of an array that only its list refers to
+
+
 def device_allocations() -> int:
     """Device allocations the library has made in this process (all handles)."""
     return int(lib().mpcd_gb_device_allocations())
@@ -176,10 +183,11 @@ class Handle:
         refers to any more where there is such (mapped already: fresh memory costs page faults).
         The handle keeps at most four, of up to 80 MiB each and
         128 MiB in all."""
-        for buf in self._results:
-            if buf.size == n and sys.getrefcount(buf) == 3:   # the list's, the loop's and the call's
+        idle = [r == _IDLE for r in _references(self._results)]
+        for buf, free in zip(self._results, idle):
+            if free and buf.size == n:
                 return buf[:]
-        self._results = [b for b in self._results if sys.getrefcount(b) > 3 or b.size == n]
+        self._results = [b for b, free in zip(self._results, idle) if not free]
         buf = np.empty(n, np.float32)
         if len(self._results) < 4 and buf.nbytes <= 80 << 20 and buf.nbytes + sum(b.nbytes for b in self._results) <= 1 << 27:
             self._results.append(buf)

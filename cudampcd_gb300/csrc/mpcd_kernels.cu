@@ -1,13 +1,13 @@
 // Kernels of the GB300 MPCD step.
 //
-// One launch of step_kernel completes step k of every box: for each cell it
-// stages the cell's bucket (the particles as they enter collision k: streamed
-// and shifted) in shared memory with bulk (TMA) copies, collides them (SRD or
-// extended MPC), undoes the grid shift, accumulates the lab-grid sample if
-// asked, streams each particle for step k+1 and scatters it into the bucket of
-// the cell it then occupies (the other parity).  The post-collision state the
-// reference exposes between steps is never stored: the getters recompute it by
-// replaying the last collision from its (still intact) input buckets.
+// One launch of a step kernel (srd_run_kernel, ext_run_kernel, or step_kernel, which
+// takes what they leave) completes step k of every box: it collides each cell's
+// bucket (the particles as they enter collision k: streamed and shifted; SRD or
+// extended MPC), undoes the grid shift, accumulates the lab-grid sample if asked,
+// streams each particle for step k+1 and scatters it into the bucket of the cell it
+// then occupies (the other parity).  The post-collision state the reference exposes
+// between steps is never stored: the getters recompute it by replaying the last
+// collision from its (still intact) input buckets.
 //
 // Reference path being replaced: translateParticles (simulation_kernels.cu:65-143),
 // srdCollision (srd_collision_strategy.cu:12-157), ext::fusedCollision

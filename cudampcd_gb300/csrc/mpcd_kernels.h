@@ -30,11 +30,12 @@ cudaError_t launch_step(const StepArgs& a, int algorithm, bool table, uint32_t p
 int run_blocks_per_sm(int algorithm);
 int run_warps_per_block(int algorithm);
 uint32_t run_cells_max(int algorithm, uint32_t n);
-// Whether srd_run_kernel can run this step (SRD, Philox draws, no replay, the adjoint
-// tape and the pressure estimator only for one box and not both, n <= 64 in every
-// box, a run table for ensembles and the wall-ghost array when boxes have walls);
-// or ext_run_kernel (extended, Philox draws, n <= kExtMaxN;
-// also the replay of a step that it ran); the caller then sets a.run_kernel, which launch_step and the step's prologue follow.
+// Whether a run kernel can run this step: srd_run_kernel (SRD, Philox draws, no replay, the
+// adjoint tape and the pressure estimator only for one box and not both, n <= 64 in every
+// box, a run table for ensembles and the wall-ghost array when boxes have walls) or
+// ext_run_kernel (extended, Philox draws, n <= kExtMaxN).  The caller then sets
+// a.run_kernel, which launch_step and the step's prologue follow; a replay sets what its
+// step ran on.
 bool run_kernel_takes(const StepArgs& a, int algorithm, bool table);
 // state->step_base += steps (the last node of a replayed step graph).
 cudaError_t launch_advance(DeviceState* state, unsigned steps, cudaStream_t st);
