@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -80,6 +81,56 @@ struct DeviceBuffer {
     T* as() const { return static_cast<T*>(p); }
 };
 
+// Pinned words for small device-to-host copies: 64 of them, a cache line each, in one page
+// that the process allocates once (a pinned allocation per handle took 0.1 ms of the 0.4 of a
+// small one).  A handle takes one and gives it back; past 64 handles the word is null and
+// the copy goes to pageable memory.
+class PinnedWords {
+public:
+    static unsigned int* take()
+    {
+        std::lock_guard<std::mutex> lock(mutex());
+        static unsigned int* page = nullptr;
+        if (!page && cudaHostAlloc((void**)&page, kWords * kStride * sizeof(unsigned int), cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            page = nullptr;
+            return nullptr;
+        }
+        base() = page;
+        for (int i = 0; i < kWords; ++i)
+            if (!(used() >> i & 1ull)) {
+                used() |= 1ull << i;
+                return page + i * kStride;
+            }
+        return nullptr;
+    }
+
+    static void give(unsigned int* word)
+    {
+        if (!word) return;
+        std::lock_guard<std::mutex> lock(mutex());
+        used() &= ~(1ull << ((word - base()) / kStride));
+    }
+
+private:
+    static constexpr int kWords = 64, kStride = 16;
+    static std::mutex& mutex()
+    {
+        static std::mutex m;
+        return m;
+    }
+    static unsigned long long& used()
+    {
+        static unsigned long long bits = 0;
+        return bits;
+    }
+    static unsigned int*& base()
+    {
+        static unsigned int* p = nullptr;
+        return p;
+    }
+};
+
 class Error : public std::exception {
 public:
     Error(int code, std::string msg) : code_(code), msg_(std::move(msg)) {}
@@ -145,7 +196,6 @@ public:
             if (branches_.join[i]) cudaEventDestroy(branches_.join[i]);
         }
         if (branches_.fork) cudaEventDestroy(branches_.fork);
-        if (flags_host_) cudaFreeHost(flags_host_);
     }
 
     // ------------------------------------------------------------ reference Backend interface
@@ -1068,7 +1118,7 @@ private:
         if (walls_) check(ghosts_.alloc(sizeof(GhostSum) * walls_ * 2), "alloc wall ghosts");   // two parities
         check(box_shifts_.alloc(sizeof(float4) * 4 * boxes_.size()), "alloc box shifts");
         check(state_.alloc(sizeof(DeviceState)), "alloc state");
-        check(cudaMallocHost((void**)&flags_host_, sizeof *flags_host_), "alloc error flags");
+        flags_host_.word = PinnedWords::take();
         check(cudaMemset(state_.p, 0, sizeof(DeviceState)), "clear state");
         check(samp_.alloc(sizeof(float4) * cells_ * 2), "alloc sample");   // two parities
         check(cudaMemset(samp_.p, 0, samp_.bytes), "clear sample");
@@ -1487,11 +1537,12 @@ private:
     void check_device_errors()
     {
         check(cudaGetLastError(), "launch");
-        check(cudaMemcpyAsync(flags_host_, (char*)state_.p + offsetof(DeviceState, error_flags), sizeof *flags_host_,
-                              cudaMemcpyDeviceToHost, stream_),
+        unsigned int word = 0, *const to = flags_host_.word ? flags_host_.word : &word;
+        check(cudaMemcpyAsync(to, (char*)state_.p + offsetof(DeviceState, error_flags), sizeof *to, cudaMemcpyDeviceToHost,
+                              stream_),
               "error flags");
         check(cudaStreamSynchronize(stream_), "step");
-        const unsigned int flags = *flags_host_;
+        const unsigned int flags = *to;
         if (flags & kErrOverflowListFull) throw Error(MPCD_GB_EDEVICE, "cell overflow list exhausted");
         if (flags & kErrWaitTimeout) throw Error(MPCD_GB_EDEVICE, "device wait timed out");
         if (flags & kErrKeyMismatch) throw Error(MPCD_GB_EDEVICE, "particle found in the wrong cell bucket");
@@ -1524,7 +1575,10 @@ private:
     bool use_table_ = false;
     bool last_step_table_ = false;
     int32_t last_step_run_ = 0, graph_run_ = 0;   // StepArgs::run_kernel of the last step, of the step graphs
-    unsigned int* flags_host_ = nullptr;   // pinned: error flags read at the end of a call
+    struct PinnedWord {
+        unsigned int* word = nullptr;
+        ~PinnedWord() { PinnedWords::give(word); }
+    } flags_host_;   // error flags read at the end of a call
     bool direct_read_ = false;   // the state of this step was replayed into a caller's buffers
     bool dense_valid_ = false;   // dense_pos_ / dense_vel_ hold the state after step step_ - 1
     DrawTables tables_{};
