@@ -577,8 +577,7 @@ public:
             auto at = [&](int i) {   // step i of the segment; three sets of cells in turn
                 AdjointStep t{};
                 t.step = adj_s0_ + (uint64_t)j * every + i;
-                t.key = tkey_.as<uint32_t>() + (size_t)i * N_;
-                t.lab = tlab_.as<uint32_t>() + (size_t)i * N_;
+                t.tape = tape_.as<uint2>() + (size_t)i * N_;
                 t.ncell = tncell_.as<uint32_t>() + (size_t)i * cells_;
                 t.lab_count = tcnt_.as<uint32_t>() + (size_t)i * cells_;
                 t.cells = adj_cells_.as<AdjointCell>() + (size_t)(i % 3) * cells_;
@@ -617,8 +616,16 @@ public:
                                           stream_),
                           "tape read");
             };
-            down(key, tkey_, N_);
-            down(lab, tlab_, N_);
+            if (key || lab) {
+                std::vector<uint2> both(N_ * (size_t)k);
+                check(cudaMemcpyAsync(both.data(), tape_.p, sizeof(uint2) * both.size(), cudaMemcpyDeviceToHost, stream_),
+                      "tape read");
+                check(cudaStreamSynchronize(stream_), "tape read");
+                for (size_t i = 0; i < both.size(); ++i) {
+                    if (key) key[t0 * N_ + i] = both[i].x;
+                    if (lab) lab[t0 * N_ + i] = both[i].y;
+                }
+            }
             down(ncell, tncell_, cells_);
             down(lab_count, tcnt_, cells_);
             if (j == 0 && bounce0)
@@ -1397,8 +1404,7 @@ private:
         auto need = [&](DeviceBuffer& d, size_t bytes, const char* what) {
             if (d.bytes < bytes) check(d.alloc(bytes), what);
         };
-        need(tkey_, sizeof(uint32_t) * N_ * K, "alloc tape");
-        need(tlab_, sizeof(uint32_t) * N_ * K, "alloc tape");
+        need(tape_, sizeof(uint2) * N_ * K, "alloc tape");
         need(tncell_, sizeof(uint32_t) * cells_ * K, "alloc tape");
         need(tcnt_, sizeof(uint32_t) * cells_ * K, "alloc tape");
         need(tb0_, sizeof(uint32_t) * N_, "alloc tape");
@@ -1420,7 +1426,7 @@ private:
             alloc_tape(steps);
         } catch (const Error& e) {
             if (e.code() != MPCD_GB_ENOMEM) throw;
-            for (DeviceBuffer* d : {&tkey_, &tlab_, &tncell_, &tcnt_}) d->release();
+            for (DeviceBuffer* d : {&tape_, &tncell_, &tcnt_}) d->release();
             return false;
         }
         return true;
@@ -1435,8 +1441,7 @@ private:
         for (int i = 0; i < steps; ++i) {
             StepArgs a = args(step_);
             a.sample = 1;
-            a.tape_key = tkey_.as<uint32_t>() + (size_t)i * N_;
-            a.tape_lab = tlab_.as<uint32_t>() + (size_t)i * N_;
+            a.tape = tape_.as<uint2>() + (size_t)i * N_;
             a.tape_ncell = tncell_.as<uint32_t>() + (size_t)i * cells_;
             use_run_kernel_ghosts(a, false);   // the run kernel records the tape of single-box SRD steps
             const bool fold = a.run_kernel && i > 1;   // (the first sample is folded as a snapshot)
@@ -1480,7 +1485,7 @@ private:
         const uint64_t k = step_;
         StepArgs a = args(k - 1);   // out_* = buckets, counts and overflow list of step k
         a.out_count = count_[k % 3].as<uint32_t>();
-        a.tape_lab = tape_b0;
+        a.tape_b0 = tape_b0;
         check(launch_scatter(a, pos ? pos : dense_pos_.as<float>(), vel ? vel : dense_vel_.as<float>(),
                              pos ? dense_pos_.as<float>() : nullptr, vel ? dense_vel_.as<float>() : nullptr, N_, cells_,
                              count_[(k + 1) % 3].as<uint32_t>(), sms_, stream_),
@@ -1596,7 +1601,7 @@ private:
         dense_vel_, offsets_, scan_status_, scan_counter_, partial_;
     DeviceBuffer t_count_, t_gpos_, t_gvel_, t_axis_, t_gate_, t_gauss_;
     // adjoint: checkpoints, tape of one segment, adjoint state
-    DeviceBuffer ckpt_, tkey_, tlab_, tncell_, tcnt_, tb0_, lam_, adj_cells_, gsum_;
+    DeviceBuffer ckpt_, tape_, tncell_, tcnt_, tb0_, lam_, adj_cells_, gsum_;
     bool adj_valid_ = false;
     bool adj_taped_ = false;   // the tape holds every step of the last forward
     bool pressure_ = false;

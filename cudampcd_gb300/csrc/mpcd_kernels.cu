@@ -590,10 +590,9 @@ __device__ void overflow_pass(const StepArgs& a, uint64_t step)
                 key = b.cell_base + storage_index(b, cell_of_wrapped(b, xs));
                 if (a.pressure && b.wall_z && vs.z != v.z)   // bounce-back: 2 |v_z| outward
                     atomicAdd(&a.state->wall_impulse[v.z > 0.0f ? 1 : 0], 2.0 * fabs((double)v.z));
-                if (a.tape_key) {
+                if (a.tape) {
                     const bool bounced = vs.x != v.x || vs.y != v.y || vs.z != v.z;
-                    a.tape_key[id] = kTapeNone;
-                    a.tape_lab[id] = (b.cell_base + storage_index(b, cell_of_wrapped(b, x))) | (bounced ? kTapeBounce : 0u);
+                    a.tape[id] = make_uint2(kTapeNone, (b.cell_base + storage_index(b, cell_of_wrapped(b, x))) | (bounced ? kTapeBounce : 0u));
                 }
             }
         }
@@ -943,13 +942,12 @@ __global__ void __launch_bounds__(kThreads, 4) step_kernel(const StepArgs a, uin
                 const uint32_t next = b.cell_base + storage_index(b, cell_of_wrapped(b, xn));
                 s_buf[p].pos = make_float4(xn.x, xn.y, xn.z, __uint_as_float(next));
                 s_buf[p].vel = make_float4(vn.x, vn.y, vn.z, vp.w);
-                const bool need_lab = a.sample || (ALGO == 0 && a.tape_key);
+                const bool need_lab = a.sample || (ALGO == 0 && a.tape);
                 const uint32_t lab = need_lab ? b.cell_base + storage_index(b, cell_of_wrapped(b, x)) : 0u;
-                if (ALGO == 0 && a.tape_key) {
+                if (ALGO == 0 && a.tape) {
                     const uint32_t id = __float_as_uint(vp.w);
                     const bool bounced = vn.x != v.x || vn.y != v.y || vn.z != v.z;
-                    a.tape_key[id] = n > 1 ? b.cell_base + c0 + ci : kTapeNone;
-                    a.tape_lab[id] = lab | (bounced ? kTapeBounce : 0u);
+                    a.tape[id] = make_uint2(n > 1 ? b.cell_base + c0 + ci : kTapeNone, lab | (bounced ? kTapeBounce : 0u));
                 }
                 if (a.sample) sample_add(a.samp, lab, v, true);
             };
@@ -1639,8 +1637,7 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
                 if (SAMPLE) sample_add(a.samp, lab, v, active);
                 if (TAPE && active) {   // collision cell (or none), lab cell and the bounce of the streaming that follows
                     const bool bounced = vn.x != v.x || vn.y != v.y || vn.z != v.z;
-                    a.tape_key[id] = __float_as_uint(cd.w) > 1 ? cur.x + i : kTapeNone;
-                    a.tape_lab[id] = lab | (bounced ? kTapeBounce : 0u);
+                    a.tape[id] = make_uint2(__float_as_uint(cd.w) > 1 ? cur.x + i : kTapeNone, lab | (bounced ? kTapeBounce : 0u));
                 }
             }
             const SlotClaim claim(a.out_count, key, active);
@@ -2391,8 +2388,8 @@ __global__ void __launch_bounds__(kThreads, 4) scatter_kernel(const StepArgs a, 
             uint32_t cell;
             x[u] = stream_shift_cell(b, x[u], v[u], SINGLE ? shift : grid_shift(b, box[u], a.step + 1, a.state), cell);
             key[u] = active ? b.cell_base + cell : kNoKey;
-            if (a.tape_lab && active)
-                a.tape_lab[i] = (v[u].x != v0.x || v[u].y != v0.y || v[u].z != v0.z) ? kTapeBounce : 0u;
+            if (a.tape_b0 && active)
+                a.tape_b0[i] = (v[u].x != v0.x || v[u].y != v0.y || v[u].z != v0.z) ? kTapeBounce : 0u;
             peers[u] = __match_any_sync(kFull, key[u]);
             slot[u] = 0;
             if (active && (int)lane == __ffs(peers[u]) - 1) slot[u] = atomicAdd(a.out_count + key[u], (uint32_t)__popc(peers[u]));
@@ -2743,8 +2740,9 @@ __global__ void __launch_bounds__(kThreads, 6) adjoint_sweep_kernel(BoxDesc b, u
     for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
         const float4 l4 = lam[i];
         float3 m = make_float3(l4.x, l4.y, l4.z);
-        const uint32_t kh = HI ? hi.key[i] : kTapeNone;
-        const uint32_t l = LO ? lo.lab[i] : 0u, kl = LO ? lo.key[i] : kTapeNone;
+        const uint32_t kh = HI ? hi.tape[i].x : kTapeNone;
+        const uint2 at = LO ? lo.tape[i] : make_uint2(kTapeNone, 0u);
+        const uint32_t l = at.y, kl = at.x;
         if (HI && kh != kTapeNone) {
             float4 cs, ax;
             load_cell(hi.cells + (kh - b.cell_base), cs, ax);
@@ -2872,8 +2870,8 @@ bool run_kernel_takes(const StepArgs& a, int algorithm, bool table)
     if (algorithm == 1)
         return !table && (!a.pressure || a.nboxes == 1) && (a.ghosts || !a.total_walls) && a.box_shifts && (a.nboxes == 1 || a.run_info) &&
                a.boxes_n_max <= kExtMaxN;
-    return algorithm == 0 && !table && !a.replay && (!a.tape_key || (a.nboxes == 1 && a.sample)) &&
-           (!a.pressure || (a.nboxes == 1 && !a.tape_key)) &&
+    return algorithm == 0 && !table && !a.replay && (!a.tape || (a.nboxes == 1 && a.sample)) &&
+           (!a.pressure || (a.nboxes == 1 && !a.tape)) &&
            (a.ghosts || !a.total_walls) && a.box_shifts && (a.nboxes == 1 || a.run_info) &&
            a.boxes_n_max <= kRunMaxN;
 }
@@ -2907,7 +2905,7 @@ cudaError_t launch_step(const StepArgs& a, int algorithm, bool table, uint32_t p
         for (int i = 0; i < nused; ++i) {
             const int cls = used[i];
             const bool staged = run_staged(a.nboxes == 1, cls, a.boxes_n_max);
-            const StepFnRun f = run_fn(cls, staged, a.sample, a.nboxes == 1, a.replay, a.replay ? a.map != nullptr : a.tape_key != nullptr, a.pressure);
+            const StepFnRun f = run_fn(cls, staged, a.sample, a.nboxes == 1, a.replay, a.replay ? a.map != nullptr : a.tape != nullptr, a.pressure);
             const uint32_t runs = a.run_class[cls + 1] - a.run_class[cls];
             const unsigned blocks = std::min((unsigned)grid, (runs + kRunWarps - 1) / (unsigned)kRunWarps);
             if (a.nboxes == 1 && !a.replay) {   // (an ensemble's classes fork and join)

@@ -200,14 +200,16 @@ struct StepArgs {
     float ext_axis[13][3];        // discrete axis set of the extended collision
     DrawTables draws;             // used by the injected-draw instantiation
     // adjoint tape of this step, by particle id / cell (null: not recorded):
-    //   tape_key[id]  = collision cell (global storage index) if the particle was
-    //                   collided (cell with n > 1), else kTapeNone;
-    //   tape_lab[id]  = lab cell it was sampled in (global storage index) |
-    //                   kTapeBounce if the streaming that follows bounced it;
+    //   tape[id].x = collision cell (global storage index) if the particle was
+    //                collided (cell with n > 1), else kTapeNone;
+    //   tape[id].y = lab cell it was sampled in (global storage index) |
+    //                kTapeBounce if the streaming that follows bounced it (one 8-byte
+    //                store at a random place; two of 4 bytes: taped step of 1.3 M particles
+    //                42.1 us against 36.5, of 16 M 1241 against 815);
     //   tape_ncell[c] = particles incl. ghosts of collided cell c (storage index).
-    // The scatter records only the bounce bit of its streaming in tape_lab.
-    uint32_t* tape_key;
-    uint32_t* tape_lab;
+    // The scatter records only the bounce bit of its streaming, in tape_b0.
+    uint2* tape;
+    uint32_t* tape_b0;
     uint32_t* tape_ncell;
     // pressure estimator on: accumulate the z impulse the fluid gives the walls
     // (bounce-backs and collisions in the wall-layer cells) into state->wall_impulse
@@ -236,7 +238,8 @@ constexpr uint32_t kTapeBounce = 0x80000000u;
 // One step of the adjoint tape (by particle id / storage cell) and its cells.
 struct AdjointStep {
     uint64_t step;
-    const uint32_t *key, *lab, *ncell, *lab_count;
+    const uint2* tape;
+    const uint32_t *ncell, *lab_count;
     AdjointCell* cells;
 };
 
