@@ -571,6 +571,8 @@ public:
         alloc_tape(adj_taped_ ? adj_steps_ : adj_every_);
         check(cudaMemsetAsync(lam_.p, 0, lam_.bytes, stream_), "adjoint");
         check(cudaMemsetAsync(gsum_.p, 0, gsum_.bytes, stream_), "adjoint");
+        float* const most = reinterpret_cast<float*>(gsum_.as<double>() + 1);
+        check(launch_adjoint_scale(b, (uint64_t)adj_steps_, d_dU, most, stream_), "adjoint scale");
         const int every = adj_taped_ ? adj_steps_ : adj_every_, nseg = (adj_steps_ + every - 1) / every;
         for (int j = nseg - 1; j >= 0; --j) {
             const int k = adj_taped_ ? adj_steps_ : record_segment(j);
@@ -581,6 +583,8 @@ public:
                 t.ncell = tncell_.as<uint32_t>() + (size_t)i * cells_;
                 t.lab_count = tcnt_.as<uint32_t>() + (size_t)i * cells_;
                 t.cells = adj_cells_.as<AdjointCell>() + (size_t)(i % 3) * cells_;
+                t.term = adj_term_.as<float>() + (size_t)(i % 3) * cells_;
+                t.left = (uint32_t)(adj_steps_ - (j * every + i));
                 return t;
             };
             check(launch_adjoint_cells(b, at(k - 1), (uint64_t)adj_steps_, d_dU, sms_ * 6, stream_), "adjoint cells");
@@ -588,7 +592,7 @@ public:
                 const AdjointStep hi = at(i), lo = at(i > 0 ? i - 1 : 0), prev = at(i > 1 ? i - 2 : 0);
                 check(launch_adjoint_sweep(b, (uint64_t)adj_steps_, lam_.as<float4>(), i < k ? &hi : nullptr,
                                            i > 0 ? &lo : nullptr, i > 1 ? &prev : nullptr, d_dU, gsum_.as<double>(),
-                                           tb0_.as<uint32_t>(), i == 0 && j == 0 ? d_dv0 : nullptr, sms_ * 6, stream_),
+                                           tb0_.as<uint32_t>(), i == 0 && j == 0 ? d_dv0 : nullptr, most, sms_ * 6, stream_),
                       "adjoint step");
             }
         }
@@ -1410,7 +1414,8 @@ private:
         need(tb0_, sizeof(uint32_t) * N_, "alloc tape");
         need(lam_, sizeof(float4) * N_, "alloc adjoint");
         need(adj_cells_, sizeof(AdjointCell) * cells_ * 3, "alloc adjoint");
-        need(gsum_, sizeof(double), "alloc adjoint");
+        need(adj_term_, sizeof(float) * cells_ * 3, "alloc adjoint");
+        need(gsum_, 2 * sizeof(double), "alloc adjoint");   // the drag's sum, then the scale of the cell sums
     }
 
     // Whether the forward records the tape of all its steps, so that the backward
@@ -1443,6 +1448,12 @@ private:
             a.sample = 1;
             a.tape = tape_.as<uint2>() + (size_t)i * N_;
             a.tape_ncell = tncell_.as<uint32_t>() + (size_t)i * cells_;
+            // 32-cell runs whatever the box: their order of arrival is that of the sampled sums,
+            // whose last bits reach the drag gradient (shorter runs moved it by up to 6e-9 in small boxes)
+            a.box0.run_cells = run_cells_max(params_.algorithm, boxes_[0].n);
+            const uint32_t runs = (boxes_[0].C + a.box0.run_cells - 1) / a.box0.run_cells;
+            for (uint32_t& r : a.run_class) r = r ? runs : 0;
+            a.num_runs = runs;
             use_run_kernel_ghosts(a, false);   // the run kernel records the tape of single-box SRD steps
             const bool fold = a.run_kernel && i > 1;   // (the first sample is folded as a snapshot)
             if (fold) {
@@ -1601,7 +1612,7 @@ private:
         dense_vel_, offsets_, scan_status_, scan_counter_, partial_;
     DeviceBuffer t_count_, t_gpos_, t_gvel_, t_axis_, t_gate_, t_gauss_;
     // adjoint: checkpoints, tape of one segment, adjoint state
-    DeviceBuffer ckpt_, tape_, tncell_, tcnt_, tb0_, lam_, adj_cells_, gsum_;
+    DeviceBuffer ckpt_, tape_, tncell_, tcnt_, tb0_, lam_, adj_cells_, adj_term_, gsum_;
     bool adj_valid_ = false;
     bool adj_taped_ = false;   // the tape holds every step of the last forward
     bool pressure_ = false;

@@ -272,15 +272,21 @@ __device__ __forceinline__ uint32_t cell_source(const StepArgs& a, const BoxDesc
 
 // ------------------------------------------------------------------ draws
 
-// SRD rotation axis of cell `ref` (box-local reference index) at `step`: uniform on the sphere.
+// SRD rotation axis of a cell from its two random words: uniform on the sphere.
+__device__ __forceinline__ float3 srd_axis_of(uint32_t a, uint32_t d)
+{
+    const float z = 1.0f - 2.0f * u01(a);
+    const float rho = sqrtf(fmaxf(0.0f, 1.0f - z * z));
+    float s, c;
+    sincospif(2.0f * u01(d), &s, &c);
+    return make_float3(rho * c, rho * s, z);
+}
+
+// The axis of cell `ref` (box-local reference index) at `step`.
 __device__ __forceinline__ float3 srd_axis_philox(const BoxDesc& b, uint64_t step, uint32_t ref)
 {
     const uint4 o = draw(b, step, kAxis, ref, 0);
-    const float z = 1.0f - 2.0f * u01(o.x);
-    const float rho = sqrtf(fmaxf(0.0f, 1.0f - z * z));
-    float s, c;
-    sincospif(2.0f * u01(o.y), &s, &c);
-    return make_float3(rho * c, rho * s, z);
+    return srd_axis_of(o.x, o.y);
 }
 
 // Velocity of wall ghost j of cell `ref` (Maxwell-Boltzmann, sqrt(T) per component).
@@ -2692,17 +2698,20 @@ __global__ void __launch_bounds__(kThreads) profile_kernel(const SampleAcc* acc,
     if (threadIdx.x == 0) profile[blockIdx.x] = (float)(red[0] * inv);
 }
 
-// Cells of a step (storage order), before its sweep adds to their sums: N_c, the axis and
-// the sampling term, so that a particle neither draws an axis nor divides.
+// Cells of a step (storage order), before its sweep adds to their sums: N_c, the random
+// words of the axis and the sampling term, so that a particle draws nothing and divides no
+// FP64.
 __device__ __forceinline__ void adjoint_cells(const BoxDesc& b, const AdjointStep& t, const float* dU, double w)
 {
     for (uint32_t c = blockIdx.x * kThreads + threadIdx.x; c < b.C; c += gridDim.x * kThreads) {
         const uint32_t cnt = t.lab_count[c], n = t.ncell[c];
         const uint3 cc = storage_coords(b, c);
         const float term = cnt ? (float)((double)dU[cc.z] * w / (double)cnt) : 0.0f;
-        const float3 a = srd_axis_philox(b, t.step, ref_index(b, cc));
-        t.cells[c].sum = make_float4(0.0f, 0.0f, 0.0f, n ? 1.0f / (float)n : 0.0f);
-        t.cells[c].axis = make_float4(a.x, a.y, a.z, term);
+        const uint4 o = draw(b, t.step, kAxis, ref_index(b, cc), 0);
+        t.cells[c].sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        t.cells[c].axis = make_float4(0.0f, 0.0f, __uint_as_float((o.x & ~0xFFu) | (n & 0xFFu)),
+                                      __uint_as_float((o.y & ~0xFFu) | (n >> 8)));   // (an axis uses 24 bits a word; n < 2^16)
+        t.term[c] = term;
     }
 }
 
@@ -2721,19 +2730,57 @@ __global__ void __launch_bounds__(kThreads) adjoint_cells_kernel(BoxDesc b, Adjo
 // dL/dV0 = B_0 lambda_0, the bounces of the initial streaming in b0.
 // What bounds it is the latency of three random sectors a particle (its cells' AdjointCell
 // and the atomic on one) behind the tape's ids.  One launch and one pass over lambda a
-// step instead of three launches and two: 64 x 64 x 34, n = 10, 46.4 -> 24.4 us a step (28.0 with
-// the cell read as two 16-byte loads; two to four particles a thread at once: 28 to 37).
+// step instead of three launches and two: 64 x 64 x 34, n = 10, 46.4 -> 24.4 us a step, with
+// plain sums (28.0 with the cell read as two 16-byte loads; two to four particles a thread
+// at once: 28 to 37).
+// The sums over a cell do not depend on the order in which the atomics arrive: a value is
+// split in two, each a multiple of a quantum, and neither part's sum rounds (SumSplit).
+// With plain FP32 sums the drag gradients of one forward at 64 x 64 x 34, n = 10, 200 steps
+// had a standard deviation of 9e-10 of their value, and 4e-10 with x alone split.  The rests
+// are a second atomic on the same sector, in which the axis's two random words take the
+// place of its components, and the sampling term has an array of its own: 24.4 us a step
+// with plain sums, 28.4 so, 34.0 with a second sector for the rests.
 // A cell with one 256-bit load (the cells of step hi are read-only in a sweep).
 __device__ __forceinline__ void load_cell(const AdjointCell* c, float4& sum, float4& axis)
 {
     load_slot(reinterpret_cast<const Slot*>(c), sum, axis);
 }
 
+// The split of values to be summed over a cell, at a step with `left` steps of the forward
+// to go.  With A = left max |dU| / (samples Lx Ly), about the sum of a cell beside the
+// largest dU, the coarse quantum is 2^-16 A, so that a sum up to 2^8 A is exact in 24 bits, and the
+// fine one 2^-17 of that: the rests of 256 particles, half a coarse quantum each at most,
+// stay below 2^24 of them.  Adding and taking away 1.5 x 2^23 quanta rounds to a multiple.
+// Where A is 0 or too far from 1 for it, the coarse part is the value and the rest 0.
+struct SumSplit {
+    float coarse, fine;
+    __device__ __forceinline__ SumSplit(float most, uint32_t left)
+    {
+        const float top = __uint_as_float(__float_as_uint((float)left * most) & 0x7F800000u) * 2.0f;   // a power of two
+        const bool plain = !(top > 0x1p-80f && top < 0x1p100f);
+        coarse = plain ? 0.0f : top * (1.5f * 0x1p23f * 0x1p-16f);
+        fine = coarse * 0x1p-17f;
+    }
+    __device__ __forceinline__ float high(float v) const { return (v + coarse) - coarse; }
+    __device__ __forceinline__ float rest(float v, float high) const { return coarse != 0.0f ? ((v - high) + fine) - fine : 0.0f; }
+};
+
+// *most = max |dU[z]| w over the layers (NaN ignored): the scale of the sweep's sums.
+__global__ void adjoint_scale_kernel(const float* dU, int layers, double w, float* most)
+{
+    float m = 0.0f;
+    for (int z = threadIdx.x; z < layers; z += 32) m = fmaxf(m, fabsf(dU[z]));
+    for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(kFull, m, o));
+    if (threadIdx.x == 0) *most = (float)((double)m * w);
+}
+
 template <bool HI, bool LO>
 __global__ void __launch_bounds__(kThreads, 6) adjoint_sweep_kernel(BoxDesc b, uint32_t n, float4* lam, AdjointStep hi,
                                                                     AdjointStep lo, AdjointStep prev, const float* dU,
-                                                                    double w, double* gsum, const uint32_t* b0, float* out)
+                                                                    double w, double* gsum, const uint32_t* b0, float* out,
+                                                                    const float* most)
 {
+    const SumSplit split(*most, LO ? lo.left : 0u);
     if (LO && prev.cells) adjoint_cells(b, prev, dU, w);
     double gl = 0;
 #pragma unroll 2
@@ -2746,8 +2793,10 @@ __global__ void __launch_bounds__(kThreads, 6) adjoint_sweep_kernel(BoxDesc b, u
         if (HI && kh != kTapeNone) {
             float4 cs, ax;
             load_cell(hi.cells + (kh - b.cell_base), cs, ax);
-            const float3 sc = make_float3(cs.x * cs.w, cs.y * cs.w, cs.z * cs.w);
-            const float3 a = make_float3(ax.x, ax.y, ax.z);
+            const uint32_t p0 = __float_as_uint(ax.z), p1 = __float_as_uint(ax.w);
+            const float inv = 1.0f / (float)((p0 & 0xFFu) | (p1 & 0xFFu) << 8);
+            const float3 sc = make_float3((cs.x + cs.w) * inv, (cs.y + ax.x) * inv, (cs.z + ax.y) * inv);
+            const float3 a = srd_axis_of(p0, p1);
             const float3 wv = make_float3(m.x - sc.x, m.y - sc.y, m.z - sc.z);
             const float d = dot3(wv, a);
             const float3 para = make_float3(a.x * d, a.y * d, a.z * d);
@@ -2759,9 +2808,12 @@ __global__ void __launch_bounds__(kThreads, 6) adjoint_sweep_kernel(BoxDesc b, u
         }
         if (LO) {
             if (l & kTapeBounce) m = make_float3(-m.x, -m.y, -m.z);
-            m.x += __ldcg(&lo.cells[(l & ~kTapeBounce) - b.cell_base].axis.w);
+            m.x += __ldg(lo.term + ((l & ~kTapeBounce) - b.cell_base));
             if (kl != kTapeNone) {
-                atomicAdd(&lo.cells[kl - b.cell_base].sum, make_float4(m.x, m.y, m.z, 0.0f));
+                const float3 h = make_float3(split.high(m.x), split.high(m.y), split.high(m.z));
+                AdjointCell* const c = lo.cells + (kl - b.cell_base);
+                atomicAdd(&c->sum, make_float4(h.x, h.y, h.z, split.rest(m.x, h.x)));
+                atomicAdd(reinterpret_cast<float2*>(&c->axis), make_float2(split.rest(m.y, h.y), split.rest(m.z, h.z)));
                 gl += (double)m.x;
             }
         }
@@ -3026,14 +3078,20 @@ cudaError_t launch_adjoint_cells(const BoxDesc& b, const AdjointStep& t, uint64_
     return cudaGetLastError();
 }
 
+cudaError_t launch_adjoint_scale(const BoxDesc& b, uint64_t samples, const float* dU, float* most, cudaStream_t st)
+{
+    adjoint_scale_kernel<<<1, 32, 0, st>>>(dU, b.L[2], 1.0 / ((double)samples * (double)b.L[0] * (double)b.L[1]), most);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_adjoint_sweep(const BoxDesc& b, uint64_t samples, float4* lam, const AdjointStep* hi,
                                  const AdjointStep* lo, const AdjointStep* prev, const float* dU, double* gsum,
-                                 const uint32_t* b0, float* out, int grid, cudaStream_t st)
+                                 const uint32_t* b0, float* out, const float* most, int grid, cudaStream_t st)
 {
     const double w = 1.0 / ((double)samples * (double)b.L[0] * (double)b.L[1]);
     const AdjointStep none{};
     auto f = hi ? (lo ? adjoint_sweep_kernel<true, true> : adjoint_sweep_kernel<true, false>) : adjoint_sweep_kernel<false, true>;
-    f<<<grid, kThreads, 0, st>>>(b, b.N, lam, hi ? *hi : none, lo ? *lo : none, prev ? *prev : none, dU, w, gsum, b0, out);
+    f<<<grid, kThreads, 0, st>>>(b, b.N, lam, hi ? *hi : none, lo ? *lo : none, prev ? *prev : none, dU, w, gsum, b0, out, most);
     return cudaGetLastError();
 }
 

@@ -58,15 +58,16 @@ cudaError_t launch_sample_finalize(float4* samp, SampleAcc* acc, uint64_t cells,
 cudaError_t launch_mean_fields(const SampleAcc* acc, const BoxDesc* boxes, int nboxes, uint64_t cells, double inverse,
                                float* density, float* velocity, cudaStream_t st);
 // Adjoint of the sampled x-velocity profile (single box, SRD): U(z) from the sample
-// sums of `samples` steps; the cells of a step before its sweep; one launch of the
-// reverse sweep: the end of step hi (or null) and the start of step lo (or null), the
+// sums of `samples` steps; the cells of a step before its sweep; the scale *most of the
+// sweep's sums; one launch of the reverse sweep: the end of step hi (or null) and the start of step lo (or null), the
 // cells of step prev on the way (or null); the last launch writes dL/dV0 to out.
 cudaError_t launch_profile(const SampleAcc* acc, const BoxDesc& b, uint64_t samples, float* profile, cudaStream_t st);
 cudaError_t launch_adjoint_cells(const BoxDesc& b, const AdjointStep& t, uint64_t samples, const float* dU, int grid,
                                  cudaStream_t st);
+cudaError_t launch_adjoint_scale(const BoxDesc& b, uint64_t samples, const float* dU, float* most, cudaStream_t st);
 cudaError_t launch_adjoint_sweep(const BoxDesc& b, uint64_t samples, float4* lam, const AdjointStep* hi,
                                  const AdjointStep* lo, const AdjointStep* prev, const float* dU, double* gsum,
-                                 const uint32_t* b0, float* out, int grid, cudaStream_t st);
+                                 const uint32_t* b0, float* out, const float* most, int grid, cudaStream_t st);
 // Layout dump, after the step's overflow selection: cells in storage order, stable
 // order within a cell (decoupled look-back scan of the counts, then one thread per
 // cell), then the overflow list's particles that do not collide, in any order;

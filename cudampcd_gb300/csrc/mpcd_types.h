@@ -137,9 +137,9 @@ struct DrawTables {
 
 // What a pass over particles needs of a cell, one sector.  Replays that gather: the mean
 // velocity and, as bits, the entries in sum, the rotation axis in axis.
-// Adjoint sweep, a cell at one step: the sums of mu over its collided particles and
-// 1 / N_c in sum.w; the rotation axis (as a collision cell), and in axis.w its sampling
-// term dU(z) / (samples Lx Ly count) (as a lab cell).
+// Adjoint sweep, a collision cell at one step: the sums of mu over its particles, the coarse
+// parts in sum.xyz and the rests in sum.w, axis.x and axis.y; as bits in axis.z and axis.w
+// the two random words of its rotation axis, whose lowest bytes hold N_c.
 struct alignas(32) AdjointCell {
     float4 sum, axis;
 };
@@ -235,12 +235,15 @@ constexpr uint32_t kNoSlot = 0xFFFFFFFFu;          // StepArgs::map of a particl
 constexpr uint32_t kTapeNone = 0xFFFFFFFFu;
 constexpr uint32_t kTapeBounce = 0x80000000u;
 
-// One step of the adjoint tape (by particle id / storage cell) and its cells.
+// One step of the adjoint tape (by particle id / storage cell) and its cells; left = the
+// steps of the forward from this one on.
 struct AdjointStep {
     uint64_t step;
+    uint32_t left;
     const uint2* tape;
     const uint32_t *ncell, *lab_count;
     AdjointCell* cells;
+    float* term;   // sampling term of a lab cell, dU(z) / (samples Lx Ly count)
 };
 
 }  // namespace mpcd_gb

@@ -231,7 +231,11 @@ int32_t mpcd_gb_set_drag(mpcd_gb_handle *h, float drag);
  * in reverse.  A forward whose events fit 4 GiB (8 bytes per particle and per cell a step)
  * keeps them instead of checkpoints, and nothing is recomputed.  Afterwards the handle's
  * particle state is that of some step of the forward; set the particles again before
- * stepping on. */
+ * stepping on.
+ * The adjoint velocities are FP32 and the drag gradient is their FP64 sum: both are within
+ * about steps 2^-23 of the gradients in 64 bits (64 x 64 x 34, n = 10, 200 steps: 2.6e-6 and
+ * 1.6e-6).  Sweeps of one forward agree to FP64 rounding; the profile of two forwards of the
+ * same inputs may differ in its last FP32 bits (the sampled sums), the drag gradient by some 1e-9. */
 int32_t mpcd_gb_profile_forward(mpcd_gb_handle *h, int32_t steps, int32_t checkpoint_every, float *d_profile);
 int32_t mpcd_gb_profile_backward(mpcd_gb_handle *h, const float *d_grad_profile, float *d_grad_velocities,
                                  double *grad_drag);
