@@ -329,8 +329,9 @@ public:
     void get_device(float* d_pos, float* d_vel)
     {
         // the first read of a state replays the step straight into the caller's buffers;
-        // later ones keep the state and copy it
-        if (d_pos && d_vel && !dense_valid_ && !direct_read_ && step_ > 0) {
+        // later ones keep the state and copy it.  After a device error nothing reaches the
+        // caller, and the replay is the one that stands particles that were lost.
+        if (d_pos && d_vel && !dense_valid_ && !direct_read_ && step_ > 0 && !device_errors_) {
             launch_replay(d_pos, d_vel, gathers());
             check_device_errors();
             direct_read_ = true;
@@ -1558,7 +1559,7 @@ private:
                               stream_),
               "error flags");
         check(cudaStreamSynchronize(stream_), "step");
-        const unsigned int flags = *to;
+        const unsigned int flags = device_errors_ = *to;
         if (flags & kErrOverflowListFull) throw Error(MPCD_GB_EDEVICE, "cell overflow list exhausted");
         if (flags & kErrWaitTimeout) throw Error(MPCD_GB_EDEVICE, "device wait timed out");
         if (flags & kErrKeyMismatch) throw Error(MPCD_GB_EDEVICE, "particle found in the wrong cell bucket");
@@ -1595,6 +1596,7 @@ private:
         unsigned int* word = nullptr;
         ~PinnedWord() { PinnedWords::give(word); }
     } flags_host_;   // error flags read at the end of a call
+    unsigned int device_errors_ = 0;   // error flags at the end of the last call that read them (they stay set)
     bool direct_read_ = false;   // the state of this step was replayed into a caller's buffers
     bool dense_valid_ = false;   // dense_pos_ / dense_vel_ hold the state after step step_ - 1
     DrawTables tables_{};

@@ -2328,6 +2328,7 @@ __global__ void __launch_bounds__(kThreads, 4) gather_kernel(const StepArgs a, u
     const BoxDesc& b = a.box0;
     const float4 s4 = a.box_shifts[0];
     const float3 s = make_float3(s4.x, s4.y, s4.z);
+    const uint32_t slots = (uint32_t)a.total_slots + a.ext_cap;   // a particle that was lost has no entry: its word may be anything
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t warp = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) >> 5, warps = (uint64_t)gridDim.x * (kThreads / 32);
     for (uint64_t base = warp * 32 * kEach; base < n; base += warps * 32 * kEach) {
@@ -2336,7 +2337,10 @@ __global__ void __launch_bounds__(kThreads, 4) gather_kernel(const StepArgs a, u
 #pragma unroll
         for (int u = 0; u < kEach; ++u) slot[u] = base + 32 * u + lane < n ? a.map[base + 32 * u + lane] : kNoSlot;
 #pragma unroll
-        for (int u = 0; u < kEach; ++u) load_slot(a.in_slots + (slot[u] == kNoSlot ? 0u : slot[u]), xp[u], vp[u]);
+        for (int u = 0; u < kEach; ++u) {
+            if (slot[u] >= slots) slot[u] = kNoSlot;
+            load_slot(a.in_slots + (slot[u] == kNoSlot ? 0u : slot[u]), xp[u], vp[u]);
+        }
 #pragma unroll
         for (int u = 0; u < kEach; ++u) {
             float3 x = make_float3(xp[u].x, xp[u].y, xp[u].z), v = make_float3(vp[u].x, vp[u].y, vp[u].z);
