@@ -1420,14 +1420,19 @@ private:
     }
 
     // Whether the forward records the tape of all its steps, so that the backward
-    // recomputes nothing (and the forward keeps no checkpoints): up to kTapeBytes, where
-    // they can be had.  64 x 64 x 34, n = 10, 200 steps (2.3 GB): forward and backward
+    // recomputes nothing (and the forward keeps no checkpoints): up to 4 GiB, where they can be
+    // had.  64 x 64 x 34, n = 10, 200 steps (2.3 GB): forward and backward
     // 36.5 -> 17 ms, the fused sweep included.
-    static constexpr size_t kTapeBytes = size_t(4) << 30;
+    size_t tape_bytes_ = tape_bytes();
+    static size_t tape_bytes()
+    {
+        const char* e = std::getenv("MPCD_GB_TAPE_BYTES");   // test hook: 0 makes every forward checkpoint
+        return e ? (size_t)std::strtoull(e, nullptr, 10) : size_t(4) << 30;
+    }
 
     bool keep_tape(int steps)
     {
-        if (8 * (N_ + cells_) > kTapeBytes / (size_t)steps) return false;
+        if (8 * (N_ + cells_) > tape_bytes_ / (size_t)steps) return false;
         try {
             alloc_tape(steps);
         } catch (const Error& e) {
