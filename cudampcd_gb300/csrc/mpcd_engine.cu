@@ -549,6 +549,8 @@ public:
         if (adj_taped_) {   // one segment, recorded as it runs
             materialise();
             record_steps(steps, true);
+            sampling_ = true;   // the sums hold its samples, as after step(steps, true)
+            sample_counter_ = (uint64_t)(steps - 1);
             check_device_errors();
         }
         for (int j = 0; !adj_taped_ && j < nseg; ++j) {
