@@ -328,16 +328,32 @@ public:
 
     void get_device(float* d_pos, float* d_vel)
     {
-        // the first read of a state replays the step straight into the caller's buffers;
-        // later ones keep the state and copy it.  After a device error nothing reaches the
-        // caller, and the replay is the one that stands particles that were lost.
-        if (d_pos && d_vel && !dense_valid_ && !direct_read_ && step_ > 0 && !device_errors_) {
-            launch_replay(d_pos, d_vel, gathers());
-            check_device_errors();
-            direct_read_ = true;
-            return;
+        // The first read of a state replays the step straight into the caller's buffers,
+        // and into the dense arrays beside them while the rows are few (fit_l2).  A larger box
+        // reads the dense state's copy back from the caller's buffers, or has it copied to
+        // them, until such a copy turned out to be of no use (the next state came without
+        // it), and from then on keeps none, until something asks for one after all.
+        // After a device error nothing reaches the caller, and the replay is the one that
+        // stands particles that were lost.
+        const bool apart = d_pos && d_vel && (d_pos + 3 * N_ <= d_vel || d_vel + 3 * N_ <= d_pos);
+        if (apart && !dense_valid_ && !direct_read_ && step_ > 0 && !device_errors_ && last_step_run_) {
+            const bool small = fit_l2(), gather = gathers(), drop = !small && dense_use_ == DenseUse::none;
+            if (small || gather || drop) {
+                launch_replay(d_pos, d_vel, gather, small);
+                if (!small && !drop) {
+                    check(cudaMemcpyAsync(dense_pos_.p, d_pos, sizeof(float) * 3 * N_, cudaMemcpyDeviceToDevice, stream_), "positions read");
+                    check(cudaMemcpyAsync(dense_vel_.p, d_vel, sizeof(float) * 3 * N_, cudaMemcpyDeviceToDevice, stream_), "velocities read");
+                }
+                check_device_errors();
+                dense_valid_ = !drop;
+                direct_read_ = drop;
+                dense_kept_ = !small && !drop;
+                return;
+            }
         }
+        const bool fresh = !dense_valid_;
         materialise();
+        dense_kept_ = fresh && d_pos && d_vel;
         if (d_pos)
             check(cudaMemcpyAsync(d_pos, dense_pos_.p, sizeof(float) * 3 * N_, cudaMemcpyDeviceToDevice, stream_),
                   "positions read");
@@ -1308,7 +1324,7 @@ private:
         step_ += (uint64_t)done;
         last_step_table_ = false;
         last_step_run_ = graph_run_;
-        dense_valid_ = direct_read_ = false;
+        new_state();
         return done;
     }
 
@@ -1357,7 +1373,7 @@ private:
         last_step_table_ = use_table_;   // a replay of this step must consume the same draws
         use_table_ = false;
         ++step_;
-        dense_valid_ = direct_read_ = false;
+        new_state();
         return a.fold_samp != nullptr;
     }
 
@@ -1365,12 +1381,17 @@ private:
     // particle id.  A run kernel replays its own steps, from the wall ghosts and grid
     // shifts that the step's prologue left.
     // gather: in two passes, with the (then unused) dense arrays as scratch.
-    void launch_replay(float* pos, float* vel, bool gather = false)
+    // keep: into the dense arrays too (a run kernel's step).
+    void launch_replay(float* pos, float* vel, bool gather = false, bool keep = false)
     {
         StepArgs a = args(step_ - 1, true);
         a.dense_pos = pos;
         a.dense_vel = vel;
         a.run_kernel = last_step_run_;
+        if (keep) {
+            a.keep_pos = dense_pos_.as<float>();
+            a.keep_vel = dense_vel_.as<float>();
+        }
         if (gather) {
             a.map = dense_pos_.as<uint32_t>();
             a.map_cells = dense_vel_.as<AdjointCell>();
@@ -1387,21 +1408,31 @@ private:
     // and 216, 5.2 M 589 and 536, 10.5 M 1189 and 1014, 40 M 5054 and 4934.
     bool gathers() const
     {
-        return boxes_.size() == 1 && last_step_run_ == kRunSrd && 24 * N_ > kGatherBytes && 12 * N_ >= sizeof(AdjointCell) * cells_;
+        return boxes_.size() == 1 && last_step_run_ == kRunSrd && !fit_l2() && 12 * N_ >= sizeof(AdjointCell) * cells_;
     }
-    static constexpr uint64_t kGatherBytes = 20u << 20;
+    bool fit_l2() const { return 24 * N_ <= (20u << 20); }
 
     // The post-step state, by particle id, in dense_pos_ / dense_vel_: recompute
     // the collision of the last step from its inputs (same draws, same
     // arithmetic, bit-identical) unless the dense arrays already hold it.
     void materialise()
     {
+        dense_kept_ = false;   // of use
         if (!dense_valid_) {
             if (step_ == 0) throw Error(MPCD_GB_ESTATE, "no state to read");
+            if (direct_read_) dense_use_ = DenseUse::some;
             launch_replay(dense_pos_.as<float>(), dense_vel_.as<float>());
             check_device_errors();
             dense_valid_ = true;
         }
+    }
+
+    // Another state takes the place of the one that the dense arrays may hold.
+    void new_state(bool dense = false)
+    {
+        if (dense_kept_ && dense_use_ == DenseUse::unknown) dense_use_ = DenseUse::none;
+        dense_kept_ = direct_read_ = false;
+        dense_valid_ = dense;
     }
 
     // Room for a tape of K steps and the adjoint state.
@@ -1478,7 +1509,7 @@ private:
             ++step_;
         }
         last_step_table_ = false;
-        dense_valid_ = direct_read_ = false;
+        new_state();
     }
 
     // Restore checkpoint j and recompute its steps with the tape recorded
@@ -1509,8 +1540,7 @@ private:
                              pos ? dense_pos_.as<float>() : nullptr, vel ? dense_vel_.as<float>() : nullptr, N_, cells_,
                              count_[(k + 1) % 3].as<uint32_t>(), sms_, stream_),
               "scatter");
-        dense_valid_ = true;
-        direct_read_ = false;
+        new_state(true);
     }
 
     void layout(uint32_t* cell, uint32_t* slot, uint32_t* prev, uint32_t* id)
@@ -1604,7 +1634,9 @@ private:
         ~PinnedWord() { PinnedWords::give(word); }
     } flags_host_;   // error flags read at the end of a call
     unsigned int device_errors_ = 0;   // error flags at the end of the last call that read them (they stay set)
-    bool direct_read_ = false;   // the state of this step was replayed into a caller's buffers
+    bool direct_read_ = false;   // the state of this step was replayed into a caller's buffers alone
+    bool dense_kept_ = false;    // the dense arrays hold a copy of a device read that nothing has asked for
+    enum class DenseUse { unknown, none, some } dense_use_ = DenseUse::unknown;   // whether such copies are of use
     bool dense_valid_ = false;   // dense_pos_ / dense_vel_ hold the state after step step_ - 1
     DrawTables tables_{};
     int inject_valid_[kMaxInjectedShifts] = {0, 0, 0, 0};

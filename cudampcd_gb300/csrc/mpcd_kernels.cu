@@ -589,6 +589,10 @@ __device__ void overflow_pass(const StepArgs& a, uint64_t step)
                 const uint64_t i3 = 3 * (uint64_t)id;
                 a.dense_pos[i3] = x.x; a.dense_pos[i3 + 1] = x.y; a.dense_pos[i3 + 2] = x.z;
                 a.dense_vel[i3] = v.x; a.dense_vel[i3 + 1] = v.y; a.dense_vel[i3 + 2] = v.z;
+                if (a.keep_pos) {
+                    a.keep_pos[i3] = x.x; a.keep_pos[i3 + 1] = x.y; a.keep_pos[i3 + 2] = x.z;
+                    a.keep_vel[i3] = v.x; a.keep_vel[i3 + 1] = v.y; a.keep_vel[i3 + 2] = v.z;
+                }
                 if (a.map) a.map[id] = kNoSlot;   // done: the gather passes it by
             } else {
                 vs = v;
@@ -1317,8 +1321,8 @@ __device__ __forceinline__ uint32_t wall_side(const BoxDesc& b, uint32_t z)
 // floats), so that consecutive lanes write consecutive words of a row and a warp's store
 // touches a third of the sectors that a store per component does (replay of 1.49e7
 // particles in random order 1600 -> 1216 us, bound by the random writes; of 449,000 that
-// fit L2 26.7 -> 12.7).
-__device__ __forceinline__ void write_rows(float* stage, float* dense, uint32_t id, float3 r, unsigned mask)
+// fit L2 26.7 -> 12.7).  keep (or null): another array that gets them.
+__device__ __forceinline__ void write_rows(float* stage, float* dense, float* keep, uint32_t id, float3 r, unsigned mask)
 {
     const uint32_t lane = threadIdx.x & 31u;
     stage[3 * lane] = r.x;
@@ -1330,6 +1334,7 @@ __device__ __forceinline__ void write_rows(float* stage, float* dense, uint32_t 
         const uint32_t w = 32 * t + lane, row = w / 3;
         const uint64_t at = 3 * (uint64_t)__shfl_sync(kFull, id, (int)row) + (w - 3 * row);
         if (mask >> row & 1u) dense[at] = stage[w];
+        if (keep && (mask >> row & 1u)) keep[at] = stage[w];
     }
     __syncwarp();
 }
@@ -1619,8 +1624,8 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
                     // staged in the places of the pass, which every lane has read
                     float* const stage = STAGED ? &ring.pos[gpos].x : shared_rows[REPLAY && !STAGED ? threadIdx.x >> 5 : 0];
                     __syncwarp();
-                    write_rows(stage, a.dense_pos, __float_as_uint(vp.w), x, rows);
-                    write_rows(stage, a.dense_vel, __float_as_uint(vp.w), v, rows);
+                    write_rows(stage, a.dense_pos, a.keep_pos, __float_as_uint(vp.w), x, rows);
+                    write_rows(stage, a.dense_vel, a.keep_vel, __float_as_uint(vp.w), v, rows);
                     gpos = gpos + 32 == kRing ? 0u : gpos + 32;
                     continue;
                 }
@@ -2077,8 +2082,8 @@ __global__ void __launch_bounds__(kExtThreads, kExtBlocks) ext_run_kernel(const 
                 }
                 if (REPLAY) {   // staged in the terms' room
                     const unsigned rows = __ballot_sync(kFull, active);
-                    write_rows(&sh.term[0][0], a.dense_pos, __float_as_uint(vp.w), x, rows);
-                    write_rows(&sh.term[0][0], a.dense_vel, __float_as_uint(vp.w), v, rows);
+                    write_rows(&sh.term[0][0], a.dense_pos, a.keep_pos, __float_as_uint(vp.w), x, rows);
+                    write_rows(&sh.term[0][0], a.dense_vel, a.keep_vel, __float_as_uint(vp.w), v, rows);
                     continue;
                 }
                 float3 vn = v;

@@ -185,6 +185,7 @@ struct StepArgs {
     int32_t replay;
     float* dense_pos;
     float* dense_vel;
+    float *keep_pos, *keep_vel;   // a run kernel's replay into a caller's buffers: the rows here too (or null)
     // a replay that gathers (one SRD box): the slot of every particle by id, and the cells
     uint32_t* map;
     AdjointCell* map_cells;
