@@ -319,9 +319,28 @@ public:
     }
 
     // ------------------------------------------------------------ device-pointer I/O, drag
+    // Whether kernels may use a caller's pointer: memory of the handle's own GPU.  Any other
+    // (another GPU's, managed, pinned) is copied, which needs no peer access.
+    bool own_memory(const void* p) const
+    {
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        return at.type == cudaMemoryTypeDevice && at.device == (int)params_.device_id;
+    }
+
     void set_device(const float* d_pos, const float* d_vel)
     {
         if (!d_pos || !d_vel) materialise();
+        auto reach = [&](const float*& from, const DeviceBuffer& to, const char* what) {
+            if (!from || own_memory(from)) return;
+            check(cudaMemcpyAsync(to.p, from, sizeof(float) * 3 * N_, cudaMemcpyDeviceToDevice, stream_), what);
+            from = nullptr;   // in the dense arrays now
+        };
+        reach(d_pos, dense_pos_, "positions write");
+        reach(d_vel, dense_vel_, "velocities write");
         scatter_dense(nullptr, d_pos, d_vel);
         check_device_errors();
     }
@@ -336,7 +355,7 @@ public:
         // After a device error nothing reaches the caller, and the replay is the one that
         // stands particles that were lost.
         const bool apart = d_pos && d_vel && (d_pos + 3 * N_ <= d_vel || d_vel + 3 * N_ <= d_pos);
-        if (apart && !dense_valid_ && !direct_read_ && step_ > 0 && !device_errors_ && last_step_run_) {
+        if (apart && !dense_valid_ && !direct_read_ && step_ > 0 && !device_errors_ && last_step_run_ && own_memory(d_pos) && own_memory(d_vel)) {
             const bool small = fit_l2(), gather = gathers(), drop = !small && dense_use_ == DenseUse::none;
             if (small || gather || drop) {
                 launch_replay(d_pos, d_vel, gather, small);

@@ -1,6 +1,9 @@
 """Device reads: what a caller gets when a step failed, and reads mixed with partial writes."""
 from __future__ import annotations
 
+import contextlib
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -129,6 +132,39 @@ def test_a_read_into_overlapping_buffers_leaves_the_state():
         for x in (h, r):
             x.step(2)
         h.get_particles_device(both.data_ptr(), both.data_ptr())
+        assert np.array_equal(h.positions(), r.positions()) and np.array_equal(h.velocities(), r.velocities())
+    finally:
+        h.close()
+        r.close()
+
+
+@contextlib.contextmanager
+def _managed(n):
+    """n floats of managed memory (which is not the GPU's own), by pointer and as an array."""
+    cu, at = ctypes.CDLL("libcuda.so.1"), ctypes.c_uint64()
+    assert cu.cuMemAllocManaged(ctypes.byref(at), ctypes.c_size_t(4 * n), 1) == 0
+    try:
+        yield at.value, np.ctypeslib.as_array((ctypes.c_float * n).from_address(at.value))
+    finally:
+        assert cu.cuMemFree_v2(at) == 0
+
+
+@pytest.mark.parametrize("name", ["small", "extended", "gathered"])
+def test_buffers_that_are_not_the_gpus_own_are_copied(name):
+    """Only memory of the handle's GPU is read and written by kernels."""
+    h, r = capi.Handle(**BOXES[name]), capi.Handle(**BOXES[name])
+    torch.zeros(1, device="cuda")   # a current context for the allocations
+    try:
+        with _managed(3 * h.N) as (dp, p), _managed(3 * h.N) as (dv, v):
+            for k in range(4):
+                h.step(1)
+                r.step(1)
+                h.get_particles_device(dp, dv)
+                torch.cuda.synchronize()
+                assert np.array_equal(p.reshape(-1, 3), r.positions()) and np.array_equal(v.reshape(-1, 3), r.velocities())
+                v[:] = v.reshape(-1, 3)[::-1].ravel().copy()
+                h.set_particles_device(dp if k % 2 else 0, dv)
+                r.set_velocities(v.reshape(-1, 3).copy())
         assert np.array_equal(h.positions(), r.positions()) and np.array_equal(h.velocities(), r.velocities())
     finally:
         h.close()
