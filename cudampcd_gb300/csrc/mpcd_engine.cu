@@ -160,7 +160,7 @@ public:
     Engine(const mpcd_gb_params* ps, int R) : params_(ps[0]), box_params_(ps, ps + R)
     {
         validate();
-        build_boxes();   // host-side sizes and limits, before any CUDA call
+        build_boxes(true);   // host-side sizes and limits, before any CUDA call
         check(cudaSetDevice((int)params_.device_id), "cudaSetDevice");
         check(cudaStreamCreateWithFlags(&own_stream_, cudaStreamNonBlocking), "cudaStreamCreate");
         stream_ = own_stream_;
@@ -175,8 +175,17 @@ public:
         check(cudaGetDeviceProperties(&prop, (int)params_.device_id), "cudaGetDeviceProperties");
         sms_ = prop.multiProcessorCount;
         run_grid_ = sms_ * run_blocks_per_sm(params_.algorithm);
+        if (deep_bytes_ && !roomy(deep_bytes_)) build_boxes(false);
         set_runs();
-        allocate();
+        try {
+            allocate();
+        } catch (const Error& e) {   // what the shallow buckets need may be there
+            if (e.code() != MPCD_GB_ENOMEM || !deep_bytes_) throw;
+            for (DeviceBuffer* d : {&slots_[0], &slots_[1]}) d->release();
+            build_boxes(false);
+            set_runs();
+            allocate();
+        }
         configure();
         initialise();
     }
@@ -930,6 +939,14 @@ private:
     }
     static constexpr uint64_t kDeepBytes = 32ull << 30;   // both bucket sets, up to which they are deep
 
+    // Whether memory that a handle can do without is there to take: a quarter of what is
+    // free (not asked for below 1 GiB).
+    static bool roomy(size_t bytes)
+    {
+        size_t free = 0, total = 0;
+        return bytes <= size_t(1) << 30 || (cudaMemGetInfo(&free, &total) == cudaSuccess && bytes <= free / 4);
+    }
+
     static BoxDesc make_box(const mpcd_gb_params& p, bool deep)
     {
         BoxDesc b{};
@@ -973,16 +990,18 @@ private:
         return b;
     }
 
-    void build_boxes()
+    // deep: buckets of the greater depth where they are at most kDeepBytes.
+    void build_boxes(bool deep)
     {
         boxes_.clear();
         uint64_t cells = 0, slots = 0, particles = 0, walls = 0;
         uint32_t n_max = 0;
-        double deep_bytes = 0.0;
+        double bytes = 0.0;
         for (const mpcd_gb_params& p : box_params_)
-            deep_bytes += 2.0 * sizeof(Slot) * bucket_depth(p.n, true) * p.volume_size[0] * p.volume_size[1] * p.volume_size[2];
+            bytes += 2.0 * sizeof(Slot) * bucket_depth(p.n, true) * p.volume_size[0] * p.volume_size[1] * p.volume_size[2];
+        deep_bytes_ = deep && bytes <= (double)kDeepBytes ? (size_t)bytes : 0;
         for (const mpcd_gb_params& p : box_params_) {
-            BoxDesc b = make_box(p, deep_bytes <= (double)kDeepBytes);
+            BoxDesc b = make_box(p, deep_bytes_ != 0);
             if (cells + b.C >= (1ull << 31)) throw Error(MPCD_GB_EINVAL, "too many cells in the ensemble");
             b.cell_base = (uint32_t)cells;
             b.slot_base = slots;
@@ -1167,7 +1186,7 @@ private:
         if (walls_) check(ghosts_.alloc(sizeof(GhostSum) * walls_ * 2), "alloc wall ghosts");   // two parities
         check(box_shifts_.alloc(sizeof(float4) * 4 * boxes_.size()), "alloc box shifts");
         check(state_.alloc(sizeof(DeviceState)), "alloc state");
-        flags_host_.word = PinnedWords::take();
+        if (!flags_host_.word) flags_host_.word = PinnedWords::take();
         check(cudaMemset(state_.p, 0, sizeof(DeviceState)), "clear state");
         check(samp_.alloc(sizeof(float4) * cells_ * 2), "alloc sample");   // two parities
         check(cudaMemset(samp_.p, 0, samp_.bytes), "clear sample");
@@ -1472,8 +1491,8 @@ private:
     }
 
     // Whether the forward records the tape of all its steps, so that the backward
-    // recomputes nothing (and the forward keeps no checkpoints): up to 4 GiB, where they can be
-    // had.  64 x 64 x 34, n = 10, 200 steps (2.3 GB): forward and backward
+    // recomputes nothing (and the forward keeps no checkpoints): up to 4 GiB, where there is
+    // room.  64 x 64 x 34, n = 10, 200 steps (2.3 GB): forward and backward
     // 36.5 -> 17 ms, the fused sweep included.
     size_t tape_bytes_ = tape_bytes();
     static size_t tape_bytes()
@@ -1484,7 +1503,8 @@ private:
 
     bool keep_tape(int steps)
     {
-        if (8 * (N_ + cells_) > tape_bytes_ / (size_t)steps) return false;
+        const size_t bytes = 8 * (N_ + cells_) * (size_t)steps;
+        if (8 * (N_ + cells_) > tape_bytes_ / (size_t)steps || (tape_.bytes < sizeof(uint2) * N_ * (size_t)steps && !roomy(bytes))) return false;
         try {
             alloc_tape(steps);
         } catch (const Error& e) {
@@ -1637,6 +1657,7 @@ private:
     std::vector<BoxDesc> boxes_;
     uint64_t N_ = 0, cells_ = 0, tiles_ = 0, total_slots_ = 0, walls_ = 0;
     uint32_t ov_cap_ = 0, ext_cap_ = 0, pbuf_ = 0;
+    size_t deep_bytes_ = 0;      // bytes of the deep buckets (0: shallow ones)
     uint64_t layout_tail_ = 0;   // overflow-list particles of the last layout
     uint32_t max_tile_cells_ = 0, forced_tile_cells_ = 0;   // largest tile of any box; a tile size forced for all
     double fill_ = 1.0;                                      // expected particles per tile = pbuf / fill

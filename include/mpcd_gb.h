@@ -229,7 +229,9 @@ int32_t mpcd_gb_set_drag(mpcd_gb_handle *h, float drag);
  * and wall bounces are held fixed at those of the forward trajectory: each checkpoint
  * segment is recomputed (its draws replayed from the Philox counters) and then swept
  * in reverse.  A forward whose events fit 4 GiB (8 bytes per particle and per cell a step)
- * keeps them instead of checkpoints, and nothing is recomputed.  Afterwards the handle's
+ * keeps them instead of checkpoints where they are at most a quarter of the free memory (1 GiB
+ * in any case), and nothing is recomputed; the handle holds that memory until it is destroyed.
+ * Afterwards the handle's
  * particle state is that of some step of the forward; set the particles again before
  * stepping on.
  * The adjoint velocities are FP32 and the drag gradient is their FP64 sum: both are within
