@@ -518,6 +518,11 @@ def device_memory(handle_bytes: int, n: int, cells: int, particles: int) -> dict
             "buckets_gb_at_reference_depth": 2 * 32 * cells * 4 * n / 1e9}
 
 
+def step_kernel_name(algorithm: int, n: int) -> str:
+    """The kernel that runs a box of density n (denser boxes stay on the tile kernel)."""
+    return ("srd_run_kernel" if n <= 64 else "step_kernel") if algorithm == 0 else ("ext_run_kernel" if n <= 36 else "step_kernel")
+
+
 def run_gpu_arm(args, rank, world, local_rank):
     import torch
 
@@ -585,7 +590,7 @@ def run_gpu_arm(args, rank, world, local_rank):
                          "frac": achieved / peak, "peak_kind": peak_kind,
                          "traffic": bpp * N if bpp else None, "traffic_source": src,
                          "algorithmic_bytes_per_particle": ALGO_BYTES_PER_PARTICLE,
-                         "kernel": "srd_run_kernel" if algorithm == 0 else "ext_run_kernel",
+                         "kernel": step_kernel_name(algorithm, wl["n"]),
                          "kernel_ms": per_launch_ms},
             "e2e": e2e,
             "clocks": clocks.summary(),

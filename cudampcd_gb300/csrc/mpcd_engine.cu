@@ -592,7 +592,7 @@ public:
         sampling_ = false;
         if (adj_taped_) {   // one segment, recorded as it runs
             materialise();
-            record_steps(steps, true);
+            record_steps(steps);
             sampling_ = true;   // the sums hold its samples, as after step(steps, true)
             sample_counter_ = (uint64_t)(steps - 1);
             check_device_errors();
@@ -1109,12 +1109,13 @@ private:
         for (auto& g : graph_) g.reset();   // graphs bake the tiling into their launches
     }
 
-    // Runs of srd_run_kernel: up to 32 cells of one box, {first cell, cells | box << 6},
-    // listed by batch class (16, 8, then 4 cells per batch; one launch per class).
-    // The cells of a run: 32 where the sweep is long.  A box that fills the GPU's warps
-    // (32 per SM) only k < 8 times over takes the length that makes k full rounds of
-    // them, so that no warp sweeps a run more than another, and at least the cells of
-    // one pass of 32 particles.  Step us at 61 x 61 x 85, n = 7 (2.03 rounds of 32-cell
+    // Runs of the run kernels, {first cell, cells | box << 6}: consecutive cells of one box, up
+    // to 32 for srd_run_kernel, listed by batch class (16, 8, then 4 cells per batch; one
+    // launch per class), and up to 24 for ext_run_kernel, one class (run_cells_max).
+    // The cells of a run: the most where the sweep is long.  A box that fills the GPU's warps
+    // (32 per SM, extended 24) only k < 8 times over takes the length that makes k full rounds
+    // of them, so that no warp sweeps a run more than another, and at least the cells of
+    // one pass of 32 particles (adjoint tapes excepted, record_steps).  Step us at 61 x 61 x 85, n = 7 (2.03 rounds of 32-cell
     // runs), 33 x 47 x 29, n = 10 (0.29) and 16^3, n = 10 (0.03): 62.9 -> 57.2, 26.2 ->
     // 17.7 and 22.8 -> 9.7 against 32-cell runs.
     void set_runs()
@@ -1492,8 +1493,8 @@ private:
 
     // Whether the forward records the tape of all its steps, so that the backward
     // recomputes nothing (and the forward keeps no checkpoints): up to 4 GiB, where there is
-    // room.  64 x 64 x 34, n = 10, 200 steps (2.3 GB): forward and backward
-    // 36.5 -> 17 ms, the fused sweep included.
+    // room (roomy).  64 x 64 x 34, n = 10, 200 steps (2.3 GB): forward and backward 36.5 ms with
+    // checkpoints and the sweep in three passes, 14.8 so.
     size_t tape_bytes_ = tape_bytes();
     static size_t tape_bytes()
     {
@@ -1517,8 +1518,8 @@ private:
 
     // Run `steps` sampled steps from the dense state, recording the tape (slot i = the i-th
     // of them; b0 = the bounces of the initial streaming).  A step folds the sample of the
-    // one before and records its lab counts; `start`: the sums start from these steps.
-    void record_steps(int steps, bool start)
+    // one before and records its lab counts; the sums start from these steps.
+    void record_steps(int steps)
     {
         scatter_dense(tb0_.as<uint32_t>());
         for (int i = 0; i < steps; ++i) {
@@ -1541,7 +1542,7 @@ private:
             check(select_overflow(a, step_, stream_), "overflow selection");
             check(launch_step(a, params_.algorithm, false, pbuf_, a.run_kernel ? run_grid_ : grid_, stream_), "tape step");
             if (i == 0 || !a.run_kernel || i == steps - 1)
-                check(launch_sample_finalize(a.samp, acc_.as<SampleAcc>(), cells_, start && i == 0 ? 1 : 0, sms_ * 8, stream_,
+                check(launch_sample_finalize(a.samp, acc_.as<SampleAcc>(), cells_, i == 0 ? 1 : 0, sms_ * 8, stream_,
                                              tcnt_.as<uint32_t>() + (size_t)i * cells_),
                       "tape sample");
             last_step_run_ = a.run_kernel;
@@ -1561,7 +1562,7 @@ private:
         check(cudaMemcpyAsync(dense_pos_.p, c, per / 2, cudaMemcpyDeviceToDevice, stream_), "restore");
         check(cudaMemcpyAsync(dense_vel_.p, c + per / 2, per / 2, cudaMemcpyDeviceToDevice, stream_), "restore");
         step_ = adj_s0_ + (uint64_t)j * adj_every_;
-        record_steps(k, true);
+        record_steps(k);
         return k;
     }
 

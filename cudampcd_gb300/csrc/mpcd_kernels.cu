@@ -1402,8 +1402,8 @@ __global__ void __launch_bounds__(kThreads, 4) srd_run_kernel(const StepArgs a, 
         if (!REPLAY && valid) a.zero_count[cur.x + lane] = 0;   // counts of step k-1: step k+1 fills them
         // sampled steps: the previous step's sample of this lane's (lab) cell into the
         // FP64 sums, where the engine defers it to this step (every cell is one lane's);
-        // its loads wait beside another wait of the run (at the top of the run a sampled
-        // step of 10 x 10 x 102, n = 10 took 10.7 us, so 10.0)
+        // its loads wait beside another wait of the run (a sampled step of 10 x 10 x 102,
+        // n = 10 takes 10.0 us; with the fold at the top of the run 10.7)
         auto fold = [&]() {
             if (SAMPLE && a.fold_samp && valid) fold_sample(a.fold_samp, a.acc, cur.x + lane, 0, TAPE ? a.fold_count : nullptr);
         };
@@ -2894,7 +2894,10 @@ static StepFnRun run_fn(int cls, bool staged, bool sample, bool single, bool rep
 // Ensembles stage their particles through the ring, a single box does not: us a step,
 // unstaged and staged, 64 uneven channels 1144 and 978 (sampled 1399 and 1196); 500 x 500
 // x 22, n = 20 1478 and 1544 (1780 and 1862); 300 x 300 x 102, n = 10 1572 and 1552 (1900
-// and 1931).  Staging spares the finish its slot loads, of which only 30 % hit L1, but
+// and 1931); boxes of one round of runs or two: 33 x 47 x 29, n = 10 14.7 and 15.9 (16.9 and
+// 17.6), 61 x 61 x 85, n = 7 56.9 and 59.9 (65.8 and 67.9), 64 x 64 x 34, n = 10 29.6 and
+// 30.2 (34.4 and 33.8; with the adjoint tape 40.5 and 40.1), 10 x 10 x 102, n = 10 9.0 and 9.3
+// (10.3 and 11.0).  Staging spares the finish its slot loads, of which only 30 % hit L1, but
 // leaves the copies less lead than the L2 prefetch of a single box's sweep.  Batches that
 // fit the ring only in part wait for room (copied in part: 1056 and 1726).
 static bool run_staged(bool single, int cls, uint32_t n_max) { return !single && (cls < 2 || n_max <= kRingMaxN); }
