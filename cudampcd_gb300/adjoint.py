@@ -15,9 +15,15 @@ adjoint holds the discrete events of the forward trajectory fixed:
 - ghost counts;
 - wall bounces.
 
-A forward whose events fit 4 GiB keeps them all.  A longer one checkpoints the state
-every `checkpoint_every` steps, and the backward recomputes one segment at a time, then
-sweeps it in reverse. It returns dL/dV0 for every particle and dL/d(drag).
+A forward whose events fit 4 GiB, and a quarter of the free memory, keeps them all.  A
+longer one checkpoints the state every `checkpoint_every` steps, and the backward recomputes
+one segment at a time, then sweeps it in reverse.  It returns dL/dV0 for every particle and
+dL/d(drag).
+
+The adjoint velocities are float32 and dL/d(drag) is their float64 sum: both are within about
+steps 2^-23 of the float64 gradients (64 x 64 x 34, n = 10, 200 steps: 2.6e-6 and 1.6e-6).
+Backward passes of one forward agree to float64 rounding; two forwards of the same inputs may
+differ in the last bits of the float32 profile, and dL/d(drag) then by some 1e-9.
 """
 from __future__ import annotations
 

@@ -1528,7 +1528,9 @@ private:
             a.tape = tape_.as<uint2>() + (size_t)i * N_;
             a.tape_ncell = tncell_.as<uint32_t>() + (size_t)i * cells_;
             // 32-cell runs whatever the box: their order of arrival is that of the sampled sums,
-            // whose last bits reach the drag gradient (shorter runs moved it by up to 6e-9 in small boxes)
+            // whose last bits reach the drag gradient (shorter runs moved it by up to 6e-9 in
+            // small boxes).  A taped step of 10 x 10 x 102, n = 10 takes 24.5 us so and 10.7 with
+            // short runs, of 64 x 64 x 34 37.5 and 36.2.
             a.box0.run_cells = run_cells_max(params_.algorithm, boxes_[0].n);
             const uint32_t runs = (boxes_[0].C + a.box0.run_cells - 1) / a.box0.run_cells;
             for (uint32_t& r : a.run_class) r = r ? runs : 0;

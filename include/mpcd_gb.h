@@ -231,9 +231,8 @@ int32_t mpcd_gb_set_drag(mpcd_gb_handle *h, float drag);
  * in reverse.  A forward whose events fit 4 GiB (8 bytes per particle and per cell a step)
  * keeps them instead of checkpoints where they are at most a quarter of the free memory (1 GiB
  * in any case), and nothing is recomputed; the handle holds that memory until it is destroyed.
- * Afterwards the handle's
- * particle state is that of some step of the forward; set the particles again before
- * stepping on.
+ * Afterwards the handle's particle state is that of some step of the forward; set the
+ * particles again before stepping on.
  * The adjoint velocities are FP32 and the drag gradient is their FP64 sum: both are within
  * about steps 2^-23 of the gradients in 64 bits (64 x 64 x 34, n = 10, 200 steps: 2.6e-6 and
  * 1.6e-6).  Sweeps of one forward agree to FP64 rounding; the profile of two forwards of the
