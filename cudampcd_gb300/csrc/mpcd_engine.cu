@@ -356,18 +356,18 @@ public:
 
     void get_device(float* d_pos, float* d_vel)
     {
-        // The first read of a state replays the step straight into the caller's buffers,
-        // and into the dense arrays beside them while the rows are few (fit_l2).  A larger box
-        // reads the dense state's copy back from the caller's buffers, or has it copied to
-        // them, until such a copy turned out to be of no use (the next state came without
-        // it), and from then on keeps none, until something asks for one after all.
+        // The first read of a state replays the step straight into the caller's buffers.  The
+        // dense arrays get a copy, written beside them while the rows are few (fit_l2), read
+        // back from them or copied to them in a larger box, until such a copy turned out to be
+        // of no use (the next state came without it); from then on none is kept, until
+        // something asks for one after all.
         // After a device error nothing reaches the caller, and the replay is the one that
         // stands particles that were lost.
         const bool apart = d_pos && d_vel && (d_pos + 3 * N_ <= d_vel || d_vel + 3 * N_ <= d_pos);
         if (apart && !dense_valid_ && !direct_read_ && step_ > 0 && !device_errors_ && last_step_run_ && own_memory(d_pos) && own_memory(d_vel)) {
-            const bool small = fit_l2(), gather = gathers(), drop = !small && dense_use_ == DenseUse::none;
+            const bool small = fit_l2(), gather = gathers(), drop = dense_use_ == DenseUse::none;
             if (small || gather || drop) {
-                launch_replay(d_pos, d_vel, gather, small);
+                launch_replay(d_pos, d_vel, gather, small && !drop);
                 if (!small && !drop) {
                     check(cudaMemcpyAsync(dense_pos_.p, d_pos, sizeof(float) * 3 * N_, cudaMemcpyDeviceToDevice, stream_), "positions read");
                     check(cudaMemcpyAsync(dense_vel_.p, d_vel, sizeof(float) * 3 * N_, cudaMemcpyDeviceToDevice, stream_), "velocities read");
@@ -375,7 +375,7 @@ public:
                 check_device_errors();
                 dense_valid_ = !drop;
                 direct_read_ = drop;
-                dense_kept_ = !small && !drop;
+                dense_kept_ = !drop;
                 return;
             }
         }
